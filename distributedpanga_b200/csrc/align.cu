@@ -270,8 +270,7 @@ __device__ AlignSpec launch_spec(const AlignLaunch &P) {
   spec.trace_space = TSPACE;
   spec.ave_path = P.ave_path;
   spec.reach = 0;
-  spec.score = P.score;
-  spec.table = P.table;
+  spec.dscore = P.dscore;
   return spec;
 }
 
@@ -279,17 +278,11 @@ __device__ AlignSpec launch_spec(const AlignLaunch &P) {
 __device__ WarpWork warp_work(const AlignLaunch &P, int64_t wid) {
   WarpWork W;
   int *wb = P.wave + wid * (int64_t)P.vcap * WAVE_INTS;
-  W.V[0] = wb;
-  W.V[1] = wb + P.vcap;
-  W.M[0] = wb + 2 * P.vcap;
-  W.M[1] = wb + 3 * P.vcap;
-  W.HA[0] = wb + 4 * P.vcap;
-  W.HA[1] = wb + 5 * P.vcap;
-  W.NA = wb + 6 * P.vcap;
-  W.HM[0] = wb + 7 * P.vcap;
-  W.HM[1] = wb + 8 * P.vcap;
-  W.T[0] = (uint64_t *)(wb + 9 * P.vcap);
-  W.T[1] = (uint64_t *)(wb + 11 * P.vcap);
+  W.C[0] = (RingCell *)wb;
+  W.C[1] = (RingCell *)wb + P.vcap;
+  W.V[0] = wb + 8 * P.vcap;
+  W.V[1] = wb + 9 * P.vcap;
+  W.NA = wb + 10 * P.vcap;
   W.vcap = P.vcap;
   W.points = P.points + wid * P.point_cap;
   W.point_cap = P.point_cap;
@@ -310,14 +303,11 @@ __device__ WarpWork warp_work(const AlignLaunch &P, int64_t wid) {
 __device__ Seq contig_seq(const AlignLaunch &P, int c, bool as_a, bool comp) {
   const uint8_t *buf = (as_a && comp) ? P.rc : P.fwd;
   Seq S{buf + P.soff[c], (int)P.clen[c]};
-  const uint64_t *base = P.pk + P.poff[c] * 4;
-  if (as_a) {
-    S.pf = base + (comp ? 2 : 0) * P.pwords[c];
-    S.pr = base + (comp ? 3 : 1) * P.pwords[c];
-  } else {
-    S.pf = base;
-    S.pr = base + P.pwords[c];
-  }
+  const uint32_t *base = (const uint32_t *)(P.pk + P.poff[c] * 4);
+  const int64_t nw = 2 * P.pwords[c];
+  const int first = as_a && comp ? 2 : 0;
+  S.pf = base + first * nw;
+  S.pr = base + (first + 1) * nw;
   return S;
 }
 
@@ -763,8 +753,9 @@ __global__ void k_numeric(const uint8_t *__restrict__ bps, const int64_t *__rest
   }
 }
 
-// 2-bit packed copies of every contig, 32 bases per word, first base in the
-// top bits, one zero pad word after each: forward, reversed, reverse
+// 2-bit packed copies of every contig, 16 bases per 32-bit word, first base
+// in the top bits (stored two words at a time), zero pad words after each:
+// forward, reversed, reverse
 // complement and complement-only (the reverse of the reverse complement) --
 // the packed forms of the sequences the forward and reverse snakes read.
 __global__ void k_pack(const uint8_t *__restrict__ fwd, const int64_t *__restrict__ soff,
@@ -784,10 +775,11 @@ __global__ void k_pack(const uint8_t *__restrict__ fwd, const int64_t *__restric
         bf = s[i];
         br = s[n - 1 - i];
       }
-      f |= bf << (62 - 2 * q);
-      r |= br << (62 - 2 * q);
-      rc |= (i < n ? (3 - br) : 0) << (62 - 2 * q);
-      co |= (i < n ? (3 - bf) : 0) << (62 - 2 * q);
+      const int sh = q < 16 ? 30 - 2 * q : 94 - 2 * q;  // the pair's first word is its low half
+      f |= bf << sh;
+      r |= br << sh;
+      rc |= (i < n ? (3 - br) : 0) << sh;
+      co |= (i < n ? (3 - bf) : 0) << sh;
     }
     F[w] = f;
     R[w] = r;

@@ -10,7 +10,7 @@
 namespace pga {
 
 constexpr int ALIGN_THREADS = 128;  // 4 warps per CTA, one pair per warp at a time
-constexpr int WAVE_INTS = 13;       // per diagonal slot: V,M,HA,HM x2, NA, T x2 (uint64)
+constexpr int WAVE_INTS = 11;       // per diagonal slot: RingCell x2, V x2, NA
 
 // One (anchor, partner) pair of a unit: seeds [lo, hi) of the unit's sorted
 // keys.  seg < 0: the whole pair, finished by the same warp.  seg >= 0: band
@@ -91,8 +91,7 @@ struct AlignLaunch {
   const int64_t *soff, *clen;
   const uint64_t *pk;            // packed sequences: contig c at word 4*poff[c]: F, R, RC, CO (pwords[c] each)
   const int64_t *poff, *pwords;
-  const int16_t *score, *table;
-  int ave_path;
+  int ave_path, dscore;          // New_Align_Spec's path average and mismatch penalty
   int64_t amxpos, maxdag;
   int64_t nwarps;
   int *wave;

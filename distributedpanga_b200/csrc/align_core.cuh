@@ -54,14 +54,16 @@ constexpr int64_t MAX_I64 = 0x7fffffffffffffffll;
 
 enum : int { ALN_ERR_VCAP = 1, ALN_ERR_CELLS = 2, ALN_ERR_POINTS = 4, ALN_ERR_OVLS = 8, ALN_ERR_TRACE = 16 };
 
-// Trim tables and path parameters of New_Align_Spec (lib/align.c:222-268),
-// built on the host by build_align_spec.
+// Path parameters of New_Align_Spec (lib/align.c:222-268), from the host's
+// align_params.  The device's trim test needs the mismatch penalty alone; the
+// host harness reads the trim tables built by build_align_spec.
 struct AlignSpec {
   int trace_space;
   int ave_path;
   int reach;
-  const int16_t *score;  // TRIM_MASK+1 entries
-  const int16_t *table;  // TRIM_MASK+1 entries
+  int dscore;                      // mismatch penalty, in 1/1000 units (a match scores 1000 - dscore)
+  const int16_t *score = nullptr;  // TRIM_MASK+1 entries
+  const int16_t *table = nullptr;  // TRIM_MASK+1 entries
 };
 
 struct Pebble {
@@ -74,14 +76,14 @@ struct Path {
 };
 
 // A sequence with sentinel value 4 at [-1] and [len], NUMERIC bases 0..3.
-// The device aligner also reads it 2-bit packed, 32 bases per word with the
+// The device aligner also reads it 2-bit packed, 16 bases per word with the
 // first base in the top bits: pf forwards, pr reversed (pr's base i is
-// s[len-1-i]); both end with a zero pad word.  The host code leaves them null.
+// s[len-1-i]); both end with zero pad words.  The host code leaves them null.
 struct Seq {
   const uint8_t *s;
   int len;
-  const uint64_t *pf = nullptr;
-  const uint64_t *pr = nullptr;
+  const uint32_t *pf = nullptr;
+  const uint32_t *pr = nullptr;
 };
 
 // ---------------------------------------------------------------------------

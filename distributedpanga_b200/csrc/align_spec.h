@@ -23,9 +23,9 @@ inline void fill_trim_tables(int bit, int prefix, int score, int max, int mscore
   }
 }
 
-// freq: the GDB's base frequencies (float, as stored).  Fills score_t and
-// table_t (32768 entries each) and returns ave_path.
-inline int build_align_spec(const float *freq, int16_t *score_t, int16_t *table_t) {
+// freq: the GDB's base frequencies (float, as stored).  Sets the mismatch
+// penalty dscore (1/1000 units) and returns ave_path.
+inline int align_params(const float *freq, int *dscore) {
   static const double bias_factor[10] = {.690, .690, .690, .690, .780, .850, .900, .933, .966, 1.000};
   const double ave_corr = 1. - 0.3;
   float fm = freq[0] + freq[3];
@@ -34,10 +34,15 @@ inline int build_align_spec(const float *freq, int16_t *score_t, int16_t *table_
   if (match > .5) match = 1. - match;
   int bias = (int)((match + .025) * 20. - 1.);
   if (match < .2) bias = 3;
-  int ave_path = (int)(60 * (1. - bias_factor[bias] * (1. - ave_corr)));
-  int mscore = (int)(1000 * bias_factor[bias] * (1. - ave_corr));
-  int dscore = 1000 - mscore;
-  fill_trim_tables(0, 0, 0, 0, mscore, dscore, score_t, table_t);
+  *dscore = 1000 - (int)(1000 * bias_factor[bias] * (1. - ave_corr));
+  return (int)(60 * (1. - bias_factor[bias] * (1. - ave_corr)));
+}
+
+// Fills score_t and table_t (32768 entries each) and returns ave_path.
+inline int build_align_spec(const float *freq, int16_t *score_t, int16_t *table_t) {
+  int dscore = 0;
+  const int ave_path = align_params(freq, &dscore);
+  fill_trim_tables(0, 0, 0, 0, 1000 - dscore, dscore, score_t, table_t);
   return ave_path;
 }
 

@@ -2,23 +2,38 @@
 // Local_Alignment (lib/align.c:352-1576) with the 32 lanes of a warp
 // updating the diagonals of a wave in parallel.
 //
-// The sequential loop of the reference visits the diagonals of a wave in one
-// order (forward: k = hgh..low, reverse: k = low..hgh) and reads, for k, the
-// previous wave's values at k-1, k and k+1.  Every lane here reads those from
-// the previous wave's buffer (the ring buffers are double-buffered), so the
-// new values equal the reference's.  What the reference accumulates in visit
-// order is rebuilt with warp scans in visit order (lane 0 = first visited):
-//   besta / bestx       running maximum (minimum in reverse): a diagonal is a
-//                       record if it beats the maximum before it
-//   lasta / trim*       the last record that passes the path-average and trim
-//                       table tests
-//   aclip / bclip       the last / extreme diagonal that met a sentinel
-//   pebbles             every lane counts its new trace pebbles, a warp scan
-//                       gives their slots in a global pool (slot numbers only
-//                       name pebbles; the linked chains are the reference's)
-// The rest of a wave step (boundaries, clipping, WAVE_LAG pruning) and the
-// final trace-back are the reference's sequential code, run by all lanes on
-// lane-uniform values.
+// Growth coordinates.  Both directions run one code: the reverse wave is the
+// forward wave under x -> -x, y -> -y.  Diagonals, antidiagonals and trace
+// marks negate with them, the lowest diagonal becomes the highest, and the
+// visit order (forward hgh..low, reverse low..hgh) and the tie rules carry
+// over unchanged; the bases are read from the reversed packed copies.  Only
+// pebbles keep the caller's coordinates, for the trace-back.
+//
+// The sequential loop of the reference visits the diagonals of a wave from
+// high to low and reads, for k, the previous wave's values at k-1, k, k+1.
+// Every lane here reads those from the previous wave, so the new values equal
+// the reference's.  What the reference accumulates in visit order is rebuilt:
+//   besta / bestx       the wave's best; a diagonal is a record if it beats
+//                       every higher diagonal and the best so far, so the
+//                       last record is the highest diagonal with the best
+//   lasta / trim*       the last record that passes the path-average and the
+//                       trim tests, found going back through the records
+//   aclip / bclip       the lowest diagonal that met A's end, the highest
+//                       that met B's
+//   pebbles             slot numbers only name pebbles, so they are taken in
+//                       lane order from a global pool
+//
+// What the loop costs.  A wave step is a few hundred instructions on one warp
+// with a dependent chain through it (neighbours, snake loads, best, prune):
+// with many warps per SM it is bound by instruction fetch, with few by its
+// latency, so both want few instructions in few places.  Hence one copy of
+// the code for both directions (no direction tests inside), and:
+//   * no match count: it is the number of ones among the 61 low bits of the
+//     match history, taken only for a record;
+//   * no trim tables: they (lib/align.c:222-268) ask whether every suffix of
+//     1..30 history bits scores at least 0; lane i tests the suffix of i + 1
+//     bits of the one record's history and a vote answers;
+//   * clips, earlier records and pebble refills are branches off the path.
 #pragma once
 #include <stdint.h>
 #include "align_core.cuh"
@@ -35,10 +50,16 @@ struct PebblePool {
   int64_t cap;
 };
 
+// A diagonal's match history, head pebble and that pebble's mark.
+struct __align__(16) RingCell {
+  uint64_t T;
+  int HA, HM;
+};
+
 struct WarpWork {
-  int *V[2], *M[2], *HA[2], *HM[2];  // HM: mark of pebble HA (marks never change once written)
-  uint64_t *T[2];
-  int *NA;
+  RingCell *C[2];  // waves by diagonal & (vcap - 1), in growth coordinates
+  int *V[2];
+  int *NA;         // next trace mark of each diagonal
   int vcap;
   uint16_t *points;
   int64_t point_cap;
@@ -62,7 +83,7 @@ __device__ __forceinline__ int64_t warp_pebbles(WarpWork &W, int cnt) {
     unsigned long long base = 0;
     if ((threadIdx.x & 31) == 0) base = atomicAdd(W.pool.next, (unsigned long long)want);
     base = __shfl_sync(FULL, base, 0);
-    if ((int64_t)base + want > W.pool.cap) {
+    if ((int64_t)base + want > min(W.pool.cap, (int64_t)I32MAX)) {
       W.err |= ALN_ERR_CELLS;
       return -1;
     }
@@ -84,1529 +105,765 @@ __device__ __forceinline__ int warp_excl_sum(int v, int lane) {
   return x - v;
 }
 
-__device__ __forceinline__ int warp_sum(int v) {
+// The antidiagonal of a diagonal outside the wave: below every real one.
+constexpr int NO_WAVE = -2147483647 - 1;
+constexpr uint32_t HIST_HI = 0x1fffffffu;  // the upper word of the history's 61 bits
+
+// The match count of lib/align.c:663-668: ones among the last 61 history bits.
+__device__ __forceinline__ int hist_ones(uint64_t t) {
+  return __popc((uint32_t)t) + __popc((uint32_t)(t >> 32) & HIST_HI);
+}
+
+// A mismatch and `run` matches shifted into a history.
+__device__ __forceinline__ uint64_t hist_step(uint64_t t, int run) {
+  const int s = min(run, 63);
+  return ((t << 1) << s) | ((1ull << s) - 1);
+}
+
+// Matching bases of 16 * N + 15 loaded ones a (from 2-bit shift sa) and b
+// (from sb): 16 * N bases compared, 16 * N when all match.
+template <int N>
+__device__ __forceinline__ int match_loaded(const uint32_t (&a)[N + 1], int sa, const uint32_t (&b)[N + 1], int sb) {
+  uint32_t w = 0;
+  int o = 0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-  return v;
-}
-
-// exclusive running max (forward) in lane order, seeded with `init`
-__device__ __forceinline__ int warp_excl_max(int v, int lane, int init) {
-  int x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    int y = __shfl_up_sync(FULL, x, o);
-    if (lane >= o) x = max(x, y);
-  }
-  int ex = __shfl_up_sync(FULL, x, 1);
-  if (lane == 0) ex = init;
-  return max(ex, init);
-}
-
-__device__ __forceinline__ int warp_excl_min(int v, int lane, int init) {
-  int x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    int y = __shfl_up_sync(FULL, x, o);
-    if (lane >= o) x = min(x, y);
-  }
-  int ex = __shfl_up_sync(FULL, x, 1);
-  if (lane == 0) ex = init;
-  return min(ex, init);
-}
-
-__device__ __forceinline__ int warp_max(int v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(FULL, v, o));
-  return v;
-}
-__device__ __forceinline__ int warp_min(int v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(FULL, v, o));
-  return v;
-}
-
-// Highest lane with a set bit (the last in visit order), -1 if none.
-__device__ __forceinline__ int last_lane(uint32_t ballot) { return ballot ? 31 - __clz(ballot) : -1; }
-
-// 32 bases of a packed sequence starting at base o.
-__device__ __forceinline__ uint64_t bases32(const uint64_t *p, int o) {
-  int w = o >> 5, sh = (o & 31) << 1;
-  uint64_t v = p[w];
-  return sh ? (v << sh) | (p[w + 1] >> (64 - sh)) : v;
-}
-
-// Matching run of two packed sequences from offsets oa, ob, at most mx bases.
-__device__ __forceinline__ int match_run(const uint64_t *pa, int oa, const uint64_t *pb, int ob, int mx) {
-  int t = 0;
-  while (t < mx) {
-    uint64_t d = bases32(pa, oa + t) ^ bases32(pb, ob + t);
-    int chunk = mx - t < 32 ? mx - t : 32;
-    if (d) {
-      int lead = __clzll(d) >> 1;
-      if (lead < chunk) return t + lead;
+  for (int i = N - 1; i >= 0; i--) {
+    const uint32_t d = __funnelshift_l(a[i + 1], a[i], sa) ^ __funnelshift_l(b[i + 1], b[i], sb);
+    if (i == N - 1 || d != 0) {
+      w = d;
+      o = 32 * i;
     }
-    t += chunk;
   }
-  return mx;
+  return (o + __clz(w)) >> 1;
 }
 
-// Forward snake along diagonal k from a-position x (A[x..], B[x-k..]): the
-// reference's byte loop stops at the first mismatch, or at B's sentinel
-// (B[blen], checked first) or A's (A[alen]).  Starts outside the sequences
-// count as meeting that sequence's sentinel, so no read leaves the buffers.
-__device__ __forceinline__ int snake_fwd(const Seq &A, const Seq &B, int x, int k, int *hitb, int *hita) {
-  int y = x - k;
-  *hitb = *hita = 0;
-  if (y < 0 || y > B.len) {
-    *hitb = 1;
-    return x;
+// The same of words q and r.  The words read may lie past the sequence's
+// copy: the packed buffer has spare words at its end.
+template <int N>
+__device__ __forceinline__ int match_words(const uint32_t *q, int sq, const uint32_t *r, int sr) {
+  uint32_t a[N + 1], b[N + 1];
+#pragma unroll
+  for (int i = 0; i <= N; i++) {
+    a[i] = __ldg(q + i);
+    b[i] = __ldg(r + i);
   }
-  if (x < 0 || x > A.len) {
-    *hita = 1;
-    return x;
-  }
-  int ra = A.len - x, rb = B.len - y;
-  int mx = ra < rb ? ra : rb;
-  int t = match_run(A.pf, x, B.pf, y, mx);
-  if (t == mx) {
-    if (rb <= ra) *hitb = 1;
-    else *hita = 1;
-  }
-  return x + t;
+  return match_loaded<N>(a, sq, b, sr);
 }
 
-// Reverse snake along diagonal k from x: compares A[x-1], A[x-2], .. with
-// B[x-k-1], ..; sentinels A[-1] and B[-1] (read through the reversed copies).
-__device__ __forceinline__ int snake_rev(const Seq &A, const Seq &B, int x, int k, int *hitb, int *hita) {
-  int y = x - k;
-  *hitb = *hita = 0;
-  if (y <= 0 || y >= B.len + 1) {  // B[-1], B[blen] or outside
-    *hitb = 1;
-    return x;
-  }
-  if (x <= 0 || x > A.len) {
-    *hita = 1;
-    return x;
-  }
-  int ra = x, rb = y;
-  int mx = ra < rb ? ra : rb;
-  int t = match_run(A.pr, A.len - x, B.pr, B.len - y, mx);
-  if (t == mx) {
-    if (rb <= ra) *hitb = 1;
-    else *hita = 1;
-  }
-  return x - t;
-}
-
-// The reference shifts one 1 into the match history b per matched base and
-// counts m up while b's PATH_TOP bit is clear (lib/align.c:663-668): the
-// closed form for a run of r bases.
-__device__ __forceinline__ void history_run(uint64_t &b, int &m, int r) {
-  if (r <= 0) return;
-  int L = r < 61 ? r : 61;
-  uint64_t mask = ((1ull << L) - 1) << (61 - L);
-  m += L - __popcll(b & mask);
-  b = r >= 64 ? ~0ull : ((b << r) | ((1ull << r) - 1));
-}
-
-// ---------------------------------------------------------------------------
-// One wave of forward_wave / reverse_wave after its boundary diagonals are
-// set: every diagonal of [low, hgh] computed from the previous wave's buffer
-// (cur) into the other buffer, in the reference's visit order (forward:
-// k = hgh..low, reverse: k = low..hgh).
-//
-// Each lane takes up to WJ consecutive diagonals of the visit order (lane 0
-// the first), so a wave of up to 32*WJ diagonals is one pass: the lane's
-// loads and snakes are independent and run side by side, and the visit-order
-// scans are a lane-local pass plus one warp scan.  Wider waves take several
-// passes, carried in visit order.
-// ---------------------------------------------------------------------------
-constexpr int WJ = 4;
-
-// What a one-pass sweep leaves in registers for wave_prune.
-struct WaveSlice {
-  int c[WJ];
-  int k0;       // the lane's first diagonal
-  int nact;     // its diagonals
-  bool single;  // one pass covered [low, hgh]
+// One extension (forward_wave or reverse_wave): its lane-uniform inputs and
+// state, in growth coordinates.  Base i of a sequence in growth order is at
+// x + off, and lim - x bases remain from x.
+struct Wave {
+  const uint32_t *pa, *pb;
+  int offA, offB, limA, limB;
+  int minp, maxp;
+  int tspace, ave_path, dscore;
+  int sg;    // 1 forward, -1 reverse
+  int low, hgh, dif, cur;
+  int besta, bestx, lasta, trima, trimx, trimd, trimha;
+  int more, morem, morea, morex, mored, moreha;
 };
 
-// Lockstep snakes of a lane's diagonals: forward along A.pf / B.pf from
-// (x, x-k), reverse along A.pr / B.pr from (A.len-x, B.len-y); stops and
-// sentinel hits as snake_fwd / snake_rev.
-template <int J>
-__device__ __forceinline__ void lane_snakes(const bool FWD, const Seq &A, const Seq &B, int nact, const int *k, int *x,
-                                            int *run, int *hb, int *hA) {
-  int oa[J], ob[J], mx[J], t[J];
-  bool go[J];
-#pragma unroll
-  for (int j = 0; j < J; j++) {
-    go[j] = false;
-    hb[j] = hA[j] = 0;
-    t[j] = 0;
-    mx[j] = 0;
-    oa[j] = ob[j] = 0;
-    if (j < nact) {
-      int xx = x[j], y = xx - k[j];
-      if (FWD) {
-        if (y < 0 || y > B.len) hb[j] = 1;
-        else if (xx < 0 || xx > A.len) hA[j] = 1;
-        else {
-          int ra = A.len - xx, rb = B.len - y;
-          mx[j] = ra < rb ? ra : rb;
-          oa[j] = xx;
-          ob[j] = y;
-          go[j] = mx[j] > 0;
-        }
-      } else {
-        if (y <= 0 || y >= B.len + 1) hb[j] = 1;
-        else if (xx <= 0 || xx > A.len) hA[j] = 1;
-        else {
-          mx[j] = xx < y ? xx : y;
-          oa[j] = A.len - xx;
-          ob[j] = B.len - y;
-          go[j] = mx[j] > 0;
-        }
-      }
-    }
+// Snake along diagonal k from x in rounds of 16 * N bases: stops at the first
+// mismatch or a sequence's end.  Where x is outside the sequences
+// (`go` false) it does not move, and no read leaves the buffers.
+template <int N>
+__device__ __forceinline__ int snake(const Wave &E, int x, int k, bool act, int mx, bool &go) {
+  const int ia = x + E.offA, ib = x - k + E.offB;
+  go = act && (mx | ia | ib) >= 0;
+  int run = 0;
+  if (go) {
+    int r;
+    do {
+      const int qa = ia + run, qb = ib + run;
+      r = match_words<N>(E.pa + (qa >> 4), (qa & 15) << 1, E.pb + (qb >> 4), (qb & 15) << 1);
+      run += r;
+    } while (r == 16 * N && run < mx);
+    run = min(run, mx);
   }
-  const uint64_t *pa = FWD ? A.pf : A.pr, *pb = FWD ? B.pf : B.pr;
-  bool any = false;
-#pragma unroll
-  for (int j = 0; j < J; j++) any |= go[j];
-  while (any) {
-    any = false;
-#pragma unroll
-    for (int j = 0; j < J; j++) {
-      if (go[j]) {
-        uint64_t d = bases32(pa, oa[j] + t[j]) ^ bases32(pb, ob[j] + t[j]);
-        int chunk = mx[j] - t[j] < 32 ? mx[j] - t[j] : 32;
-        int lead = d ? (__clzll(d) >> 1) : 32;
-        if (lead < chunk) {
-          t[j] += lead;
-          go[j] = false;
-        } else {
-          t[j] += chunk;
-          go[j] = t[j] < mx[j];
-        }
-        any |= go[j];
-      }
-    }
+  return run;
+}
+
+// Which end a snake that could go no further met: true B's (checked first by
+// the reference's byte loop), false A's.  x is the snake's start; one that
+// starts outside the sequences counts as meeting an end, B's if y is outside.
+__device__ __forceinline__ bool met_b(const Wave &E, int x, int k, bool go) {
+  const int ra = E.limA - x, rb = E.limB - x + k;
+  return go ? rb <= ra : (x - k + E.offB < 0 || rb < (E.sg > 0 ? 0 : 1));
+}
+
+// The trim test on a record's history (New_Align_Spec's tables,
+// lib/align.c:222-268, with match score 1000 - dscore and mismatch -dscore):
+// every suffix of 1..30 bits scores at least 0.  The tables cut the 30 bits
+// at TRIM_LEN: TABLE[low 15] >= 0 is the suffixes up to 15 bits,
+// TABLE[high 15] + SCORE[low 15] >= 0 the longer ones.
+struct TrimTest {
+  uint32_t mask;  // this lane's suffix
+  int need;       // matches it needs
+  __device__ __forceinline__ TrimTest(int dscore) {
+    const int lane = threadIdx.x & 31;
+    mask = lane < 2 * TRIM_LEN ? (2u << lane) - 1u : 0u;
+    need = lane < 2 * TRIM_LEN ? ((lane + 1) * dscore + 999) / 1000 : 0;
   }
-#pragma unroll
-  for (int j = 0; j < J; j++) {
-    if (j < nact && !hb[j] && !hA[j]) {
-      if (t[j] == mx[j]) {
-        int xx = x[j], y = xx - k[j];
-        int ra = FWD ? A.len - xx : xx, rb = FWD ? B.len - y : y;
-        if (rb <= ra) hb[j] = 1;
-        else hA[j] = 1;
-      }
-      x[j] = FWD ? x[j] + t[j] : x[j] - t[j];
+  __device__ __forceinline__ bool operator()(uint64_t t) const {
+    return __all_sync(FULL, __popc((uint32_t)t & mask) >= need);
+  }
+};
+
+// The trace marks the lanes' snakes passed: one pebble each unless the path
+// has it already (hm).  next / end: the warp's pebble chunk.  Returns false
+// when the pool is full.
+__device__ __forceinline__ bool drop_pebbles(const WarpWork &W, const Wave &E, bool act, int k, int x, int dif, int &ha,
+                                             int &hm, int &nak, int &next, int &end) {
+  const int lane = threadIdx.x & 31;
+  bool cross = act && x >= nak;
+  do {
+    const bool mk = cross && hm < nak;
+    const uint32_t mb = __ballot_sync(FULL, mk);
+    const int cnt = __popc(mb);
+    if (next + cnt > end) {
+      unsigned long long base = 0;
+      if (lane == 0) base = atomicAdd(W.pool.next, (unsigned long long)PEBBLE_CHUNK);
+      base = __shfl_sync(FULL, base, 0);
+      // pebble numbers are int
+      if ((int64_t)base + PEBBLE_CHUNK > min(W.pool.cap, (int64_t)I32MAX)) return false;
+      next = (int)base;
+      end = next + PEBBLE_CHUNK;
     }
-    run[j] = t[j];
+    if (mk) {
+      const int s = next + __popc(mb & ((1u << lane) - 1u));
+      *reinterpret_cast<int4 *>(W.pool.cells + s) = make_int4(ha, E.sg * k, dif, E.sg * nak);
+      ha = s;
+      hm = nak;
+    }
+    next += cnt;
+    if (cross) nak += E.tspace;
+    cross = cross && x >= nak;
+  } while (__any_sync(FULL, cross));
+  return true;
+}
+
+// The records before the one on diagonal kr (the higher diagonals; `passed`:
+// the later ones already gave lasta), back to the last that also passes the
+// trim test.  carry: the best before the wave.
+__device__ __forceinline__ void earlier_records(Wave &S, int &lasta, const TrimTest &trim, bool act, int k, int c,
+                                                uint64_t b, int ha, int dif, int carry, int kr, bool passed) {
+  const bool good = act && c > carry && hist_ones(b) >= S.ave_path;
+  while (__any_sync(FULL, good && k > kr)) {  // else none of them passes
+    const bool cand = act && k > kr && c > carry;
+    const int rc = __reduce_max_sync(FULL, cand ? c : NO_WAVE);
+    kr = __reduce_max_sync(FULL, cand && c == rc ? k : NO_WAVE);
+    const int L = __ffs(__ballot_sync(FULL, act && k == kr)) - 1;
+    const uint64_t t = __shfl_sync(FULL, b, L);
+    if (hist_ones(t) < S.ave_path) continue;
+    if (!passed) lasta = rc;
+    passed = true;
+    if (trim(t)) {
+      S.trima = rc;
+      S.trimx = (rc + kr) >> 1;
+      S.trimd = dif;
+      S.trimha = __shfl_sync(FULL, ha, L);
+      return;
+    }
   }
 }
 
-// 32 bases of a packed sequence from a 2-bit shift sh (0..62) into words
-// (w0, w1): w0 << sh with w1's top bits shifted in, no branch on sh == 0.
-__device__ __forceinline__ uint64_t join32(uint64_t w0, uint64_t w1, int sh) {
-  return (w0 << sh) | ((w1 >> 1) >> (63 - sh));
+// The records of one pass over up to 32 diagonals (lane's diagonal k at c
+// with history b), none of them above the pass: the wave's best, and the last
+// record that passes the path-average test and the last that also passes the
+// trim test.
+__device__ __forceinline__ void take_records(Wave &S, int &besta, int &lasta, const TrimTest &trim, bool act, int k,
+                                             int c, uint64_t b, int ha, int dif) {
+  const int rc = __reduce_max_sync(FULL, act ? c : NO_WAVE);
+  if (rc <= besta) return;
+  const int kr = __reduce_max_sync(FULL, act && c == rc ? k : NO_WAVE);
+  const int L = __ffs(__ballot_sync(FULL, act && k == kr)) - 1;
+  const uint64_t t = __shfl_sync(FULL, b, L);
+  const bool pass = hist_ones(t) >= S.ave_path, tip = trim(t);
+  S.bestx = (rc + kr) >> 1;
+  if (pass) lasta = rc;
+  if (pass && tip) {
+    S.trima = rc;
+    S.trimx = (rc + kr) >> 1;
+    S.trimd = dif;
+    S.trimha = __shfl_sync(FULL, ha, L);
+  } else
+    earlier_records(S, lasta, trim, act, k, c, b, ha, dif, besta, kr, pass);
+  besta = rc;
 }
 
-// The snake of one diagonal (the one-diagonal-per-lane case of
-// lane_snakes): the same stops and sentinel hits, 64 bases per round from
-// three words of each packed sequence loaded together.  The third word may
-// lie past this sequence's copy (its bases are beyond mx and never count);
-// the packed buffer has spare words at its end.
-__device__ __forceinline__ void snake1(const bool FWD, const Seq &A, const Seq &B, bool act, int k, int &x, int &run,
-                                       int &hb, int &hA) {
-  hb = hA = 0;
-  run = 0;
-  if (!act) return;
-  const int y = x - k;
-  int oa, ob, mx;
-  const uint64_t *pa, *pb;
-  if (FWD) {
-    if (y < 0 || y > B.len) {
-      hb = 1;
-      return;
-    }
-    if (x < 0 || x > A.len) {
-      hA = 1;
-      return;
-    }
-    const int ra = A.len - x, rb = B.len - y;
-    mx = ra < rb ? ra : rb;
-    oa = x;
-    ob = y;
-    pa = A.pf;
-    pb = B.pf;
-  } else {
-    if (y <= 0 || y >= B.len + 1) {
-      hb = 1;
-      return;
-    }
-    if (x <= 0 || x > A.len) {
-      hA = 1;
-      return;
-    }
-    mx = x < y ? x : y;
-    oa = A.len - x;
-    ob = B.len - y;
-    pa = A.pr;
-    pb = B.pr;
+// A path that met a sequence's end on a clipped diagonal.
+__device__ __forceinline__ void note_end(Wave &S, int kc, uint64_t t, int c, int ha, int dif) {
+  const int m = hist_ones(t);
+  if (S.morem <= m) {
+    S.morem = m;
+    S.morea = c;
+    S.morex = (c + kc) >> 1;
+    S.mored = dif;
+    S.moreha = ha;
   }
-  int t = 0;
-  while (t < mx) {
-    const int qa = oa + t, qb = ob + t;
-    const uint64_t *ua = pa + (qa >> 5), *ub = pb + (qb >> 5);
-    const int sa = (qa & 31) << 1, sb = (qb & 31) << 1;
-    const uint64_t a0 = ua[0], a1 = ua[1], a2 = ua[2], b0 = ub[0], b1 = ub[1], b2 = ub[2];
-    const uint64_t d0 = join32(a0, a1, sa) ^ join32(b0, b1, sb);
-    const uint64_t d1 = join32(a1, a2, sa) ^ join32(b1, b2, sb);
-    const int lead = d0 ? (__clzll(d0) >> 1) : 32 + (d1 ? (__clzll(d1) >> 1) : 32);
-    const int chunk = mx - t < 64 ? mx - t : 64;
-    if (lead < chunk) {
-      t += lead;
+}
+
+// Whether the furthest path can still grow (neither sequence's end reached).
+__device__ __forceinline__ int can_grow(const Wave &S, int besta) {
+  return S.limB - besta + S.bestx != 0 && S.limA - S.bestx != 0 ? 1 : 0;
+}
+
+// ---------------------------------------------------------------------------
+// Narrow waves, at most 31 diagonals: diagonal k lives in lane k mod 32, its
+// state in registers, the previous wave's neighbours come by shuffle.  The
+// free lane between the window's ends (like every lane outside it) holds
+// NO_WAVE, so the neighbours of the ends need no range test.
+//
+// A long alignment is one warp's chain of these steps, so the step is laid
+// out along its critical path: neighbours -> start points -> sequence words
+// -> snakes -> the wave's best -> the next window.  The wave's pebbles and
+// its record's tests are not on it: they are settled in the next step, while
+// that step's sequence words are on their way, before the loop's end
+// conditions are tested and anything of the new wave is kept.
+//
+// Runs until the loop ends, the next wave does not fit, or the wave count
+// reaches `stop`.  Returns 1 when the pebble pool is full.
+// ---------------------------------------------------------------------------
+constexpr int NARROW = 31;
+constexpr int PAST_MAX = (1 << 26) - 1;  // a best further past than this takes the general record search
+
+__device__ __forceinline__ int narrow_waves(WarpWork &W, Wave &io, int stop) {
+  const int lane = threadIdx.x & 31;
+  const int lup = (lane + 1) & 31, ldn = (lane - 1) & 31;
+  Wave S = io;
+  const TrimTest trim(S.dscore);
+  const int vmask = W.vcap - 1;
+  int next = (int)W.chunk_next, end = (int)W.chunk_end;
+  int ncells = 0;
+  int low = S.low, hgh = S.hgh, dif = S.dif, besta = S.besta, lasta = S.lasta;
+
+  // the last wave: lane's diagonal kw (if live), its furthest x, what came with it
+  int V = NO_WAVE, HA = -1, HM = 0, NA = 0, X = 0, kw = low + ((lane - low) & 31);
+  bool live = false;
+  uint64_t T = 0;
+  // its record, if any: the best rc on diagonal kr, past the best before it
+  int rc = besta, kr = 0, carry = besta;
+  if (kw <= hgh) {
+    const RingCell c = W.C[S.cur][kw & vmask];
+    V = W.V[S.cur][kw & vmask];
+    NA = W.NA[kw & vmask];
+    T = c.T;
+    HA = c.HA;
+    HM = c.HM;
+  }
+  // the last wave's pebbles and record; once done, doing it again changes nothing
+  auto settle = [&]() {
+    if (!drop_pebbles(W, S, live, kw, X, dif, HA, HM, NA, next, end)) return false;
+    const int L = kr & 31;
+    const uint64_t t = __shfl_sync(FULL, T, L);
+    const int hr = __shfl_sync(FULL, HA, L);
+    const bool tip = trim(t), rec = rc > carry, pass = rec && hist_ones(t) >= S.ave_path;
+    if (rec) S.bestx = (rc + kr) >> 1;
+    if (pass) lasta = rc;
+    if (pass && tip) {
+      S.trima = rc;
+      S.trimx = (rc + kr) >> 1;
+      S.trimd = dif;
+      S.trimha = hr;
+    } else if (rec)
+      earlier_records(S, lasta, trim, live, kw, (X << 1) - kw, T, HA, dif, carry, kr, pass);
+    carry = rc;
+    return true;
+  };
+  bool full = false;
+  while (true) {
+    const int nlow = max(low - 1, S.minp), nhgh = min(hgh + 1, S.maxp);  // a window end is never past its border
+    const int wide = nhgh - nlow;
+    const int p = (lane - nlow) & 31, k = nlow + p;
+    const bool act = p <= wide;
+
+    // the furthest point each diagonal starts from
+    const int vup = __shfl_sync(FULL, V, lup), vdn = __shfl_sync(FULL, V, ldn);
+    const bool up = vup > max(V, vdn), dn = !up && vdn > V;
+    const int x = ((up ? vup + 1 : (dn ? vdn + 1 : V + 2)) + k) >> 1;
+    const int mx = min(S.limA - x, S.limB - x + k);
+    const int ia = x + S.offA, ib = x - k + S.offB;
+    const bool go = act && (mx | ia | ib) >= 0;
+    uint32_t a[5], b[5];
+    {
+      const uint32_t *qa = S.pa + (go ? ia >> 4 : 0), *qb = S.pb + (go ? ib >> 4 : 0);
+#pragma unroll
+      for (int i = 0; i < 5; i++) {
+        a[i] = __ldg(qa + i);
+        b[i] = __ldg(qb + i);
+      }
+    }
+
+    if (!settle()) {
+      full = true;
       break;
     }
-    t += chunk;
-  }
-  if (t == mx) {
-    const int ra = FWD ? A.len - x : x, rb = FWD ? B.len - y : y;
-    if (rb <= ra) hb = 1;
-    else hA = 1;
-  }
-  x = FWD ? x + t : x - t;
-  run = t;
-}
+    if (!(S.more && lasta >= besta - TRIM_MLAG && low <= hgh && wide < NARROW && dif < stop)) break;
+    dif += 1;
+    ncells += wide + 1;
 
-// v[j] for a per-lane index j < J, without local memory
-template <int J>
-__device__ __forceinline__ int pick(const int *v, int j) {
-  int r = v[0];
-#pragma unroll
-  for (int q = 1; q < J; q++)
-    if (j == q) r = v[q];
-  return r;
-}
+    // what comes with the start points; a new end diagonal copies its
+    // neighbour's trace mark
+    const int sl = up ? lup : (dn ? ldn : lane);
+    const int nlo = __shfl_sync(FULL, NA, low & 31), nhi = __shfl_sync(FULL, NA, hgh & 31);
+    HA = __shfl_sync(FULL, HA, sl);
+    HM = __shfl_sync(FULL, HM, sl);
+    T = __shfl_sync(FULL, T, sl);
+    NA = k < low ? nlo : (k > hgh ? nhi : NA);
 
-// One pass of a wave over visit positions [p0, p0 + 32*J): lane l takes
-// positions p0 + l*J .. p0 + l*J + J-1.  carry is the running best before
-// the pass.
-template <int J>
-__device__ __forceinline__ int wave_pass(const bool FWD, WarpWork &W, const AlignSpec &spec, const Seq &A, const Seq &B,
-                                         int low, int hgh, int w, int p0, int dif, int cur, int &carry, int &besta,
-                                         int &bestx, int &lasta, int &trima, int &trimx, int &trimd, int &trimha,
-                                         int &more, int &aclip, int &bclip, WaveSlice &WS) {
-  const int lane = threadIdx.x & 31;
-  const int vmask = W.vcap - 1;
-  const int tspace = spec.trace_space;
-  const int PATH_AVE = spec.ave_path;
-  const int16_t *SCORE = spec.score;
-  const int16_t *TABLE = spec.table;
-  const int *Vo = W.V[cur], *Mo = W.M[cur], *HAo = W.HA[cur], *HMo = W.HM[cur];
-  const uint64_t *To = W.T[cur];
-  int *Vn = W.V[cur ^ 1], *Mn = W.M[cur ^ 1], *HAn = W.HA[cur ^ 1], *HMn = W.HM[cur ^ 1];
-  uint64_t *Tn = W.T[cur ^ 1];
-  int *NA = W.NA;
-  Pebble *cells = W.pool.cells;
-  const int pl = p0 + lane * J;
-  int nact = w - pl;
-  if (nact > J) nact = J;
-  if (nact < 0) nact = 0;
-  const int k0 = FWD ? hgh - pl : low + pl;
-  int k[J], c[J], x[J], m[J], ha[J], hm[J], nak[J], run[J], hb[J], hA[J], npb[J];
-  uint64_t b[J];
-  // previous wave around the lane's diagonals: forward nv[i] = V[k0+1-i],
-  // reverse nv[i] = V[k0-1+i]
-  int nv[J + 2];
-#pragma unroll
-  for (int i = 0; i < J + 2; i++) {
-    nv[i] = 0;
-    if (nact > 0 && i < nact + 2) nv[i] = Vo[(FWD ? k0 + 1 - i : k0 - 1 + i) & vmask];
-  }
-#pragma unroll
-  for (int j = 0; j < J; j++) {
-    k[j] = FWD ? k0 - j : k0 + j;
-    c[j] = x[j] = m[j] = hm[j] = nak[j] = npb[j] = 0;
-    ha[j] = -1;
-    b[j] = 0;
-    if (j < nact) {
-      int src, sk;
-      if (FWD) {
-        int ap = nv[j], ac = nv[j + 1], am = nv[j + 2];
-        if (ac < am) src = (am < ap) ? 1 : -1;
-        else src = (ac < ap) ? 1 : 0;
-        c[j] = src == 1 ? ap + 1 : (src == -1 ? am + 1 : ac + 2);
-      } else {
-        int am = nv[j], ac = nv[j + 1], ap = nv[j + 2];
-        if (ac > ap) src = (ap > am) ? -1 : 1;
-        else src = (ac > am) ? -1 : 0;
-        c[j] = src == -1 ? am - 1 : (src == 1 ? ap - 1 : ac - 2);
+    // snakes, 64 bases per round
+    int run = 0;
+    if (go) {
+      run = match_loaded<4>(a, (ia & 15) << 1, b, (ib & 15) << 1);
+      for (int r = run; r == 64 && run < mx; run += r) {
+        const int qa = ia + run, qb = ib + run;
+        r = match_words<4>(S.pa + (qa >> 4), (qa & 15) << 1, S.pb + (qb >> 4), (qb & 15) << 1);
       }
-      sk = k[j] + src;
-      bool dflt = FWD ? (src == 1 && k[j] == hgh) : (src == -1 && k[j] == low);
-      if (dflt) {
-        m[j] = PATH_LEN;
-        b[j] = PATH_INT;
-      } else {
-        int si = sk & vmask;
-        m[j] = Mo[si];
-        b[j] = To[si];
-        ha[j] = HAo[si];
-        hm[j] = HMo[si];
-      }
-      nak[j] = NA[k[j] & vmask];
-      if ((b[j] & PATH_TOP) != 0) m[j] -= 1;
-      b[j] <<= 1;
-      x[j] = (c[j] + k[j]) >> 1;
+      run = min(run, mx);
     }
-  }
-  lane_snakes<J>(FWD, A, B, nact, k, x, run, hb, hA);
-  int npl = 0;
-#pragma unroll
-  for (int j = 0; j < J; j++) {
-    if (j < nact) {
-      history_run(b[j], m[j], run[j]);
-      c[j] = (x[j] << 1) - k[j];
-      int hq = hm[j];
-      if (FWD) {
-        for (int q = nak[j]; x[j] >= q; q += tspace)
-          if (hq < q) {
-            npb[j]++;
-            hq = q;
-          }
-      } else {
-        for (int q = nak[j]; x[j] <= q; q -= tspace)
-          if (hq > q) {
-            npb[j]++;
-            hq = q;
-          }
+    const uint32_t hits = __ballot_sync(FULL, act && (!go || run == mx));
+    X = x + run;
+    const int c = (X << 1) - k;
+    // the wave's best: how far a diagonal is past the best so far, then the
+    // highest such diagonal, in one reduction
+    const int past = min(max(c - besta, 0), PAST_MAX);
+    const int key = __reduce_max_sync(FULL, act ? (past << 5) + p : 0);
+    T = hist_step(T, run);
+    live = act;
+    kw = k;
+    carry = besta;
+    rc = besta + (key >> 5);
+    kr = nlow + (key & 31);
+    low = nlow;
+    hgh = nhgh;
+    if (hits || key >= (PAST_MAX << 5)) {
+      if (key >= (PAST_MAX << 5)) {
+        rc = __reduce_max_sync(FULL, act ? c : NO_WAVE);
+        kr = __reduce_max_sync(FULL, act && c == rc ? k : NO_WAVE);
       }
-      npl += npb[j];
-    }
-  }
-  // pebble slots in visit order
-  int off, tot;
-  if (__ballot_sync(FULL, npl > 1) == 0) {
-    uint32_t one = __ballot_sync(FULL, npl == 1);
-    off = __popc(one & ((1u << lane) - 1));
-    tot = __popc(one);
-  } else {
-    off = warp_excl_sum(npl, lane);
-    tot = warp_sum(npl);
-  }
-  int64_t pb0 = warp_pebbles(W, tot);
-  if (pb0 < 0) return 1;
-  int64_t s = pb0 + off;
-#pragma unroll
-  for (int j = 0; j < J; j++) {
-    if (j < nact) {
-      if (FWD) {
-        while (x[j] >= nak[j]) {
-          if (hm[j] < nak[j]) {
-            cells[s] = {ha[j], k[j], dif, nak[j]};
-            ha[j] = (int)s;
-            hm[j] = nak[j];
-            s += 1;
-          }
-          nak[j] += tspace;
+      if (hits) {
+        // snakes that reached a sequence's end clip the window
+        if (!settle()) {
+          full = true;
+          break;
         }
-      } else {
-        while (x[j] <= nak[j]) {
-          if (hm[j] > nak[j]) {
-            cells[s] = {ha[j], k[j], dif, nak[j]};
-            ha[j] = (int)s;
-            hm[j] = nak[j];
-            s += 1;
-          }
-          nak[j] -= tspace;
+        const bool hit = hits >> lane & 1, hb = met_b(S, x, k, go);
+        const int ka = __reduce_min_sync(FULL, hit && !hb ? k : I32MAX);
+        const int kb = __reduce_max_sync(FULL, hit && hb ? k : NO_WAVE);
+        S.more = can_grow(S, rc);
+        if (ka != I32MAX) {
+          hgh = ka - 1;
+          note_end(S, ka, __shfl_sync(FULL, T, ka & 31), __shfl_sync(FULL, c, ka & 31),
+                   __shfl_sync(FULL, HA, ka & 31), dif);
         }
-      }
-      int vi = k[j] & vmask;
-      NA[vi] = nak[j];
-      Vn[vi] = c[j];
-      Tn[vi] = b[j];
-      Mn[vi] = m[j];
-      HAn[vi] = ha[j];
-      HMn[vi] = hm[j];
-    }
-  }
-  // clips: bclip from the first visited diagonal that met B's end, aclip
-  // from the last visited that met A's end
-  int fb = -1, la = -1;
-#pragma unroll
-  for (int j = J - 1; j >= 0; j--)
-    if (j < nact && hb[j]) fb = j;
-#pragma unroll
-  for (int j = 0; j < J; j++)
-    if (j < nact && hA[j]) la = j;
-  uint32_t bbl = __ballot_sync(FULL, fb >= 0), bal = __ballot_sync(FULL, la >= 0);
-  if (bbl) {
-    more = 0;
-    int L = __ffs(bbl) - 1;
-    int kk = __shfl_sync(FULL, FWD ? k0 - fb : k0 + fb, L);
-    if (FWD ? (bclip < kk) : (bclip > kk)) bclip = kk;
-  }
-  if (bal) {
-    more = 0;
-    int L = last_lane(bal);
-    aclip = __shfl_sync(FULL, FWD ? k0 - la : k0 + la, L);
-  }
-  // records: c beyond the running best (max forward, min reverse) in visit order
-  int agg = FWD ? -2147483647 : 2147483647;
-#pragma unroll
-  for (int j = 0; j < J; j++)
-    if (j < nact) agg = FWD ? max(agg, c[j]) : min(agg, c[j]);
-  int pm = FWD ? warp_excl_max(agg, lane, carry) : warp_excl_min(agg, lane, carry);
-  int lr = -1, lp = -1, lt = -1;
-#pragma unroll
-  for (int j = 0; j < J; j++) {
-    if (j < nact) {
-      bool rec = FWD ? c[j] > pm : c[j] < pm;
-      if (rec) {
-        pm = c[j];
-        lr = j;
-        if (m[j] >= PATH_AVE) {
-          lp = j;
-          if (TABLE[b[j] & TRIM_MASK] >= 0 && TABLE[(b[j] >> TRIM_LEN) & TRIM_MASK] + SCORE[b[j] & TRIM_MASK] >= 0)
-            lt = j;
+        if (kb != NO_WAVE) {
+          low = kb + 1;
+          note_end(S, kb, __shfl_sync(FULL, T, kb & 31), __shfl_sync(FULL, c, kb & 31),
+                   __shfl_sync(FULL, HA, kb & 31), dif);
         }
       }
     }
+    besta = rc;
+    // WAVE_LAG pruning from either end, between the clipped ends
+    const uint32_t keep = __ballot_sync(FULL, k >= low && k <= hgh && c >= besta - WAVE_LAG);
+    const uint32_t kept = __funnelshift_r(keep, keep, nlow & 31);  // bit q: diagonal nlow + q
+    low = nlow + __clz(__brev(kept));                              // none: low = nlow + 32, above hgh = nlow - 1
+    hgh = nlow + 31 - __clz(kept);
+    V = k >= low && k <= hgh ? c : NO_WAVE;
   }
-  uint32_t rb = __ballot_sync(FULL, lr >= 0);
-  if (rb) {
-    int L = last_lane(rb);
-    carry = __shfl_sync(FULL, pick<J>(c, lr), L);
-    besta = carry;
-    bestx = __shfl_sync(FULL, pick<J>(x, lr), L);
-    uint32_t pab = __ballot_sync(FULL, lp >= 0);
-    if (pab) {
-      lasta = __shfl_sync(FULL, pick<J>(c, lp), last_lane(pab));
-      uint32_t trb = __ballot_sync(FULL, lt >= 0);
-      if (trb) {
-        int T2 = last_lane(trb);
-        trima = __shfl_sync(FULL, pick<J>(c, lt), T2);
-        trimx = __shfl_sync(FULL, pick<J>(x, lt), T2);
-        trimd = dif;
-        trimha = __shfl_sync(FULL, pick<J>(ha, lt), T2);
-      }
-    }
+  W.waves += dif - S.dif;
+  W.cells += ncells;
+  W.chunk_next = next;
+  W.chunk_end = end;
+  if (full) {
+    W.err |= ALN_ERR_CELLS;
+    return 1;
   }
-  if (WS.single) {
-#pragma unroll
-    for (int j = 0; j < J; j++) WS.c[j] = c[j];
-    WS.k0 = k0;
-    WS.nact = nact;
+  // (the diagonals of [low, hgh] are where they were in the last wave)
+  if (kw >= low && kw <= hgh) {
+    W.V[S.cur][kw & vmask] = V;
+    W.C[S.cur][kw & vmask] = RingCell{T, HA, HM};
+    W.NA[kw & vmask] = NA;
   }
-  return 0;
-}
-
-// The whole wave: one pass of single diagonals when it is at most 32 wide,
-// else passes of WJ diagonals per lane.
-__device__ __forceinline__ int wave_sweep(const bool FWD, WarpWork &W, const AlignSpec &spec, const Seq &A,
-                                          const Seq &B, int low, int hgh, int dif, int cur, int &besta, int &bestx,
-                                          int &lasta, int &trima, int &trimx, int &trimd, int &trimha, int &more,
-                                          int &aclip, int &bclip, WaveSlice &WS) {
-  const int w = hgh - low + 1;
-  WS.single = w <= 32 * WJ;
-  WS.nact = 0;
-  WS.k0 = 0;
-  int carry = besta;
-  if (w <= 32)
-    return wave_pass<1>(FWD, W, spec, A, B, low, hgh, w, 0, dif, cur, carry, besta, bestx, lasta, trima, trimx,
-                             trimd, trimha, more, aclip, bclip, WS);
-  for (int p0 = 0; p0 < w; p0 += 32 * WJ)
-    if (wave_pass<WJ>(FWD, W, spec, A, B, low, hgh, w, p0, dif, cur, carry, besta, bestx, lasta, trima, trimx,
-                           trimd, trimha, more, aclip, bclip, WS))
-      return 1;
-  return 0;
-}
-
-// WAVE_LAG pruning of [low, hgh] (already clipped) on the wave just made:
-// hgh becomes the largest and low the smallest diagonal within WAVE_LAG of
-// the best antidiagonal, or hgh = low - 1 when none is (the reference's
-// loop from either end).  V is the new wave's buffer.
-__device__ __forceinline__ void wave_prune(const bool FWD, const WarpWork &W, const int *V, int besta, int &low,
-                                           int &hgh, const WaveSlice &WS) {
-  if (hgh < low) return;
-  const int vmask = W.vcap - 1;
-  const int n = FWD ? besta - WAVE_LAG : besta + WAVE_LAG;
-  if (WS.single) {
-    int kmax = -2147483647, kmin = 2147483647;
-#pragma unroll
-    for (int j = 0; j < WJ; j++) {
-      int k = FWD ? WS.k0 - j : WS.k0 + j;
-      if (j < WS.nact && k >= low && k <= hgh && (FWD ? WS.c[j] >= n : WS.c[j] <= n)) {
-        kmax = max(kmax, k);
-        kmin = min(kmin, k);
-      }
-    }
-    kmax = __reduce_max_sync(FULL, kmax);
-    kmin = __reduce_min_sync(FULL, kmin);
-    if (kmin <= kmax) {
-      hgh = kmax;
-      low = kmin;
-    } else
-      hgh = low - 1;
-    return;
-  }
-  if (FWD) {
-    while (hgh >= low)
-      if (V[hgh & vmask] < n)
-        hgh -= 1;
-      else {
-        while (V[low & vmask] < n) low += 1;
-        break;
-      }
-  } else {
-    while (hgh >= low)
-      if (V[hgh & vmask] > n)
-        hgh -= 1;
-      else {
-        while (V[low & vmask] > n) low += 1;
-        break;
-      }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Register-resident waves.  While a wave is at most 32 diagonals wide (and
-// the previous one was not empty) diagonal k lives in lane k mod 32: its
-// antidiagonal, match count, match history, head pebble, head mark and next
-// trace mark stay in registers, the previous wave's neighbours come by
-// shuffle, and the visit-order questions (pebble slots, records, clips,
-// pruning) are answered with ballots rotated into visit order and warp
-// reductions.  NA is also written through to memory; the other fields go to
-// the memory ring only when a wider wave hands over to wave_sweep.
-// ---------------------------------------------------------------------------
-struct RegWave {
-  int V, M, HA, HM, NA;
-  uint64_t T;
-};
-
-// What a register wave needs of WarpWork, held in the wave loop's registers
-// (WarpWork itself lives in addressable memory).
-struct RegCtx {
-  int vmask;
-  int *NA;
-  Pebble *cells;
-  unsigned long long *pool_next;
-  int64_t pool_cap;
-  int64_t chunk_next, chunk_end;  // the warp's current pebble chunk
-  int err;
-};
-
-// warp_pebbles on a RegCtx.
-__device__ __forceinline__ int64_t reg_pebbles(RegCtx &X, int cnt) {
-  if (cnt == 0) return 0;
-  if (X.chunk_next + cnt > X.chunk_end) {
-    int64_t want = cnt > PEBBLE_CHUNK ? cnt : PEBBLE_CHUNK;
-    unsigned long long base = 0;
-    if ((threadIdx.x & 31) == 0) base = atomicAdd(X.pool_next, (unsigned long long)want);
-    base = __shfl_sync(FULL, base, 0);
-    if ((int64_t)base + want > X.pool_cap) {
-      X.err |= ALN_ERR_CELLS;
-      return -1;
-    }
-    X.chunk_next = (int64_t)base;
-    X.chunk_end = (int64_t)base + want;
-  }
-  int64_t s = X.chunk_next;
-  X.chunk_next += cnt;
-  return s;
-}
-
-// Visit position of lane l's diagonal (forward: hgh first, reverse: low first).
-__device__ __forceinline__ int reg_pos(const bool FWD, int l, int low, int hgh) {
-  return FWD ? ((hgh - l) & 31) : ((l - low) & 31);
-}
-__device__ __forceinline__ int reg_lane(const bool FWD, int p, int low, int hgh) {
-  return FWD ? ((hgh - p) & 31) : ((low + p) & 31);
-}
-// A lane mask reordered so that bit p is the lane at visit position p.
-__device__ __forceinline__ uint32_t reg_posmask(const bool FWD, uint32_t m, int low, int hgh) {
-  return FWD ? __brev(__funnelshift_l(m, m, 31 - (hgh & 31))) : __funnelshift_r(m, m, low & 31);
-}
-
-// Memory ring (buffer cur) -> registers for the diagonals of [plow, phgh].
-__device__ __forceinline__ void reg_load(const WarpWork &W, int cur, int plow, int phgh, RegWave &R) {
-  const int lane = threadIdx.x & 31, vmask = W.vcap - 1;
-  const int k = plow + ((lane - plow) & 31);
-  if (k <= phgh) {
-    const int vi = k & vmask;
-    R.V = W.V[cur][vi];
-    R.M = W.M[cur][vi];
-    R.T = W.T[cur][vi];
-    R.HA = W.HA[cur][vi];
-    R.HM = W.HM[cur][vi];
-    R.NA = W.NA[vi];
-  }
-}
-
-// Registers -> memory ring (buffer cur) for the diagonals of [plow, phgh].
-__device__ __forceinline__ void reg_store(WarpWork &W, int cur, int plow, int phgh, const RegWave &R) {
-  const int lane = threadIdx.x & 31, vmask = W.vcap - 1;
-  const int k = plow + ((lane - plow) & 31);
-  if (k <= phgh) {
-    const int vi = k & vmask;
-    W.V[cur][vi] = R.V;
-    W.M[cur][vi] = R.M;
-    W.T[cur][vi] = R.T;
-    W.HA[cur][vi] = R.HA;
-    W.HM[cur][vi] = R.HM;
-    W.NA[vi] = R.NA;
-  }
-}
-
-// One wave in registers: [low, hgh] (at most 32 wide) from the previous
-// wave [plow, phgh] (not empty, inside [low-1, hgh+1]).  Same results as
-// wave_sweep; fills WS for wave_prune.
-__device__ __forceinline__ int reg_wave(const bool FWD, RegCtx &X, const AlignSpec &spec, const Seq &A, const Seq &B,
-                                        int low, int hgh, int plow, int phgh, int dif, RegWave &R, int &besta,
-                                        int &bestx, int &lasta, int &trima, int &trimx, int &trimd, int &trimha,
-                                        int &more, int &aclip, int &bclip, WaveSlice &WS) {
-  const int lane = threadIdx.x & 31;
-  const int vmask = X.vmask;
-  const int tspace = spec.trace_space;
-  const int BV = FWD ? -1 : I32MAX;
-  const int k = low + ((lane - low) & 31);
-  const bool act = k <= hgh;
-  // the previous wave at k+1, k, k-1
-  const int vp = __shfl_sync(FULL, R.V, (lane + 1) & 31), vm = __shfl_sync(FULL, R.V, (lane - 1) & 31);
-  const int ap = (k + 1 >= plow && k + 1 <= phgh) ? vp : BV;
-  const int ac = (k >= plow && k <= phgh) ? R.V : BV;
-  const int am = (k - 1 >= plow && k - 1 <= phgh) ? vm : BV;
-  int src, c;
-  if (FWD) {
-    if (ac < am) src = (am < ap) ? 1 : -1;
-    else src = (ac < ap) ? 1 : 0;
-    c = src == 1 ? ap + 1 : (src == -1 ? am + 1 : ac + 2);
-  } else {
-    if (ac > ap) src = (ap > am) ? -1 : 1;
-    else src = (ac > am) ? -1 : 0;
-    c = src == -1 ? am - 1 : (src == 1 ? ap - 1 : ac - 2);
-  }
-  const int sl = (k + src) & 31;
-  const int sM = __shfl_sync(FULL, R.M, sl), sHA = __shfl_sync(FULL, R.HA, sl), sHM = __shfl_sync(FULL, R.HM, sl);
-  const uint64_t sT = __shfl_sync(FULL, R.T, sl);
-  // next trace mark: a new bottom diagonal copies the one above it, a new top
-  // diagonal the one below it
-  const int nlo = __shfl_sync(FULL, R.NA, plow & 31), nhi = __shfl_sync(FULL, R.NA, phgh & 31);
-  const bool dflt = FWD ? (src == 1 && k == hgh) : (src == -1 && k == low);
-  int m = dflt ? PATH_LEN : sM;
-  uint64_t b = dflt ? PATH_INT : sT;
-  int ha = dflt ? -1 : sHA, hm = dflt ? 0 : sHM;
-  int nak = (k >= plow && k <= phgh) ? R.NA : (k < plow ? nlo : nhi);
-  if ((b & PATH_TOP) != 0) m -= 1;
-  b <<= 1;
-  int x = (c + k) >> 1;
-  int run[1], hb[1], hA[1];
-  snake1(FWD, A, B, act, k, x, run[0], hb[0], hA[0]);
-  int npb = 0;
-  if (act) {
-    history_run(b, m, run[0]);
-    c = (x << 1) - k;
-    int hq = hm;
-    if (FWD) {
-      for (int q = nak; x >= q; q += tspace)
-        if (hq < q) {
-          npb++;
-          hq = q;
-        }
-    } else {
-      for (int q = nak; x <= q; q -= tspace)
-        if (hq > q) {
-          npb++;
-          hq = q;
-        }
-    }
-  }
-  // trim test of this diagonal's history (used if it is a record)
-  bool tr = false;
-  if (act && m >= spec.ave_path)
-    tr = spec.table[b & TRIM_MASK] >= 0 &&
-         spec.table[(b >> TRIM_LEN) & TRIM_MASK] + spec.score[b & TRIM_MASK] >= 0;
-  // pebble slots in visit order
-  const int pos = reg_pos(FWD, lane, low, hgh);
-  int off, tot;
-  if (__ballot_sync(FULL, npb > 1) == 0) {
-    uint32_t one = reg_posmask(FWD, __ballot_sync(FULL, npb == 1), low, hgh);
-    off = __popc(one & ((1u << pos) - 1));
-    tot = __popc(one);
-  } else {
-    // visit-order exclusive sum over positions
-    int xsum = npb;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      int y = __shfl_sync(FULL, xsum, reg_lane(FWD, pos - d, low, hgh));
-      if (pos >= d) xsum += y;
-    }
-    off = xsum - npb;
-    tot = __reduce_add_sync(FULL, npb);
-  }
-  int64_t pb0 = reg_pebbles(X, tot);
-  if (pb0 < 0) return 1;
-  if (act) {
-    int64_t s = pb0 + off;
-    Pebble *cells = X.cells;
-    if (FWD) {
-      while (x >= nak) {
-        if (hm < nak) {
-          cells[s] = {ha, k, dif, nak};
-          ha = (int)s;
-          hm = nak;
-          s += 1;
-        }
-        nak += tspace;
-      }
-    } else {
-      while (x <= nak) {
-        if (hm > nak) {
-          cells[s] = {ha, k, dif, nak};
-          ha = (int)s;
-          hm = nak;
-          s += 1;
-        }
-        nak -= tspace;
-      }
-    }
-    X.NA[k & vmask] = nak;
-    R.V = c;
-    R.M = m;
-    R.T = b;
-    R.HA = ha;
-    R.HM = hm;
-    R.NA = nak;
-  }
-  // clips: bclip from the first visited diagonal that met B's end, aclip
-  // from the last visited that met A's end
-  const uint32_t hbm = reg_posmask(FWD, __ballot_sync(FULL, act && hb[0]), low, hgh);
-  const uint32_t ham = reg_posmask(FWD, __ballot_sync(FULL, act && hA[0]), low, hgh);
-  if (hbm) {
-    more = 0;
-    const int p = __ffs(hbm) - 1;
-    const int kb = FWD ? hgh - p : low + p;
-    if (FWD ? (bclip < kb) : (bclip > kb)) bclip = kb;
-  }
-  if (ham) {
-    more = 0;
-    const int p = 31 - __clz(ham);
-    aclip = FWD ? hgh - p : low + p;
-  }
-  // records: c beyond the running best in visit order.  The last record is
-  // the first diagonal reaching the wave's best; the one before it the first
-  // reaching the best of the earlier positions, and so on.
-  const int carry = besta;
-  const int cv = act ? c : (FWD ? -2147483647 : 2147483647);
-  int best = FWD ? __reduce_max_sync(FULL, cv) : __reduce_min_sync(FULL, cv);
-  if (FWD ? best > carry : best < carry) {
-    const int fl = (m >= spec.ave_path ? 1 : 0) | (tr ? 2 : 0);
-    int limit = 32;  // positions below this are still candidates
-    int lp = -1, lt = -1;
-    bool first = true;
-    while (true) {
-      const uint32_t eq = reg_posmask(FWD, __ballot_sync(FULL, act && c == best && pos < limit), low, hgh);
-      const int p = __ffs(eq) - 1;
-      const int L = reg_lane(FWD, p, low, hgh);
-      if (first) {
-        besta = best;
-        bestx = __shfl_sync(FULL, x, L);
-        first = false;
-      }
-      const int f = __shfl_sync(FULL, fl, L);
-      if (lp < 0 && (f & 1)) lp = L;
-      if (f & 2) {
-        lt = L;
-        break;
-      }
-      limit = p;
-      const int cv2 = (act && pos < limit) ? c : (FWD ? -2147483647 : 2147483647);
-      best = FWD ? __reduce_max_sync(FULL, cv2) : __reduce_min_sync(FULL, cv2);
-      if (!(FWD ? best > carry : best < carry)) break;
-    }
-    if (lp >= 0) lasta = __shfl_sync(FULL, c, lp);
-    if (lt >= 0) {
-      trima = __shfl_sync(FULL, c, lt);
-      trimx = __shfl_sync(FULL, x, lt);
-      trimd = dif;
-      trimha = __shfl_sync(FULL, ha, lt);
-    }
-  }
-  WS.single = true;
-  WS.c[0] = c;
-  WS.k0 = k;
-  WS.nact = act ? 1 : 0;
-  return 0;
-}
-
-// The wave loop of forward_wave (FWD) or reverse_wave after the 0-wave:
-// grow the band, compute the wave, clip at sequence ends, prune.  Waves of
-// at most 32 diagonals run in registers (reg_wave), wider ones through the
-// memory ring (wave_sweep).
-__device__ __forceinline__ int wave_loop(const bool FWD, WarpWork &W, const AlignSpec &spec, const Seq &A, const Seq &B,
-                                         const uint8_t *aseq, const uint8_t *bseq, int minp, int maxp, int &low,
-                                         int &hgh, int &dif, int &cur, int &besta, int &bestx, int &lasta,
-                                         int &trima, int &trimx, int &trimd, int &trimha, int &more, int &aclip,
-                                         int &bclip, int &morem, int &morea, int &morex, int &mored, int &moreha,
-                                         int max_waves) {
-  const int lane = threadIdx.x & 31;
-  const int vmask = W.vcap - 1;
-  const int BV = FWD ? -1 : I32MAX;
-  int *NA = W.NA;
-  RegWave R;
-  R.V = BV;
-  R.M = R.HA = R.HM = R.NA = 0;
-  R.T = 0;
-  bool regmode = false;
-  RegCtx X{vmask, W.NA, W.pool.cells, W.pool.next, W.pool.cap, W.chunk_next, W.chunk_end, 0};
-  int nwaves = 0, ncells = 0, lwaves = 0;
-  // the register waves' read-only inputs, held in this loop's registers
-  const AlignSpec rspec = spec;
-  const Seq rA = A, rB = B;
-  // back to WarpWork: the pebble chunk, counts and errors
-  auto sync = [&]() {
-    W.chunk_next = X.chunk_next;
-    W.chunk_end = X.chunk_end;
-    W.err |= X.err;
-    W.waves += nwaves;
-    W.cells += ncells;
-    nwaves = ncells = 0;
-    X.err = 0;
-  };
-  while (more && (FWD ? lasta >= besta - TRIM_MLAG : lasta <= besta + TRIM_MLAG)) {
-    if (dif > max_waves) {
-      X.err |= ALN_ERR_VCAP;
-      sync();
-      return 1;
-    }
-    const int plow = low, phgh = hgh;
-    low -= 1;
-    hgh += 1;
-    if (hgh - low + 3 > vmask + 1) {
-      X.err |= ALN_ERR_VCAP;
-      sync();
-      return 1;
-    }
-    const bool grow_lo = low >= minp, grow_hi = hgh <= maxp;
-    if (!grow_lo) low += 1;
-    if (!grow_hi) hgh -= 1;
-    const bool use_reg = phgh >= plow && hgh - low + 1 <= 32;
-    nwaves += 1;
-    if (W.long_waves > 0 && !W.flagged && ++lwaves >= W.long_waves) {
-      // a long call: the other warps of this SM take no new task, so that it
-      // runs with the SM to itself once their current tasks end
-      if (lane == 0) {
-        unsigned sm;
-        asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
-        if (sm < SM_FLAGS) atomicExch(&W.smflag[sm], 1u);
-      }
-      W.flagged = 1;
-    }
-    ncells += hgh >= low ? hgh - low + 1 : 0;
-    WaveSlice WS;
-    if (use_reg) {
-      if (!regmode) {
-        reg_load(W, cur, plow, phgh, R);
-        regmode = true;
-      }
-      dif += 1;
-      if (reg_wave(FWD, X, rspec, rA, rB, low, hgh, plow, phgh, dif, R, besta, bestx, lasta, trima, trimx, trimd,
-                        trimha, more, aclip, bclip, WS)) {
-        sync();
-        return 1;
-      }
-    } else {
-      sync();
-      if (regmode) {
-        reg_store(W, cur, plow, phgh, R);
-        regmode = false;
-        __syncwarp();
-      }
-      // boundary diagonals on the previous wave's buffer (lane 0; visible
-      // after syncwarp); the diagonal past the top carries T = PATH_INT,
-      // M = PATH_LEN, HA = -1
-      int *Vo = W.V[cur];
-      if (lane == 0) {
-        if (grow_lo) {
-          NA[low & vmask] = NA[(low + 1) & vmask];
-          Vo[low & vmask] = BV;
-        }
-        if (grow_hi) {
-          NA[hgh & vmask] = NA[(hgh - 1) & vmask];
-          Vo[hgh & vmask] = BV;
-        }
-        Vo[(hgh + 1) & vmask] = BV;
-        Vo[(low - 1) & vmask] = BV;
-      }
-      dif += 1;
-      __syncwarp();
-      if (wave_sweep(FWD, W, spec, A, B, low, hgh, dif, cur, besta, bestx, lasta, trima, trimx, trimd, trimha, more,
-                          aclip, bclip, WS))
-        return 1;
-      X.chunk_next = W.chunk_next;
-      X.chunk_end = W.chunk_end;
-      cur ^= 1;
-      __syncwarp();
-    }
-    if (more == 0) {
-      if (bseq[besta - bestx] != 4 && aseq[bestx] != 4) more = 1;
-      // state of a diagonal of the wave just made
-      auto at = [&](int kq, int &vq, int &mq, int &haq) {
-        if (regmode) {
-          vq = __shfl_sync(FULL, R.V, kq & 31);
-          mq = __shfl_sync(FULL, R.M, kq & 31);
-          haq = __shfl_sync(FULL, R.HA, kq & 31);
-        } else {
-          vq = W.V[cur][kq & vmask];
-          mq = W.M[cur][kq & vmask];
-          haq = W.HA[cur][kq & vmask];
-        }
-      };
-      // FWD: the top side meets A's end (aclip), the bottom B's (bclip);
-      // reverse: the bottom meets A's start, the top B's
-      const bool cut_a = FWD ? hgh >= aclip : low <= aclip;
-      if (cut_a) {
-        if (FWD) hgh = aclip - 1;
-        else low = aclip + 1;
-        int vq, mq, haq;
-        at(aclip, vq, mq, haq);
-        if (morem <= mq) {
-          morem = mq;
-          morea = vq;
-          morex = (morea + aclip) >> 1;
-          mored = dif;
-          moreha = haq;
-        }
-      }
-      const bool cut_b = FWD ? low <= bclip : hgh >= bclip;
-      if (cut_b) {
-        if (FWD) low = bclip + 1;
-        else hgh = bclip - 1;
-        int vq, mq, haq;
-        at(bclip, vq, mq, haq);
-        if (morem <= mq) {
-          morem = mq;
-          morea = vq;
-          morex = (morea + bclip) >> 1;
-          mored = dif;
-          moreha = haq;
-        }
-      }
-      aclip = FWD ? I32MAX : -I32MAX;
-      bclip = FWD ? -I32MAX : I32MAX;
-    }
-    if (regmode) {
-      // WAVE_LAG pruning of a register wave: its one diagonal per lane
-      if (hgh >= low) {
-        const int n = FWD ? besta - WAVE_LAG : besta + WAVE_LAG;
-        const bool pass = WS.nact && WS.k0 >= low && WS.k0 <= hgh && (FWD ? WS.c[0] >= n : WS.c[0] <= n);
-        const int kmax = __reduce_max_sync(FULL, pass ? WS.k0 : -2147483647);
-        const int kmin = __reduce_min_sync(FULL, pass ? WS.k0 : 2147483647);
-        if (kmin <= kmax) {
-          hgh = kmax;
-          low = kmin;
-        } else
-          hgh = low - 1;
-      }
-    } else
-      wave_prune(FWD, W, W.V[cur], besta, low, hgh, WS);
-  }
-  sync();
   __syncwarp();
+  S.low = low;
+  S.hgh = hgh;
+  S.dif = dif;
+  S.besta = besta;
+  S.lasta = lasta;
+  io = S;
   return 0;
 }
 
-// The wave loop's state across the call below.
-struct WaveState {
-  int low, hgh, dif, cur, besta, bestx, lasta, trima, trimx, trimd, trimha, more, aclip, bclip, morem, morea, morex,
-      mored, moreha;
-};
-
-// One out-of-line copy of the wave loop serves both directions (FWD is a
-// run-time flag).  The alignment kernel is bound by instruction fetch: two
-// inlined copies of this loop, one per direction, kept twice the hot code in
-// the instruction cache; one shared copy cut the pair phase of a 2 x 1 Gbp
-// genome pair by a quarter with the same alignments.
-__device__ __noinline__ int wave_loop_shared(const bool FWD, WarpWork &W, const AlignSpec &spec, const Seq &A,
-                                             const Seq &B, const uint8_t *aseq, const uint8_t *bseq, int minp,
-                                             int maxp, WaveState *io, int max_waves) {
-  WaveState s = *io;
-  const int r = wave_loop(FWD, W, spec, A, B, aseq, bseq, minp, maxp, s.low, s.hgh, s.dif, s.cur, s.besta, s.bestx,
-                          s.lasta, s.trima, s.trimx, s.trimd, s.trimha, s.more, s.aclip, s.bclip, s.morem, s.morea,
-                          s.morex, s.mored, s.moreha, max_waves);
-  *io = s;
-  return r;
-}
-
-// wave_loop through the shared copy, with the caller's variables.
-__device__ __forceinline__ int wave_loop_call(const bool FWD, WarpWork &W, const AlignSpec &spec, const Seq &A,
-                                              const Seq &B, const uint8_t *aseq, const uint8_t *bseq, int minp,
-                                              int maxp, int &low, int &hgh, int &dif, int &cur, int &besta,
-                                              int &bestx, int &lasta, int &trima, int &trimx, int &trimd,
-                                              int &trimha, int &more, int &aclip, int &bclip, int &morem, int &morea,
-                                              int &morex, int &mored, int &moreha, int max_waves) {
-  WaveState s{low,   hgh,  dif,   cur,   besta, bestx, lasta, trima, trimx, trimd,
-              trimha, more, aclip, bclip, morem, morea, morex, mored, moreha};
-  const int r = wave_loop_shared(FWD, W, spec, A, B, aseq, bseq, minp, maxp, &s, max_waves);
-  low = s.low, hgh = s.hgh, dif = s.dif, cur = s.cur, besta = s.besta, bestx = s.bestx, lasta = s.lasta;
-  trima = s.trima, trimx = s.trimx, trimd = s.trimd, trimha = s.trimha, more = s.more, aclip = s.aclip;
-  bclip = s.bclip, morem = s.morem, morea = s.morea, morex = s.morex, mored = s.mored, moreha = s.moreha;
-  return r;
-}
-
-#define WVI(k) ((k) & vmask)
-
 // ---------------------------------------------------------------------------
-// forward_wave, warp version.  Returns 1 on an arena overflow (W.err set).
+// Wide waves: the ring in memory (L1-resident at the widths that occur), 32
+// diagonals per pass from the highest down.  The waves past an alignment's
+// end run here: they widen by two diagonals per step until the trim lag ends
+// the loop.  Runs until the loop ends, the window narrows to WIDE_OUT
+// diagonals, or the wave count reaches `stop`.
 // ---------------------------------------------------------------------------
-__device__ int forward_wave_w(WarpWork &W, const AlignSpec &spec, const Seq &A, const Seq &B, Path &P, int *mind,
-                              int maxd, int mida, int minp, int maxp, int aoff) {
+constexpr int WIDE_OUT = 20;
+
+__device__ __forceinline__ int wide_waves(WarpWork &W, Wave &io, int stop) {
   const int lane = threadIdx.x & 31;
-  const uint8_t *aseq = A.s;
-  const uint8_t *bseq = B.s;
+  Wave S = io;
+  const TrimTest trim(S.dscore);
   const int vmask = W.vcap - 1;
-  int cur = 0;
-  int *NA = W.NA;
-  Pebble *cells = W.pool.cells;
-  const int tspace = spec.trace_space;
+  int next = (int)W.chunk_next, end = (int)W.chunk_end;
+  const int dif0 = S.dif;
+  int ncells = 0, err = 0;
+  while (S.more && S.lasta >= S.besta - TRIM_MLAG) {
+    if (S.hgh - S.low < WIDE_OUT || S.dif >= stop) break;
+    if (S.hgh - S.low + 5 > W.vcap) {
+      err = ALN_ERR_VCAP;
+      break;
+    }
+    const RingCell *Co = W.C[S.cur];
+    RingCell *Cn = W.C[S.cur ^ 1];
+    int *Vo = W.V[S.cur], *Vn = W.V[S.cur ^ 1];
+    if (lane == 0) {
+      // the diagonals just outside, and the trace marks of grown ends
+      const bool glo = S.low > S.minp, ghi = S.hgh < S.maxp;
+      Vo[(S.low - 1) & vmask] = Vo[(S.hgh + 1) & vmask] = NO_WAVE;
+      if (glo) {
+        Vo[(S.low - 2) & vmask] = NO_WAVE;
+        W.NA[(S.low - 1) & vmask] = W.NA[S.low & vmask];
+      }
+      if (ghi) {
+        Vo[(S.hgh + 2) & vmask] = NO_WAVE;
+        W.NA[(S.hgh + 1) & vmask] = W.NA[S.hgh & vmask];
+      }
+    }
+    __syncwarp();
+    const int low = S.low - (S.low > S.minp ? 1 : 0), hgh = S.hgh + (S.hgh < S.maxp ? 1 : 0);
+    S.low = low;
+    S.hgh = hgh;
+    S.dif += 1;
+    ncells += hgh - low + 1;
+    int ka = I32MAX, kb = NO_WAVE;
+    for (int top = hgh; top >= low; top -= 32) {
+      const int k = top - lane, vi = k & vmask;
+      const bool act = k >= low;
+      int c = 0, ha = -1, hm = 0, nak = 0, x = 0, mx = 0;
+      uint64_t t0 = 0;
+      if (act) {
+        const int vup = Vo[(k + 1) & vmask], v = Vo[vi], vdn = Vo[(k - 1) & vmask];
+        nak = W.NA[vi];
+        const bool up = vup > max(v, vdn), dn = !up && vdn > v;
+        c = up ? vup + 1 : (dn ? vdn + 1 : v + 2);
+        const RingCell q = Co[(k + (up ? 1 : (dn ? -1 : 0))) & vmask];
+        t0 = q.T;
+        ha = q.HA;
+        hm = q.HM;
+        x = (c + k) >> 1;
+        mx = min(S.limA - x, S.limB - x + k);
+      }
+      bool go;
+      const int run = snake<2>(S, x, k, act, mx, go);
+      const bool hit = act && (!go || run == mx);
+      const uint64_t b = hist_step(t0, run);
+      x += run;
+      c = (x << 1) - k;
+      if (!drop_pebbles(W, S, act, k, x, S.dif, ha, hm, nak, next, end)) {
+        err = ALN_ERR_CELLS;
+        break;
+      }
+      if (act) {
+        Vn[vi] = c;
+        Cn[vi] = RingCell{b, ha, hm};
+        W.NA[vi] = nak;
+      }
+      take_records(S, S.besta, S.lasta, trim, act, k, c, b, ha, S.dif);
+      if (__any_sync(FULL, hit)) {
+        const bool hb = met_b(S, x - run, k, go);
+        ka = min(ka, __reduce_min_sync(FULL, hit && !hb ? k : I32MAX));
+        kb = max(kb, __reduce_max_sync(FULL, hit && hb ? k : NO_WAVE));
+      }
+    }
+    if (err) break;
+    S.cur ^= 1;
+    __syncwarp();
+    if (ka != I32MAX || kb != NO_WAVE) {
+      S.more = can_grow(S, S.besta);
+      if (ka != I32MAX) {
+        S.hgh = ka - 1;
+        const RingCell q = Cn[ka & vmask];
+        note_end(S, ka, q.T, Vn[ka & vmask], q.HA, S.dif);
+      }
+      if (kb != NO_WAVE) {
+        S.low = kb + 1;
+        const RingCell q = Cn[kb & vmask];
+        note_end(S, kb, q.T, Vn[kb & vmask], q.HA, S.dif);
+      }
+    }
+    // WAVE_LAG pruning from either end
+    if (S.hgh >= S.low) {
+      const int n = S.besta - WAVE_LAG;
+      int nh = S.low - 1;
+      for (int top = S.hgh; top >= S.low; top -= 32) {
+        const int k = top - lane;
+        const uint32_t keep = __ballot_sync(FULL, k >= S.low && Vn[k & vmask] >= n);
+        if (keep) {
+          nh = top - __ffs(keep) + 1;
+          break;
+        }
+      }
+      S.hgh = nh;
+      for (int bot = S.low; bot <= nh; bot += 32) {
+        const int k = bot + lane;
+        const uint32_t keep = __ballot_sync(FULL, k <= nh && Vn[k & vmask] >= n);
+        if (keep) {
+          S.low = bot + __ffs(keep) - 1;
+          break;
+        }
+      }
+    }
+  }
+  __syncwarp();
+  W.chunk_next = next;
+  W.chunk_end = end;
+  W.waves += S.dif - dif0;
+  W.cells += ncells;
+  if (err) {
+    W.err |= err;
+    return 1;
+  }
+  io = S;
+  return 0;
+}
 
-  int hgh = maxd, low = *mind, dif = 0;
-  int besta, bestx, trima, trimx, trimd, trimha, morea, morex, mored, moreha, more, morem, lasta;
-  int aclip, bclip;
-  if (hgh - low + 3 > W.vcap) {
+// forward_wave (fwd) or reverse_wave of a path, out of line: one copy of the
+// code serves both directions and every call.  `start` is the forward wave's
+// lowest diagonal on entry and, on return, the diagonal the path starts on.
+// Returns 1 on a work-space overflow (W.err set).
+__device__ __noinline__ int extend(const bool fwd, WarpWork &W, const AlignSpec &spec, const Seq &A, const Seq &B,
+                                   Path &P, int &start, int maxd, int mida, int minp, int maxp, int aoff) {
+  const int lane = threadIdx.x & 31;
+  const int tspace = spec.trace_space;
+  const int vmask = W.vcap - 1;
+  Pebble *cells = W.pool.cells;
+  if (maxd - start + 3 > W.vcap) {
     W.err |= ALN_ERR_VCAP;
     return 1;
   }
-  more = 1;
-  aclip = I32MAX;
-  bclip = -I32MAX;
-  besta = trima = morea = lasta = mida;
-  bestx = trimx = morex = (mida + hgh) >> 1;
-  trimd = mored = 0;
-  trimha = moreha = 0;
-  morem = -1;
+  Wave S;
+  S.pa = fwd ? A.pf : A.pr;
+  S.pb = fwd ? B.pf : B.pr;
+  S.offA = fwd ? 0 : A.len;
+  S.offB = fwd ? 0 : B.len;
+  S.limA = fwd ? A.len : 0;
+  S.limB = fwd ? B.len : 0;
+  S.minp = fwd ? minp : -maxp;
+  S.maxp = fwd ? maxp : -minp;
+  S.tspace = tspace;
+  S.ave_path = spec.ave_path;
+  S.dscore = spec.dscore;
+  S.sg = fwd ? 1 : -1;
+  S.low = fwd ? start : -maxd;
+  S.hgh = fwd ? maxd : -start;
+  S.dif = S.cur = 0;
+  S.besta = S.lasta = S.trima = S.morea = S.sg * mida;
+  S.bestx = S.trimx = S.morex = S.sg * ((mida + maxd) >> 1);
+  S.trimd = S.mored = S.trimha = S.moreha = 0;
+  S.more = 1;
+  S.morem = -1;
   int64_t call_base = -1;  // this call's first pebble: the reference's cells[0]
-  const int max_waves = A.len + B.len + 1024;
 
-  // 0-wave: diagonals visited hgh..low
-  for (int base = hgh; base >= low; base -= 32) {
-    int k = base - lane;
-    bool act = k >= low;
-    int x = 0, c = 0, na = 0, hb = 0, ha_ = 0, npb = 0;
+  // 0-wave: diagonals visited from the highest down
+  int ka = I32MAX, kb = NO_WAVE;
+  for (int top = S.hgh; top >= S.low; top -= 32) {
+    const int k = top - lane;
+    const bool act = k >= S.low;
+    int x = 0, mark = 0, nak = 0, mx = 0;
     if (act) {
-      x = (mida + k) >> 1;
-      na = ((x + (tspace - aoff)) / tspace - 1) * tspace + aoff;
-      x = snake_fwd(A, B, x, k, &hb, &ha_);
-      c = (x << 1) - k;
-      npb = 1;
-      for (int q = na + tspace; x >= q; q += tspace) npb++;
+      const int x0 = (mida + S.sg * k) >> 1;
+      // forward: the trace mark at or below the start is its pebble's mark;
+      // reverse: the start itself, and the mark below it comes next
+      const int m0 = ((x0 + (tspace - aoff) - (fwd ? 0 : 1)) / tspace - 1) * tspace + aoff;
+      x = S.sg * x0;
+      mark = fwd ? m0 : x;
+      nak = fwd ? m0 + tspace : -m0;
+      mx = min(S.limA - x, S.limB - x + k);
     }
-    int off = warp_excl_sum(npb, lane);
-    int tot = warp_sum(npb);
-    int64_t pb0 = warp_pebbles(W, tot);
+    bool go;
+    const int xs = x, run = snake<4>(S, x, k, act, mx, go);
+    const bool hit = act && (!go || run == mx);
+    x += run;
+    const int c = (x << 1) - k;
+    const int npb = act ? 1 + (x >= nak ? (x - nak) / tspace + 1 : 0) : 0;
+    const int off = warp_excl_sum(npb, lane);
+    const int tot = __reduce_add_sync(FULL, npb);
+    const int64_t pb0 = warp_pebbles(W, tot);
     if (pb0 < 0) return 1;
     if (call_base < 0) {
       call_base = pb0;
-      trimha = moreha = (int)pb0;
+      S.trimha = S.moreha = (int)pb0;
     }
-    int ha = -1;
+    int ha = (int)pb0 + off;
     if (act) {
-      int64_t s = pb0 + off;
-      cells[s] = {-1, k, 0, na};
-      ha = (int)s;
-      int hm = na;
-      na += tspace;
-      while (x >= na) {
-        s += 1;
-        cells[s] = {ha, k, 0, na};
-        ha = (int)s;
-        hm = na;
-        na += tspace;
+      *reinterpret_cast<int4 *>(cells + ha) = make_int4(-1, S.sg * k, 0, S.sg * mark);
+      for (; x >= nak; nak += tspace) {
+        mark = nak;
+        *reinterpret_cast<int4 *>(cells + ha + 1) = make_int4(ha, S.sg * k, 0, S.sg * mark);
+        ha += 1;
       }
-      int vi = WVI(k);
-      W.V[cur][vi] = c;
-      W.T[cur][vi] = PATH_INT;
-      W.M[cur][vi] = PATH_LEN;
-      W.HA[cur][vi] = ha;
-      W.HM[cur][vi] = hm;
-      NA[vi] = na;
+      const int vi = k & vmask;
+      W.V[0][vi] = c;
+      W.C[0][vi] = RingCell{PATH_INT, ha, mark};
+      W.NA[vi] = nak;
     }
-    // clips: bclip = largest k that met B's end, aclip = last visited (smallest) k that met A's end
-    uint32_t bb = __ballot_sync(FULL, act && hb), ba = __ballot_sync(FULL, act && ha_);
-    if (bb) {
-      more = 0;
-      int kk = base - (__ffs(bb) - 1);
-      if (bclip < kk) bclip = kk;
+    if (__any_sync(FULL, hit)) {
+      const bool hb = met_b(S, xs, k, go);
+      ka = min(ka, __reduce_min_sync(FULL, hit && !hb ? k : I32MAX));
+      kb = max(kb, __reduce_max_sync(FULL, hit && hb ? k : NO_WAVE));
     }
-    if (ba) {
-      more = 0;
-      aclip = base - last_lane(ba);
-    }
-    // records: c > running maximum
-    int pm = warp_excl_max(act ? c : -2147483647, lane, besta);
-    bool rec = act && c > pm;
-    uint32_t rb = __ballot_sync(FULL, rec);
-    if (rb) {
-      int L = last_lane(rb);
-      besta = trima = lasta = __shfl_sync(FULL, c, L);
-      bestx = trimx = __shfl_sync(FULL, x, L);
-      trimha = __shfl_sync(FULL, ha, L);
+    // the last record is the highest diagonal with the pass's best
+    const int rc = __reduce_max_sync(FULL, act ? c : NO_WAVE);
+    if (rc > S.besta) {
+      const int L = __ffs(__ballot_sync(FULL, act && c == rc)) - 1;
+      S.besta = S.trima = S.lasta = rc;
+      S.bestx = S.trimx = __shfl_sync(FULL, x, L);
+      S.trimha = __shfl_sync(FULL, ha, L);
     }
   }
   __syncwarp();
-  {
-    int *V = W.V[cur], *M = W.M[cur], *HA = W.HA[cur];
-    if (more == 0) {
-      if (bseq[besta - bestx] != 4 && aseq[bestx] != 4) more = 1;
-      if (hgh >= aclip) {
-        hgh = aclip - 1;
-        if (morem <= M[WVI(aclip)]) {
-          morem = M[WVI(aclip)];
-          morea = V[WVI(aclip)];
-          morex = (morea + aclip) >> 1;
-          moreha = HA[WVI(aclip)];
-        }
-      }
-      if (low <= bclip) {
-        low = bclip + 1;
-        if (morem <= M[WVI(bclip)]) {
-          morem = M[WVI(bclip)];
-          morea = V[WVI(bclip)];
-          morex = (morea + bclip) >> 1;
-          moreha = HA[WVI(bclip)];
-        }
-      }
-      aclip = I32MAX;
-      bclip = -I32MAX;
+  if (ka != I32MAX || kb != NO_WAVE) {
+    S.more = can_grow(S, S.besta);
+    if (ka != I32MAX) {
+      S.hgh = ka - 1;
+      const RingCell q = W.C[0][ka & vmask];
+      note_end(S, ka, PATH_INT, W.V[0][ka & vmask], q.HA, 0);
+    }
+    if (kb != NO_WAVE && S.low <= kb) {
+      S.low = kb + 1;
+      const RingCell q = W.C[0][kb & vmask];
+      note_end(S, kb, PATH_INT, W.V[0][kb & vmask], q.HA, 0);
     }
   }
 
-  if (wave_loop_call(true, W, spec, A, B, aseq, bseq, minp, maxp, low, hgh, dif, cur, besta, bestx, lasta, trima,
-                     trimx, trimd, trimha, more, aclip, bclip, morem, morea, morex, mored, moreha, max_waves))
-    return 1;
-  __syncwarp();
-
-  // trace-back (lane-uniform sequential code; only lane 0 writes)
-  {
-    uint16_t *atrace = W.points + P.trace_off;
-    int atlen = 0, trimy, a, b, k, h, d, e;
-    if (morem >= 0 && spec.reach) {
-      trimx = morex;
-      trimy = morea - morex;
-      trimd = mored;
-      trimha = moreha;
-    } else
-      trimy = trima - trimx;
-    // reverse the pebble chain: done by lane 0, read back by all
-    int bad = 0;
-    if (lane == 0) {
-      int64_t steps = 0, lim = W.chunk_next - call_base + 1;
-      a = -1;
-      for (h = trimha; h >= 0; h = b) {
-        if (h < call_base || ++steps > lim) {
-          bad = 1;
-          break;
-        }
-        b = cells[h].ptr;
-        cells[h].ptr = a;
-        a = h;
-      }
-    }
-    if (__shfl_sync(FULL, bad, 0)) {
-      W.err |= ALN_ERR_CELLS;
+  const int max_waves = A.len + B.len + 1024;
+  while (S.more && S.lasta >= S.besta - TRIM_MLAG) {
+    // no wave to grow from, or more waves than bases: neither ends by itself
+    if (S.hgh < S.low || S.dif > max_waves) {
+      W.err |= ALN_ERR_VCAP;
       return 1;
     }
-    __syncwarp();
-    a = __shfl_sync(FULL, a, 0);
-    h = a;
-    k = cells[h].diag;
-    b = (mida - k) >> 1;
-    e = 0;
-    low = k;
-    for (h = cells[h].ptr; h >= 0; h = cells[h].ptr) {
-      k = cells[h].diag;
-      a = cells[h].mark - k;
-      d = cells[h].diff;
-      if (P.trace_off + atlen + 2 > W.point_cap) {
-        W.err |= ALN_ERR_POINTS;
-        return 1;
-      }
-      if (lane == 0) {
-        atrace[atlen] = (uint16_t)(d - e);
-        atrace[atlen + 1] = (uint16_t)(a - b);
-      }
-      atlen += 2;
-      b = a;
-      e = d;
+    int stop = max_waves + 1;
+    if (W.long_waves > 0 && !W.flagged) {
+      if (S.dif + 1 >= W.long_waves) {
+        // a long call: the other warps of this SM take no new task, so that it
+        // runs with the SM to itself once their current tasks end
+        if (lane == 0) {
+          unsigned sm;
+          asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+          if (sm < SM_FLAGS) atomicExch(&W.smflag[sm], 1u);
+        }
+        W.flagged = 1;
+      } else
+        stop = min(stop, W.long_waves - 1);
     }
-    __syncwarp();
-    if (b + k != trimx) {
-      if (P.trace_off + atlen + 2 > W.point_cap) {
-        W.err |= ALN_ERR_POINTS;
-        return 1;
-      }
-      if (lane == 0) {
-        atrace[atlen] = (uint16_t)(trimd - e);
-        atrace[atlen + 1] = (uint16_t)(trimy - b);
-      }
-      atlen += 2;
-    } else if (b != trimy) {
-      if (lane == 0) {
-        atrace[atlen - 1] = (uint16_t)(atrace[atlen - 1] + (trimy - b));
-        atrace[atlen - 2] = (uint16_t)(atrace[atlen - 2] + (trimd - e));
-      }
+    const int width = S.hgh - S.low + 1 + (S.low > S.minp ? 1 : 0) + (S.hgh < S.maxp ? 1 : 0);
+    if (width > NARROW ? wide_waves(W, S, stop) : narrow_waves(W, S, stop)) return 1;
+  }
+  __syncwarp();
+
+  // Trace-back, from the path's tip to its start: one pebble per step, read
+  // whole.  Lane 0 writes each interval's (diffs, b-delta) to the free end of
+  // the trace buffer; the warp then moves them next to the path's start.
+  int trimx = S.sg * S.trimx, trimy = S.sg * S.trima - trimx, trimd = S.trimd, h = S.trimha;
+  if (S.morem >= 0 && spec.reach) {
+    trimx = S.sg * S.morex;
+    trimy = S.sg * S.morea - trimx;
+    trimd = S.mored;
+    h = S.moreha;
+  }
+  const int64_t t0 = P.trace_off;
+  const int64_t room = (fwd ? W.point_cap - t0 : t0) >> 1;  // intervals the free end holds
+  const int64_t lim = W.chunk_next - call_base + 1;
+  const int4 *cl = reinterpret_cast<const int4 *>(cells);  // ptr, diag, diff, mark
+  int64_t n = 0;
+  // forward intervals come last first, down from the buffer's top; reverse
+  // ones first first, up from its bottom
+  auto put = [&](int dd, int db) {
+    n += 1;
+    if (lane == 0 && n <= room) {
+      uint16_t *o = W.points + (fwd ? W.point_cap - 2 * n : 2 * (n - 1));
+      o[0] = (uint16_t)dd;
+      o[1] = (uint16_t)db;
     }
-    __syncwarp();
+  };
+  // the interval of a reverse path that ends inside the forward path's first one
+  auto join = [&](int dd, int db) {
+    if (lane == 0) {
+      uint16_t *o = W.points + t0;
+      o[0] = (uint16_t)(o[0] + dd);
+      o[1] = (uint16_t)(o[1] + db);
+    }
+  };
+  int4 q = cl[h];
+  bool first = q.x < 0;
+  int qb = fwd && first ? (mida - q.y) >> 1 : q.w - q.y;
+  int dd = trimd - q.z, db = S.sg * (trimy - qb);  // past the last mark
+  const bool inside = !fwd && first && q.w % tspace != aoff;
+  if (inside || qb + q.y != trimx) {
+    if (inside && P.tlen != 0) join(dd, db);
+    else put(dd, db);
+    dd = db = 0;
+  } else if (qb == trimy)
+    dd = db = 0;
+  else if (first && !fwd)
+    join(dd, db);
+  int steps = 0;
+  while (!first) {
+    if (q.x < call_base || ++steps > lim || n > room) {
+      W.err |= n > room ? ALN_ERR_POINTS : ALN_ERR_CELLS;
+      return 1;
+    }
+    const int4 p = cl[q.x];
+    first = p.x < 0;
+    const int pb = fwd && first ? (mida - p.y) >> 1 : p.w - p.y;
+    dd += q.z - p.z;
+    db += S.sg * (qb - pb);
+    if (!fwd && first && P.tlen != 0 && p.w % tspace != aoff) join(dd, db);
+    else put(dd, db);
+    dd = db = 0;
+    q = p;
+    qb = pb;
+  }
+  if (n > room) {
+    W.err |= ALN_ERR_POINTS;
+    return 1;
+  }
+  __syncwarp();
+  {
+    uint32_t *pt = reinterpret_cast<uint32_t *>(W.points);
+    const int64_t src = fwd ? (W.point_cap >> 1) - n : 0, dst = fwd ? t0 >> 1 : (t0 >> 1) - n;
+    for (int64_t i = 0; i < n; i += 32) {
+      const int64_t j = fwd ? i + lane : n - 1 - i - lane;  // away from what is still to be read
+      uint32_t v = 0;
+      const bool in = i + lane < n;
+      if (in) v = pt[src + j];
+      __syncwarp();
+      if (in) pt[dst + j] = v;
+      __syncwarp();
+    }
+  }
+  if (fwd) {
+    start = q.y;
     P.aepos = trimx;
     P.bepos = trimy;
     P.diffs = trimd;
-    P.tlen = atlen;
-  }
-  *mind = low;
-  return 0;
-}
-
-// ---------------------------------------------------------------------------
-// reverse_wave, warp version (visit order k = low..hgh, minimum instead of
-// maximum, sequences read one position to the left).
-// ---------------------------------------------------------------------------
-__device__ int reverse_wave_w(WarpWork &W, const AlignSpec &spec, const Seq &A, const Seq &B, Path &P, int mind,
-                              int maxd, int mida, int minp, int maxp, int aoff) {
-  const int lane = threadIdx.x & 31;
-  const uint8_t *aseq = A.s - 1;
-  const uint8_t *bseq = B.s - 1;
-  const int vmask = W.vcap - 1;
-  int cur = 0;
-  int *NA = W.NA;
-  Pebble *cells = W.pool.cells;
-  const int tspace = spec.trace_space;
-
-  int hgh = maxd, low = mind, dif = 0;
-  int besta, bestx, trima, trimx, trimd, trimha, morea, morex, mored, moreha, more, morem, lasta;
-  int aclip, bclip;
-  if (hgh - low + 3 > W.vcap) {
-    W.err |= ALN_ERR_VCAP;
-    return 1;
-  }
-  more = 1;
-  aclip = -I32MAX;
-  bclip = I32MAX;
-  besta = trima = morea = lasta = mida;
-  bestx = trimx = morex = (mida + hgh) >> 1;
-  trimd = mored = 0;
-  trimha = moreha = 0;
-  morem = -1;
-  int64_t call_base = -1;  // this call's first pebble: the reference's cells[0]
-  const int max_waves = A.len + B.len + 1024;
-
-  for (int base = low; base <= hgh; base += 32) {
-    int k = base + lane;
-    bool act = k <= hgh;
-    int x = 0, c = 0, na = 0, hb = 0, hA = 0, npb = 0, x0 = 0;
-    if (act) {
-      x = (mida + k) >> 1;
-      x0 = x;
-      na = ((x + (tspace - aoff) - 1) / tspace - 1) * tspace + aoff;
-      x = snake_rev(A, B, x, k, &hb, &hA);
-      c = (x << 1) - k;
-      npb = 1;
-      for (int q = na; x <= q; q -= tspace) npb++;
-    }
-    int off = warp_excl_sum(npb, lane);
-    int tot = warp_sum(npb);
-    int64_t pb0 = warp_pebbles(W, tot);
-    if (pb0 < 0) return 1;
-    if (call_base < 0) {
-      call_base = pb0;
-      trimha = moreha = (int)pb0;
-    }
-    int ha = -1;
-    if (act) {
-      int64_t s = pb0 + off;
-      cells[s] = {-1, k, 0, x0};
-      ha = (int)s;
-      int hm = x0;
-      while (x <= na) {
-        s += 1;
-        cells[s] = {ha, k, 0, na};
-        ha = (int)s;
-        hm = na;
-        na -= tspace;
-      }
-      int vi = WVI(k);
-      W.V[cur][vi] = c;
-      W.T[cur][vi] = PATH_INT;
-      W.M[cur][vi] = PATH_LEN;
-      W.HA[cur][vi] = ha;
-      W.HM[cur][vi] = hm;
-      NA[vi] = na;
-    }
-    // bclip = smallest k that met B's start, aclip = last visited (largest) k that met A's start
-    uint32_t bb = __ballot_sync(FULL, act && hb), ba = __ballot_sync(FULL, act && hA);
-    if (bb) {
-      more = 0;
-      int kk = base + (__ffs(bb) - 1);
-      if (bclip > kk) bclip = kk;
-    }
-    if (ba) {
-      more = 0;
-      aclip = base + last_lane(ba);
-    }
-    int pm = warp_excl_min(act ? c : 2147483647, lane, besta);
-    bool rec = act && c < pm;
-    uint32_t rb = __ballot_sync(FULL, rec);
-    if (rb) {
-      int L = last_lane(rb);
-      besta = trima = lasta = __shfl_sync(FULL, c, L);
-      bestx = trimx = __shfl_sync(FULL, x, L);
-      trimha = __shfl_sync(FULL, ha, L);
-    }
-  }
-  __syncwarp();
-  {
-    int *V = W.V[cur], *M = W.M[cur], *HA = W.HA[cur];
-    if (more == 0) {
-      if (bseq[besta - bestx] != 4 && aseq[bestx] != 4) more = 1;
-      if (low <= aclip) {
-        low = aclip + 1;
-        if (morem <= M[WVI(aclip)]) {
-          morem = M[WVI(aclip)];
-          morea = V[WVI(aclip)];
-          morex = (morea + aclip) >> 1;
-          moreha = HA[WVI(aclip)];
-        }
-      }
-      if (hgh >= bclip) {
-        hgh = bclip - 1;
-        if (morem <= M[WVI(bclip)]) {
-          morem = M[WVI(bclip)];
-          morea = V[WVI(bclip)];
-          morex = (morea + bclip) >> 1;
-          moreha = HA[WVI(bclip)];
-        }
-      }
-      aclip = -I32MAX;
-      bclip = I32MAX;
-    }
-  }
-
-  if (wave_loop_call(false, W, spec, A, B, aseq, bseq, minp, maxp, low, hgh, dif, cur, besta, bestx, lasta, trima,
-                     trimx, trimd, trimha, more, aclip, bclip, morem, morea, morex, mored, moreha, max_waves))
-    return 1;
-  __syncwarp();
-
-  {
-    uint16_t *atrace = W.points + P.trace_off;
-    int atlen = 0, trimy, a, b, k, h, d, e;
-    if (morem >= 0 && spec.reach) {
-      trimx = morex;
-      trimy = morea - morex;
-      trimd = mored;
-      trimha = moreha;
-    } else
-      trimy = trima - trimx;
-    int bad = 0;
-    if (lane == 0) {
-      int64_t steps = 0, lim = W.chunk_next - call_base + 1;
-      a = -1;
-      for (h = trimha; h >= 0; h = b) {
-        if (h < call_base || ++steps > lim) {
-          bad = 1;
-          break;
-        }
-        b = cells[h].ptr;
-        cells[h].ptr = a;
-        a = h;
-      }
-    }
-    if (__shfl_sync(FULL, bad, 0)) {
-      W.err |= ALN_ERR_CELLS;
-      return 1;
-    }
-    __syncwarp();
-    a = __shfl_sync(FULL, a, 0);
-    h = a;
-    k = cells[h].diag;
-    b = cells[h].mark - k;
-    e = 0;
-    if ((b + k) % tspace != aoff) {
-      h = cells[h].ptr;
-      if (h < 0) {
-        a = trimy;
-        d = trimd;
-      } else {
-        k = cells[h].diag;
-        a = cells[h].mark - k;
-        d = cells[h].diff;
-      }
-      if (P.tlen == 0) {
-        if (P.trace_off + atlen - 2 < 0) {
-          W.err |= ALN_ERR_POINTS;
-          return 1;
-        }
-        if (lane == 0) {
-          atrace[atlen - 1] = (uint16_t)(b - a);
-          atrace[atlen - 2] = (uint16_t)(d - e);
-        }
-        atlen -= 2;
-      } else if (lane == 0) {
-        atrace[1] = (uint16_t)(atrace[1] + (b - a));
-        atrace[0] = (uint16_t)(atrace[0] + (d - e));
-      }
-      b = a;
-      e = d;
-    }
-    if (h >= 0) {
-      for (h = cells[h].ptr; h >= 0; h = cells[h].ptr) {
-        k = cells[h].diag;
-        a = cells[h].mark - k;
-        if (P.trace_off + atlen - 2 < 0) {
-          W.err |= ALN_ERR_POINTS;
-          return 1;
-        }
-        d = cells[h].diff;
-        if (lane == 0) {
-          atrace[atlen - 1] = (uint16_t)(b - a);
-          atrace[atlen - 2] = (uint16_t)(d - e);
-        }
-        atlen -= 2;
-        b = a;
-        e = d;
-      }
-      __syncwarp();
-      if (b + k != trimx) {
-        if (P.trace_off + atlen - 2 < 0) {
-          W.err |= ALN_ERR_POINTS;
-          return 1;
-        }
-        if (lane == 0) {
-          atrace[atlen - 1] = (uint16_t)(b - trimy);
-          atrace[atlen - 2] = (uint16_t)(trimd - e);
-        }
-        atlen -= 2;
-      } else if (b != trimy) {
-        if (lane == 0) {
-          atrace[atlen + 1] = (uint16_t)(atrace[atlen + 1] + (b - trimy));
-          atrace[atlen] = (uint16_t)(atrace[atlen] + (trimd - e));
-        }
-      }
-    }
-    __syncwarp();
+    P.tlen = (int)(2 * n);
+  } else {
     P.abpos = trimx;
     P.bbpos = trimy;
-    P.diffs = P.diffs + trimd;
-    P.tlen = P.tlen - atlen;
-    P.trace_off = P.trace_off + atlen;
+    P.diffs += trimd;
+    P.tlen += (int)(2 * n);
+    P.trace_off -= (int)(2 * n);
   }
   return 0;
 }
-
-#undef WVI
 
 // A path on the complemented A (and so on reversed B coordinates) in
 // forward coordinates: both intervals mirrored, and the trace-point pairs
@@ -1655,9 +912,10 @@ __device__ __forceinline__ int local_alignment_w(WarpWork &W, const AlignSpec &s
   const int maxp = hbord < 0 ? I32MAX : hgh + hbord;
   const int aoff = acomp ? A.len % spec.trace_space : 0;
 
-  if (forward_wave_w(W, spec, A, B, P, &low, hgh, anti, minp, maxp, aoff)) return 1;
+  int from = low;
+  if (extend(true, W, spec, A, B, P, from, hgh, anti, minp, maxp, aoff)) return 1;
   const bool fwd_away = (P.aepos + P.bepos) - anti >= DUB_TRIM;
-  if (reverse_wave_w(W, spec, A, B, P, low, low, anti, minp, maxp, aoff)) return 1;
+  if (extend(false, W, spec, A, B, P, from, from, anti, minp, maxp, aoff)) return 1;
   const bool rev_away = anti - (P.abpos + P.bbpos) >= DUB_TRIM;
 
   if (!fwd_away && !rev_away) {
@@ -1665,14 +923,15 @@ __device__ __forceinline__ int local_alignment_w(WarpWork &W, const AlignSpec &s
     P.bepos = P.bbpos = (P.bbpos + P.bepos) >> 1;
     P.tlen = 0;
   } else if (!fwd_away) {
-    int from = P.abpos - P.bbpos;
+    from = P.abpos - P.bbpos;
     P.tlen = 0;
-    if (forward_wave_w(W, spec, A, B, P, &from, from, P.abpos + P.bbpos, minp, maxp, aoff)) return 1;
+    if (extend(true, W, spec, A, B, P, from, from, P.abpos + P.bbpos, minp, maxp, aoff)) return 1;
   } else if (!rev_away) {
-    const int from = P.aepos - P.bepos, at = P.aepos + P.bepos;
+    from = P.aepos - P.bepos;
+    const int at = P.aepos + P.bepos;
     P.tlen = 0;
     P.diffs = 0;
-    if (reverse_wave_w(W, spec, A, B, P, from, from, at, minp, maxp, aoff)) return 1;
+    if (extend(false, W, spec, A, B, P, from, from, at, minp, maxp, aoff)) return 1;
   }
   if (acomp) path_to_forward(W.points + P.trace_off, A, B, P);
   return 0;

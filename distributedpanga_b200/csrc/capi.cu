@@ -115,8 +115,7 @@ struct pga_ctx {
   DBuf mlog_key, mlog_val, mlog_toff, mlog_trace, mlog_ctr;
   int64_t cap_calls = 0, cap_bytes = 0;
   // the scoring tables of the last alignment
-  std::vector<int16_t> spec_host;
-  int ave_path_host = 0;
+  int ave_path_host = 0, dscore_host = 0;
   int diag_passes[2] = {0, 0};
   SeedKeyLayout lay[2];
   bool have_diag[2] = {false, false};
@@ -127,7 +126,7 @@ struct pga_ctx {
   bool have_numeric = false;
   bool in_align = false;           // pga_align / pga_local_alignment hold the alignment buffers
   DBuf pk, poff, pwords;
-  DBuf numf, numr, soff, spec_tab, tasks, task_next, pout, wave, points, cells, cell_next, ovl, perm, cand,
+  DBuf numf, numr, soff, tasks, task_next, pout, wave, points, cells, cell_next, ovl, perm, cand,
       cand_next, recs, rec_next, outb, out_next, pflag, pidx, pstart, pab, rng_ovl, rng_next, ftasks, fout,
       ridx, rout, selfb, pstart2, pab2, small, shist, fo_dev, binfo[2], plive[2];
   // survivors in la_sort order on the device (srecs, their traces in strace,
@@ -179,8 +178,7 @@ struct pga_target {
   // they were made with.
   struct Memo {
     bool valid = false;
-    std::vector<int16_t> spec;
-    int ave_path = 0;
+    int ave_path = 0, dscore = 0;
     int64_t entries = 0, cap = 0;
     DBuf key, val, toff, trace;
   } memo;
@@ -1004,13 +1002,8 @@ int prepare_sequences(pga_ctx *ctx, int *ave_path) {
     }
     ctx->have_numeric = true;
   }
-  std::vector<int16_t> tab(2 * 32768);
-  *ave_path = aln::build_align_spec(ctx->base_freq, tab.data(), tab.data() + 32768);
-  ENSURE(ctx->spec_tab, sizeof(int16_t) * tab.size());
-  CK(cudaMemcpyAsync(ctx->spec_tab.p, tab.data(), sizeof(int16_t) * tab.size(), cudaMemcpyHostToDevice, ctx->st));
-  ctx->spec_host.swap(tab);  // (a pageable source is staged before the copy call returns)
+  *ave_path = aln::align_params(ctx->base_freq, &ctx->dscore_host);
   ctx->ave_path_host = *ave_path;
-
   return PGA_OK;
 }
 
@@ -1039,9 +1032,8 @@ int prepare_workspace(pga_ctx *ctx, AlignLaunch &L, int ave_path) {
   L.pk = P<uint64_t>(ctx->pk);
   L.poff = P<int64_t>(ctx->poff);
   L.pwords = P<int64_t>(ctx->pwords);
-  L.score = P<int16_t>(ctx->spec_tab);
-  L.table = P<int16_t>(ctx->spec_tab) + 32768;
   L.ave_path = ave_path;
+  L.dscore = ctx->dscore_host;
   L.amxpos = ctx->maxctg;
   L.maxdag = 2 * ctx->maxctg;
   L.nwarps = 148 * 20;  // work spaces for the five-CTA build's resident warps
@@ -1249,7 +1241,7 @@ int run_align(pga_ctx *ctx) {
   if (rt) {
     const pga_target::Memo &M = rt->memo;
     int why = M.valid ? 0 : 1;
-    if (!why && (M.spec != ctx->spec_host || M.ave_path != ctx->ave_path_host)) why = 3;
+    if (!why && (M.dscore != ctx->dscore_host || M.ave_path != ctx->ave_path_host)) why = 3;
     ctx->reuse_stats[3] = why;
     if (!why) {
       memo_on = true;
@@ -1777,7 +1769,7 @@ void pga_ctx_destroy(pga_ctx *ctx) {
   if (!ctx) return;
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->st);
-  DBuf *abufs[] = {&ctx->pk, &ctx->poff, &ctx->pwords, &ctx->numf, &ctx->numr, &ctx->soff, &ctx->spec_tab, &ctx->tasks, &ctx->task_next, &ctx->pout, &ctx->binfo[0], &ctx->binfo[1], &ctx->plive[0], &ctx->plive[1],
+  DBuf *abufs[] = {&ctx->pk, &ctx->poff, &ctx->pwords, &ctx->numf, &ctx->numr, &ctx->soff, &ctx->tasks, &ctx->task_next, &ctx->pout, &ctx->binfo[0], &ctx->binfo[1], &ctx->plive[0], &ctx->plive[1],
                    &ctx->wave, &ctx->points, &ctx->cells, &ctx->cell_next, &ctx->ovl, &ctx->perm, &ctx->cand,
                    &ctx->cand_next, &ctx->recs, &ctx->rec_next, &ctx->outb, &ctx->out_next, &ctx->pflag,
                    &ctx->pidx, &ctx->pstart, &ctx->pab, &ctx->rng_ovl, &ctx->rng_next, &ctx->ftasks,
@@ -2675,7 +2667,7 @@ int build_memo(pga_ctx *ctx, pga_target *t) {
   CK(cudaStreamSynchronize(ctx->st));
   M.cap = T.cap;
   M.entries = T.entries;
-  M.spec = ctx->spec_host;
+  M.dscore = ctx->dscore_host;
   M.ave_path = ctx->ave_path_host;
   M.valid = true;
   return PGA_OK;
