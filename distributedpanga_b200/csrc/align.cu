@@ -187,6 +187,7 @@ struct KeySeeds {
   }
 };
 
+template <bool BLOCKS>
 struct WarpAligner {
   WarpWork &W;
   const AlignSpec &spec;
@@ -230,7 +231,7 @@ struct WarpAligner {
         return 0;
       }
     }
-    const int r = local_alignment_w(W, spec, A, B, acomp, P, low, hgh, anti, lbord, hbord);
+    const int r = local_alignment_w<BLOCKS>(W, spec, A, B, acomp, P, low, hgh, anti, lbord, hbord);
     if (keyed && M.lkey && r == 0) {
       // the target's own run: append the call to the log
       unsigned long long e = 0, tb = 0;
@@ -382,7 +383,7 @@ __device__ int align_pair_dev(const KeySeeds &S, const uint16_t *info, bool comp
   if (bhi < 0 || bhi > n) bhi = n;
   if (blo < 0) blo = 0;
   if (blo >= bhi) return 0;
-  ChainSink<WarpAligner> K{comp, self, A, B, AL, path, O, R, lane, 32, amxpos, (int64_t)A.len + B.len,
+  ChainSink<Aligner> K{comp, self, A, B, AL, path, O, R, lane, 32, amxpos, (int64_t)A.len + B.len,
                            (int64_t)A.len - maxdag, (int64_t)A.len - amxpos, 0, 0, -1};
   int64_t pend = -1;  // the last band start seen, its block not yet decided
   int pend_sum = 0;
@@ -540,11 +541,13 @@ struct SmallSums {
 
 // The persistent alignment loop, in four builds: MINB = 1 keeps every
 // register a warp's wave loop wants (255, two CTAs per SM), for launches
-// bounded by their longest task; MINB = 3, 4 and 5 trade spills for more
+// bounded by their longest tasks; MINB = 3, 4 and 5 trade spills for more
 // resident warps (three to five CTAs per SM: 168, 128 or 96 registers), for
-// launches bounded by throughput (many pairs), where a wave step's latency
-// is hidden by the other warps of its SM (five: the 2 x 1 Gbp pair launch
-// 3.50 s against 3.70 with four).
+// launches bounded by throughput (many pairs with calls), where a wave step's
+// latency is hidden by the other warps of its SM.  The last two leave out the
+// register form of the waves of 32 to 124 diagonals (align_warp.cuh, extend).
+// 2 x 200 Mbp repeat-rich, two to five CTAs: 342, 298, 240, 224 ms of pair
+// phase; 2 x 41 kbp: 10.8, 11.1, 14.4, 14.8.
 template <int MINB>
 __global__ void __launch_bounds__(ALIGN_THREADS, MINB) k_align_pairs(AlignLaunch P) {
   __shared__ BlockSeed s_block[ALIGN_THREADS / 32][32];
@@ -589,7 +592,7 @@ __global__ void __launch_bounds__(ALIGN_THREADS, MINB) k_align_pairs(AlignLaunch
       bhi = next_band_start(S, tk.shi - tk.lo, S.n, lane);
     }
     PairResult R;
-    WarpAligner AL{W, spec, P.memo, tk.a, tk.b};
+    WarpAligner<(MINB <= 3)> AL{W, spec, P.memo, tk.a, tk.b};
     const uint16_t *info = (tk.comp ? P.infoC : P.infoN) + tk.lo;
     int rc = align_pair_dev(S, info, tk.comp != 0, tk.self != 0, A, B, P.amxpos, P.maxdag, AL, path, O, R, lane,
                             blo, bhi);
@@ -700,7 +703,7 @@ k_local_batch(AlignLaunch P) {
     Path path;
     path.tlen = path.diffs = path.abpos = path.bbpos = path.aepos = path.bepos = 0;
     path.trace_off = 0;
-    int status = local_alignment_w(W, spec, A, B, comp, path, q[3], q[4], q[5], q[6], q[7]) ? (W.err | 0x100) : 0;
+    int status = local_alignment_w<true>(W, spec, A, B, comp, path, q[3], q[4], q[5], q[6], q[7]) ? (W.err | 0x100) : 0;
     int64_t off = -1;
     if (status == 0 && path.tlen > 0) {
       unsigned long long o = 0;

@@ -19,7 +19,9 @@
 //   lasta / trim*       the last record that passes the path-average and the
 //                       trim tests, found going back through the records
 //   aclip / bclip       the lowest diagonal that met A's end, the highest
-//                       that met B's
+//                       that met B's (what the reference keeps of them beyond
+//                       the clip, mor*, is read only with reach set; the
+//                       driver's specification has it 0)
 //   pebbles             slot numbers only name pebbles, so they are taken in
 //                       lane order from a global pool
 //
@@ -161,7 +163,7 @@ struct Wave {
   int sg;    // 1 forward, -1 reverse
   int low, hgh, dif, cur;
   int besta, bestx, lasta, trima, trimx, trimd, trimha;
-  int more, morem, morea, morex, mored, moreha;
+  int more;
 };
 
 // Snake along diagonal k from x in rounds of 16 * N bases: stops at the first
@@ -290,18 +292,6 @@ __device__ __forceinline__ void take_records(Wave &S, int &besta, int &lasta, co
   } else
     earlier_records(S, lasta, trim, act, k, c, b, ha, dif, besta, kr, pass);
   besta = rc;
-}
-
-// A path that met a sequence's end on a clipped diagonal.
-__device__ __forceinline__ void note_end(Wave &S, int kc, uint64_t t, int c, int ha, int dif) {
-  const int m = hist_ones(t);
-  if (S.morem <= m) {
-    S.morem = m;
-    S.morea = c;
-    S.morex = (c + kc) >> 1;
-    S.mored = dif;
-    S.moreha = ha;
-  }
 }
 
 // Whether the furthest path can still grow (neither sequence's end reached).
@@ -452,16 +442,8 @@ __device__ __forceinline__ int narrow_waves(WarpWork &W, Wave &io, int stop) {
         const int ka = __reduce_min_sync(FULL, hit && !hb ? k : I32MAX);
         const int kb = __reduce_max_sync(FULL, hit && hb ? k : NO_WAVE);
         S.more = can_grow(S, rc);
-        if (ka != I32MAX) {
-          hgh = ka - 1;
-          note_end(S, ka, __shfl_sync(FULL, T, ka & 31), __shfl_sync(FULL, c, ka & 31),
-                   __shfl_sync(FULL, HA, ka & 31), dif);
-        }
-        if (kb != NO_WAVE) {
-          low = kb + 1;
-          note_end(S, kb, __shfl_sync(FULL, T, kb & 31), __shfl_sync(FULL, c, kb & 31),
-                   __shfl_sync(FULL, HA, kb & 31), dif);
-        }
+        if (ka != I32MAX) hgh = ka - 1;
+        if (kb != NO_WAVE) low = kb + 1;
       }
     }
     besta = rc;
@@ -497,15 +479,268 @@ __device__ __forceinline__ int narrow_waves(WarpWork &W, Wave &io, int stop) {
 }
 
 // ---------------------------------------------------------------------------
-// Wide waves: the ring in memory (L1-resident at the widths that occur), 32
-// diagonals per pass from the highest down.  The waves past an alignment's
-// end run here: they widen by two diagonals per step until the trim lag ends
-// the loop.  Runs until the loop ends, the window narrows to WIDE_OUT
-// diagonals, or the wave count reaches `stop`.
+// Block waves, at most J * 31 diagonals: lane l holds the J diagonals of one
+// aligned block, blocks dealt to the lanes in turn, all state in registers;
+// only the blocks' edges come by shuffle.  The waves past an alignment's end
+// run here: they widen by two diagonals per step until the trim lag ends the
+// loop, nearly all snakes stopping at once, so a step is the fixed work per
+// diagonal; a lane's J independent diagonals overlap in it where passes of 32
+// through memory would follow one another.  Runs until the loop ends, the
+// window narrows to BLOCK_OUT diagonals or no longer fits, or the wave count
+// reaches `stop`.
 // ---------------------------------------------------------------------------
-constexpr int WIDE_OUT = 20;
+constexpr int BLOCK = 4;
+constexpr int BLOCK_OUT = 20;
 
-__device__ __forceinline__ int wide_waves(WarpWork &W, Wave &io, int stop) {
+// v[j] for a per-lane index j < J, without local memory
+template <int J, class T>
+__device__ __forceinline__ T pick(const T (&v)[J], int j) {
+  T r = v[0];
+#pragma unroll
+  for (int q = 1; q < J; q++)
+    if (j == q) r = v[q];
+  return r;
+}
+
+template <int J>
+__device__ __forceinline__ int block_waves(WarpWork &W, Wave &io, int stop) {
+  constexpr int LG = J == 2 ? 1 : 2;
+  static_assert(J == 1 << LG, "J is 2 or 4");
+  const int lane = threadIdx.x & 31;
+  const int lup = (lane + 1) & 31, ldn = (lane - 1) & 31;
+  Wave S = io;
+  const TrimTest trim(S.dscore);
+  const int vmask = W.vcap - 1;
+  int next = (int)W.chunk_next, end = (int)W.chunk_end;
+  int ncells = 0;
+  int low = S.low, hgh = S.hgh, dif = S.dif, besta = S.besta, lasta = S.lasta;
+  bool full = false;
+
+  int V[J], HA[J], HM[J], NA[J];
+  uint64_t T[J];
+  int kw = ((low >> LG) + ((lane - (low >> LG)) & 31)) << LG;  // the lane's first diagonal
+#pragma unroll
+  for (int j = 0; j < J; j++) {
+    const int k = kw + j;
+    V[j] = NO_WAVE;
+    HA[j] = -1;
+    HM[j] = NA[j] = 0;
+    T[j] = 0;
+    if (k >= low && k <= hgh) {
+      const RingCell c = W.C[S.cur][k & vmask];
+      V[j] = W.V[S.cur][k & vmask];
+      NA[j] = W.NA[k & vmask];
+      T[j] = c.T;
+      HA[j] = c.HA;
+      HM[j] = c.HM;
+    }
+  }
+  while (true) {
+    const int nlow = max(low - 1, S.minp), nhgh = min(hgh + 1, S.maxp);
+    const int wide = nhgh - nlow;
+    if (!(S.more && lasta >= besta - TRIM_MLAG && low <= hgh && wide < J * NARROW && wide >= BLOCK_OUT && dif < stop))
+      break;
+    dif += 1;
+    ncells += wide + 1;
+    const int bl = nlow >> LG;
+    kw = (bl + ((lane - bl) & 31)) << LG;
+
+    // start points and what comes with them
+    const int nlo = __shfl_sync(FULL, pick<J>(NA, low & (J - 1)), (low >> LG) & 31);
+    const int nhi = __shfl_sync(FULL, pick<J>(NA, hgh & (J - 1)), (hgh >> LG) & 31);
+    const int vup = __shfl_sync(FULL, V[0], lup), vdn = __shfl_sync(FULL, V[J - 1], ldn);
+    const int hau = __shfl_sync(FULL, HA[0], lup), had = __shfl_sync(FULL, HA[J - 1], ldn);
+    const int hmu = __shfl_sync(FULL, HM[0], lup), hmd = __shfl_sync(FULL, HM[J - 1], ldn);
+    const uint64_t tu = __shfl_sync(FULL, T[0], lup), td = __shfl_sync(FULL, T[J - 1], ldn);
+    int x[J], run[J], mx[J];
+    bool act[J], go[J];
+    {
+      int ha[J], hm[J];
+      uint64_t t[J];
+#pragma unroll
+      for (int j = 0; j < J; j++) {
+        const int jp = j < J - 1 ? j + 1 : j, jm = j > 0 ? j - 1 : j, k = kw + j;
+        const int ap = j < J - 1 ? V[jp] : vup, am = j > 0 ? V[jm] : vdn;
+        const bool up = ap > max(V[j], am), dn = !up && am > V[j];
+        x[j] = ((up ? ap + 1 : (dn ? am + 1 : V[j] + 2)) + k) >> 1;
+        ha[j] = up ? (j < J - 1 ? HA[jp] : hau) : (dn ? (j > 0 ? HA[jm] : had) : HA[j]);
+        hm[j] = up ? (j < J - 1 ? HM[jp] : hmu) : (dn ? (j > 0 ? HM[jm] : hmd) : HM[j]);
+        t[j] = up ? (j < J - 1 ? T[jp] : tu) : (dn ? (j > 0 ? T[jm] : td) : T[j]);
+        act[j] = k >= nlow && k <= nhgh;
+        NA[j] = k < low ? nlo : (k > hgh ? nhi : NA[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < J; j++) {
+        HA[j] = ha[j];
+        HM[j] = hm[j];
+        T[j] = t[j];
+      }
+    }
+
+    // snakes: 32 bases each, then the few that go on
+    bool more32 = false;
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+      const int k = kw + j, ia = x[j] + S.offA, ib = x[j] - k + S.offB;
+      mx[j] = min(S.limA - x[j], S.limB - x[j] + k);
+      go[j] = act[j] && (mx[j] | ia | ib) >= 0;
+      run[j] = 0;
+      if (go[j]) run[j] = match_words<2>(S.pa + (ia >> 4), (ia & 15) << 1, S.pb + (ib >> 4), (ib & 15) << 1);
+      more32 |= run[j] == 32 && mx[j] > 32;
+    }
+    if (more32) {
+#pragma unroll 1
+      for (int j = 0; j < J; j++) {
+        int t = pick<J>(run, j);
+        const int xj = pick<J>(x, j), m = pick<J>(mx, j), ia = xj + S.offA, ib = xj - kw - j + S.offB;
+        for (int r = t; r == 32 && t < m; t += r)
+          r = match_words<2>(S.pa + ((ia + t) >> 4), ((ia + t) & 15) << 1, S.pb + ((ib + t) >> 4),
+                             ((ib + t) & 15) << 1);
+#pragma unroll
+        for (int q = 0; q < J; q++)
+          if (q == j) run[q] = t;
+      }
+    }
+
+    bool hit = false, cross = false;
+    int key = 0, c[J];
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+      const int k = kw + j;
+      run[j] = min(run[j], max(mx[j], 0));
+      hit |= act[j] && (!go[j] || run[j] == mx[j]);
+      T[j] = hist_step(T[j], run[j]);
+      x[j] += run[j];
+      c[j] = (x[j] << 1) - k;
+      cross |= act[j] && x[j] >= NA[j];
+      const int past = min(max(c[j] - besta, 0), PAST_MAX >> 2);
+      if (act[j]) key = max(key, (past << 7) + (k - nlow));
+    }
+    if (__any_sync(FULL, cross)) {
+#pragma unroll
+      for (int j = 0; j < J; j++)
+        full |= !drop_pebbles(W, S, act[j], kw + j, x[j], dif, HA[j], HM[j], NA[j], next, end);
+      if (full) break;
+    }
+
+    // the record: the highest diagonal of the wave's best
+    key = __reduce_max_sync(FULL, key);
+    if (key >= 128) {
+      const int carry = besta;
+      int rc = besta + (key >> 7), kr = nlow + (key & 127);
+      if (key >= (PAST_MAX >> 2) << 7) {
+        int m = NO_WAVE, mk = NO_WAVE;
+#pragma unroll
+        for (int j = 0; j < J; j++) m = max(m, act[j] ? c[j] : NO_WAVE);
+        rc = __reduce_max_sync(FULL, m);
+#pragma unroll
+        for (int j = 0; j < J; j++)
+          if (act[j] && c[j] == rc) mk = kw + j;
+        kr = __reduce_max_sync(FULL, mk);
+      }
+      besta = rc;
+      S.bestx = (rc + kr) >> 1;
+      bool passed = false;
+      while (true) {
+        const int L = (kr >> LG) & 31, q = kr & (J - 1);
+        const uint64_t t = __shfl_sync(FULL, pick<J>(T, q), L);
+        if (hist_ones(t) >= S.ave_path) {
+          if (!passed) lasta = rc;
+          passed = true;
+          if (trim(t)) {
+            S.trima = rc;
+            S.trimx = (rc + kr) >> 1;
+            S.trimd = dif;
+            S.trimha = __shfl_sync(FULL, pick<J>(HA, q), L);
+            break;
+          }
+        }
+        // an earlier record (a higher diagonal), if one could pass
+        bool good = false;
+        int m = NO_WAVE, mk = NO_WAVE;
+#pragma unroll
+        for (int j = 0; j < J; j++)
+          if (act[j] && kw + j > kr && c[j] > carry) {
+            good |= hist_ones(T[j]) >= S.ave_path;
+            m = max(m, c[j]);
+          }
+        if (!__any_sync(FULL, good)) break;
+        rc = __reduce_max_sync(FULL, m);
+#pragma unroll
+        for (int j = 0; j < J; j++)
+          if (act[j] && kw + j > kr && c[j] == rc) mk = kw + j;
+        kr = __reduce_max_sync(FULL, mk);
+      }
+    }
+
+    low = nlow;
+    hgh = nhgh;
+    if (__any_sync(FULL, hit)) {
+      // snakes that reached a sequence's end clip the window
+      int ka = I32MAX, kb = NO_WAVE;
+#pragma unroll
+      for (int j = 0; j < J; j++)
+        if (act[j] && (!go[j] || run[j] == mx[j])) {
+          if (met_b(S, x[j] - run[j], kw + j, go[j])) kb = max(kb, kw + j);
+          else ka = min(ka, kw + j);
+        }
+      ka = __reduce_min_sync(FULL, ka);
+      kb = __reduce_max_sync(FULL, kb);
+      S.more = can_grow(S, besta);
+      if (ka != I32MAX) hgh = ka - 1;
+      if (kb != NO_WAVE) low = kb + 1;
+    }
+    // WAVE_LAG pruning from either end, between the clipped ends
+    int kmin = I32MAX, kmax = NO_WAVE;
+#pragma unroll
+    for (int j = 0; j < J; j++)
+      if (kw + j >= low && kw + j <= hgh && c[j] >= besta - WAVE_LAG) {
+        kmin = min(kmin, kw + j);
+        kmax = max(kmax, kw + j);
+      }
+    kmin = __reduce_min_sync(FULL, kmin);
+    kmax = __reduce_max_sync(FULL, kmax);
+    if (kmin <= kmax) {
+      low = kmin;
+      hgh = kmax;
+    } else
+      hgh = low - 1;
+#pragma unroll
+    for (int j = 0; j < J; j++) V[j] = kw + j >= low && kw + j <= hgh ? c[j] : NO_WAVE;
+  }
+  W.waves += dif - S.dif;
+  W.cells += ncells;
+  W.chunk_next = next;
+  W.chunk_end = end;
+  if (full) {
+    W.err |= ALN_ERR_CELLS;
+    return 1;
+  }
+#pragma unroll
+  for (int j = 0; j < J; j++) {
+    const int k = kw + j;
+    if (k >= low && k <= hgh) {
+      W.V[S.cur][k & vmask] = V[j];
+      W.C[S.cur][k & vmask] = RingCell{T[j], HA[j], HM[j]};
+      W.NA[k & vmask] = NA[j];
+    }
+  }
+  __syncwarp();
+  S.low = low;
+  S.hgh = hgh;
+  S.dif = dif;
+  S.besta = besta;
+  S.lasta = lasta;
+  io = S;
+  return 0;
+}
+
+// ---------------------------------------------------------------------------
+// Wide waves: the ring in memory (L1-resident at the widths that occur), 32
+// diagonals per pass from the highest down.  Runs until the loop ends, the
+// window has at most `least` diagonals, or the wave count reaches `stop`.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ int wide_waves(WarpWork &W, Wave &io, int stop, int least) {
   const int lane = threadIdx.x & 31;
   Wave S = io;
   const TrimTest trim(S.dscore);
@@ -514,7 +749,7 @@ __device__ __forceinline__ int wide_waves(WarpWork &W, Wave &io, int stop) {
   const int dif0 = S.dif;
   int ncells = 0, err = 0;
   while (S.more && S.lasta >= S.besta - TRIM_MLAG) {
-    if (S.hgh - S.low < WIDE_OUT || S.dif >= stop) break;
+    if (S.hgh - S.low < least || S.dif >= stop) break;
     if (S.hgh - S.low + 5 > W.vcap) {
       err = ALN_ERR_VCAP;
       break;
@@ -586,16 +821,8 @@ __device__ __forceinline__ int wide_waves(WarpWork &W, Wave &io, int stop) {
     __syncwarp();
     if (ka != I32MAX || kb != NO_WAVE) {
       S.more = can_grow(S, S.besta);
-      if (ka != I32MAX) {
-        S.hgh = ka - 1;
-        const RingCell q = Cn[ka & vmask];
-        note_end(S, ka, q.T, Vn[ka & vmask], q.HA, S.dif);
-      }
-      if (kb != NO_WAVE) {
-        S.low = kb + 1;
-        const RingCell q = Cn[kb & vmask];
-        note_end(S, kb, q.T, Vn[kb & vmask], q.HA, S.dif);
-      }
+      if (ka != I32MAX) S.hgh = ka - 1;
+      if (kb != NO_WAVE) S.low = kb + 1;
     }
     // WAVE_LAG pruning from either end
     if (S.hgh >= S.low) {
@@ -636,7 +863,13 @@ __device__ __forceinline__ int wide_waves(WarpWork &W, Wave &io, int stop) {
 // forward_wave (fwd) or reverse_wave of a path, out of line: one copy of the
 // code serves both directions and every call.  `start` is the forward wave's
 // lowest diagonal on entry and, on return, the diagonal the path starts on.
+// BLOCKS: waves of 32 to 124 diagonals run in registers (block_waves), for
+// launches bounded by their longest calls (2 x 41 kbp: pair phase 10.8 ms
+// against 14.9 through memory); without, they too run as passes
+// (wide_waves), for launches bounded by throughput, where the smaller loop
+// and its registers pay (2 x 200 Mbp repeat-rich: 224 ms against 278).
 // Returns 1 on a work-space overflow (W.err set).
+template <bool BLOCKS>
 __device__ __noinline__ int extend(const bool fwd, WarpWork &W, const AlignSpec &spec, const Seq &A, const Seq &B,
                                    Path &P, int &start, int maxd, int mida, int minp, int maxp, int aoff) {
   const int lane = threadIdx.x & 31;
@@ -663,11 +896,10 @@ __device__ __noinline__ int extend(const bool fwd, WarpWork &W, const AlignSpec 
   S.low = fwd ? start : -maxd;
   S.hgh = fwd ? maxd : -start;
   S.dif = S.cur = 0;
-  S.besta = S.lasta = S.trima = S.morea = S.sg * mida;
-  S.bestx = S.trimx = S.morex = S.sg * ((mida + maxd) >> 1);
-  S.trimd = S.mored = S.trimha = S.moreha = 0;
+  S.besta = S.lasta = S.trima = S.sg * mida;
+  S.bestx = S.trimx = S.sg * ((mida + maxd) >> 1);
+  S.trimd = S.trimha = 0;
   S.more = 1;
-  S.morem = -1;
   int64_t call_base = -1;  // this call's first pebble: the reference's cells[0]
 
   // 0-wave: diagonals visited from the highest down
@@ -698,7 +930,7 @@ __device__ __noinline__ int extend(const bool fwd, WarpWork &W, const AlignSpec 
     if (pb0 < 0) return 1;
     if (call_base < 0) {
       call_base = pb0;
-      S.trimha = S.moreha = (int)pb0;
+      S.trimha = (int)pb0;
     }
     int ha = (int)pb0 + off;
     if (act) {
@@ -730,16 +962,8 @@ __device__ __noinline__ int extend(const bool fwd, WarpWork &W, const AlignSpec 
   __syncwarp();
   if (ka != I32MAX || kb != NO_WAVE) {
     S.more = can_grow(S, S.besta);
-    if (ka != I32MAX) {
-      S.hgh = ka - 1;
-      const RingCell q = W.C[0][ka & vmask];
-      note_end(S, ka, PATH_INT, W.V[0][ka & vmask], q.HA, 0);
-    }
-    if (kb != NO_WAVE && S.low <= kb) {
-      S.low = kb + 1;
-      const RingCell q = W.C[0][kb & vmask];
-      note_end(S, kb, PATH_INT, W.V[0][kb & vmask], q.HA, 0);
-    }
+    if (ka != I32MAX) S.hgh = ka - 1;
+    if (kb != NO_WAVE) S.low = kb + 1;
   }
 
   const int max_waves = A.len + B.len + 1024;
@@ -764,20 +988,18 @@ __device__ __noinline__ int extend(const bool fwd, WarpWork &W, const AlignSpec 
         stop = min(stop, W.long_waves - 1);
     }
     const int width = S.hgh - S.low + 1 + (S.low > S.minp ? 1 : 0) + (S.hgh < S.maxp ? 1 : 0);
-    if (width > NARROW ? wide_waves(W, S, stop) : narrow_waves(W, S, stop)) return 1;
+    int r;
+    if (width <= NARROW) r = narrow_waves(W, S, stop);
+    else if (BLOCKS && width <= BLOCK * NARROW) r = block_waves<BLOCK>(W, S, stop);
+    else r = wide_waves(W, S, stop, BLOCKS ? BLOCK * NARROW - 8 : BLOCK_OUT);
+    if (r) return 1;
   }
   __syncwarp();
 
   // Trace-back, from the path's tip to its start: one pebble per step, read
   // whole.  Lane 0 writes each interval's (diffs, b-delta) to the free end of
   // the trace buffer; the warp then moves them next to the path's start.
-  int trimx = S.sg * S.trimx, trimy = S.sg * S.trima - trimx, trimd = S.trimd, h = S.trimha;
-  if (S.morem >= 0 && spec.reach) {
-    trimx = S.sg * S.morex;
-    trimy = S.sg * S.morea - trimx;
-    trimd = S.mored;
-    h = S.moreha;
-  }
+  const int trimx = S.sg * S.trimx, trimy = S.sg * S.trima - trimx, trimd = S.trimd, h = S.trimha;
   const int64_t t0 = P.trace_off;
   const int64_t room = (fwd ? W.point_cap - t0 : t0) >> 1;  // intervals the free end holds
   const int64_t lim = W.chunk_next - call_base + 1;
@@ -898,6 +1120,7 @@ __device__ __forceinline__ void path_to_forward(uint16_t *trace, const Seq &A, c
 // start, a reverse re-run counts its differences afresh).  With `acomp` A is
 // the complemented contig and the path comes back in forward coordinates.
 // Returns 1 on a work-space overflow (W.err says which).
+template <bool BLOCKS>
 __device__ __forceinline__ int local_alignment_w(WarpWork &W, const AlignSpec &spec, const Seq &A, const Seq &B,
                                                  bool acomp, Path &P, int low, int hgh, int anti, int lbord,
                                                  int hbord) {
@@ -913,9 +1136,9 @@ __device__ __forceinline__ int local_alignment_w(WarpWork &W, const AlignSpec &s
   const int aoff = acomp ? A.len % spec.trace_space : 0;
 
   int from = low;
-  if (extend(true, W, spec, A, B, P, from, hgh, anti, minp, maxp, aoff)) return 1;
+  if (extend<BLOCKS>(true, W, spec, A, B, P, from, hgh, anti, minp, maxp, aoff)) return 1;
   const bool fwd_away = (P.aepos + P.bepos) - anti >= DUB_TRIM;
-  if (extend(false, W, spec, A, B, P, from, from, anti, minp, maxp, aoff)) return 1;
+  if (extend<BLOCKS>(false, W, spec, A, B, P, from, from, anti, minp, maxp, aoff)) return 1;
   const bool rev_away = anti - (P.abpos + P.bbpos) >= DUB_TRIM;
 
   if (!fwd_away && !rev_away) {
@@ -925,13 +1148,13 @@ __device__ __forceinline__ int local_alignment_w(WarpWork &W, const AlignSpec &s
   } else if (!fwd_away) {
     from = P.abpos - P.bbpos;
     P.tlen = 0;
-    if (extend(true, W, spec, A, B, P, from, from, P.abpos + P.bbpos, minp, maxp, aoff)) return 1;
+    if (extend<BLOCKS>(true, W, spec, A, B, P, from, from, P.abpos + P.bbpos, minp, maxp, aoff)) return 1;
   } else if (!rev_away) {
     from = P.aepos - P.bepos;
     const int at = P.aepos + P.bepos;
     P.tlen = 0;
     P.diffs = 0;
-    if (extend(false, W, spec, A, B, P, from, from, at, minp, maxp, aoff)) return 1;
+    if (extend<BLOCKS>(false, W, spec, A, B, P, from, from, at, minp, maxp, aoff)) return 1;
   }
   if (acomp) path_to_forward(W.points + P.trace_off, A, B, P);
   return 0;

@@ -1093,10 +1093,11 @@ int prepare_workspace(pga_ctx *ctx, AlignLaunch &L, int ave_path) {
   return PGA_OK;
 }
 
-// Pairs beyond which the alignment launch uses k_align_pairs_wide: 2 x 100 Mbp
-// (10 K pairs) is 5 % faster with <2>, 2 x 1 Gbp (101 M pairs) 19 % faster
-// with <3>.
-constexpr int64_t ALIGN_MANY_PAIRS = 1 << 20;
+// Device-planned pairs that can make a call beyond which the alignment launch
+// is bounded by throughput and takes the five-CTA build: 2 x 20 Mbp
+// repeat-rich (0.19 M tasks in all) takes 65 ms of pair phase with two CTAs
+// and 75 with five, 2 x 200 Mbp (1.4 M) 342 and 224.
+constexpr int64_t ALIGN_MANY_PAIRS = 1 << 19;
 
 // Frees what the alignment no longer reads once both diagonal sorts are done
 // -- the index (records, LCPs, entries, scratch) and the unsorted seeds -- so
@@ -1383,9 +1384,9 @@ int run_align(pga_ctx *ctx) {
     L.nseeds[u] = ctx->nseed[u];
   }
   L.fo_pos = fo_pos;
-  // the launch is bounded by its longest tasks up to about a million pairs,
-  // by throughput beyond: then the build with more resident warps
-  L.min_blocks = ctx->align_build ? ctx->align_build : npairs[0] + npairs[1] > ALIGN_MANY_PAIRS ? 5 : 2;
+  // the launch is bounded by its longest tasks up to about half a million
+  // pairs, by throughput beyond: then the build with more resident warps
+  L.min_blocks = ctx->align_build ? ctx->align_build : nsmall > ALIGN_MANY_PAIRS ? 5 : 2;
   L.sred = sred;
   L.fo_last = sred + 8;
   L.fo_earlier = sred + 8 + nc;
