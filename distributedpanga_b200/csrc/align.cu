@@ -500,6 +500,7 @@ __device__ __forceinline__ PairTask small_task(const AlignLaunch &P, uint64_t co
   t.self = 0;
   t.entry_bepos = 0;
   t.seg = -1;
+  t.step = 0;
   t.lo = P.pstart[u][p];
   t.hi = p + 1 < P.npairs[u] ? P.pstart[u][p + 1] : P.nseeds[u];
   t.slo = t.lo;
@@ -507,11 +508,33 @@ __device__ __forceinline__ PairTask small_task(const AlignLaunch &P, uint64_t co
   return t;
 }
 
-// A warp's running reduction of its device-planned pairs' outcomes (lane 0).
-struct SmallSums {
+// Task t's pair or part of a pair among the planned ones: the last whose
+// first task is not past t, found by 32 probes a step; a range's own bounds.
+__device__ PairTask planned_task(const AlignLaunch &P, unsigned t, int lane, int *item) {
+  int lo = 0, n = P.nitems;
+  while (n > 1) {
+    const int at = lo + (int)(((int64_t)n * lane) >> 5);
+    const unsigned le = __ballot_sync(FULL, P.tfirst[at] <= t);  // lane 0's always is
+    const int f = 31 - __clz(le);
+    const int nlo = lo + (int)(((int64_t)n * f) >> 5), nhi = lo + (int)(((int64_t)n * (f + 1)) >> 5);
+    lo = nlo;
+    n = nhi - nlo;
+  }
+  PairTask tk = P.tasks[lo];
+  if (tk.seg >= 0) {
+    const int r = (int)(t - P.tfirst[lo]);
+    tk.slo += r * tk.step;
+    tk.shi = min(tk.shi, tk.slo + tk.step);
+    tk.seg += r;
+  }
+  *item = lo;
+  return tk;
+}
+
+// A warp's running reduction of its tasks' outcomes (lane 0).
+struct TaskSums {
   unsigned long long calls = 0, cycles = 0, maxkey = 0, err = 0, waves = 0, cells = 0, bad = ~0ull;
-  __device__ void add(const AlignLaunch &P, const PairTask &tk, const PairOut &po, unsigned t) {
-    calls += (unsigned long long)po.calls;
+  __device__ void add(const PairOut &po, unsigned t) {
     cycles += (unsigned long long)po.cycles;
     const unsigned long long k = ((unsigned long long)po.cycles << 16) | (unsigned)min(po.calls, 65535);
     maxkey = k > maxkey ? k : maxkey;
@@ -521,6 +544,10 @@ struct SmallSums {
     }
     waves += (unsigned long long)po.waves;
     cells += (unsigned long long)po.cells;
+  }
+  // a device-planned pair: its calls, and FastGA's order keys
+  __device__ void add_small(const AlignLaunch &P, const PairTask &tk, const PairOut &po) {
+    calls += (unsigned long long)po.calls;
     if (tk.comp == 0 && po.calls > 0) {
       const int xa = P.fo_pos[tk.a], xb = P.fo_pos[tk.b];
       const unsigned long long key = ((unsigned long long)(xb + 1) << 32) | (uint32_t)po.exit_bepos;
@@ -558,7 +585,7 @@ __global__ void __launch_bounds__(ALIGN_THREADS, MINB) k_align_pairs(AlignLaunch
   WarpWork W = warp_work(P, wid);
 
   OvlArena O = warp_arena(P, wid);
-  SmallSums sums;
+  TaskSums sums;
 
   while (true) {
     unsigned t = 0;
@@ -574,7 +601,9 @@ __global__ void __launch_bounds__(ALIGN_THREADS, MINB) k_align_pairs(AlignLaunch
     if (lane == 0) t = atomicAdd(P.next_task, 1u);
     t = __shfl_sync(FULL, t, 0);
     if (t >= (unsigned)P.ntasks + (unsigned)P.nsmall) break;
-    const PairTask tk = t < (unsigned)P.ntasks ? P.tasks[t] : small_task(P, P.small[t - P.ntasks]);
+    int item = 0;
+    const PairTask tk = t < (unsigned)P.ntasks ? planned_task(P, t, lane, &item)
+                                               : small_task(P, P.small[t - P.ntasks]);
     W.err = 0;
     O.err = 0;
     const SeedKeyLayout &L = tk.comp ? P.layC : P.layN;
@@ -627,12 +656,13 @@ __global__ void __launch_bounds__(ALIGN_THREADS, MINB) k_align_pairs(AlignLaunch
       po.cycles = clock64() - t0;
     }
     if (lane == 0) {
-      if (t < (unsigned)P.ntasks) P.pout[t] = po;
-      else sums.add(P, tk, po, t);
+      sums.add(po, t);
+      if (t >= (unsigned)P.ntasks) sums.add_small(P, tk, po);
+      else if (tk.seg < 0) P.pout[item] = po;
     }
     __syncwarp();
   }
-  if (lane == 0 && P.nsmall > 0) sums.flush(P);
+  if (lane == 0) sums.flush(P);
   if (lane == 0 && W.la_cycles > 0) atomicAdd(&P.prof[0], (unsigned long long)W.la_cycles);
 }
 
@@ -660,19 +690,30 @@ k_finish_pairs(AlignLaunch P) {
     po.err = 0;
     O.nov = 0;
     O.err = 0;
-    for (int k = 0; k < ft.nseg; k++) {
-      const PairOut ro = P.rout[P.range_idx[ft.first + k]];
-      po.calls += ro.calls;
-      if (ro.calls > 0) po.exit_bepos = ro.exit_bepos;
-      if (O.nov + ro.nsurv > O.ovl_cap) {
-        po.err = ALN_ERR_OVLS | 0x1000;
-        break;
+    for (int piece = 0; piece < 3 && po.err == 0; piece++)
+      for (int base = 0; base < ft.nseg[piece]; base += 32) {
+        const bool in = base + lane < ft.nseg[piece];
+        const PairOut *ro = P.rout + ft.first[piece] + base + (in ? lane : 0);
+        const int calls = in ? ro->calls : 0, bepos = ro->exit_bepos, nsurv = in ? ro->nsurv : 0;
+        const int64_t off = ro->rec_off;
+        po.calls += __reduce_add_sync(FULL, calls);
+        const unsigned called = __ballot_sync(FULL, calls > 0);
+        if (called) po.exit_bepos = __shfl_sync(FULL, bepos, 31 - __clz(called));
+        unsigned have = ft.emit ? __ballot_sync(FULL, nsurv > 0) : 0;
+        for (; have; have &= have - 1) {
+          const int l = __ffs(have) - 1, ns = __shfl_sync(FULL, nsurv, l);
+          const int64_t from = __shfl_sync(FULL, off, l);
+          if (O.nov + ns > O.ovl_cap) {
+            po.err = ALN_ERR_OVLS | 0x1000;
+            break;
+          }
+          for (int q = lane; q < ns; q += 32) O.ovl[O.nov + q] = P.rng_ovl[from + q];
+          O.nov += ns;
+        }
+        if (po.err) break;
       }
-      for (int q = lane; q < ro.nsurv; q += 32) O.ovl[O.nov + q] = P.rng_ovl[ro.rec_off + q];
-      O.nov += ro.nsurv;
-    }
     __syncwarp();
-    if (po.err == 0) finish_and_emit(P, O, ft.a, ft.b, ft.comp, po, lane);
+    if (po.err == 0 && ft.emit) finish_and_emit(P, O, ft.a, ft.b, ft.comp, po, lane);
     po.cycles = clock64() - t0;
     if (lane == 0) P.pout[t] = po;
     __syncwarp();

@@ -13,14 +13,18 @@ constexpr int ALIGN_THREADS = 128;  // 4 warps per CTA, one pair per warp at a t
 constexpr int WAVE_INTS = 11;       // per diagonal slot: RingCell x2, V x2, NA
 
 // One (anchor, partner) pair of a unit: seeds [lo, hi) of the unit's sorted
-// keys.  seg < 0: the whole pair, finished by the same warp.  seg >= 0: band
-// range number seg of a pair run in ranges: the band blocks whose first
-// stream starts in [slo, shi), both moved forward to the next band start;
-// its candidates go to the range store, its PairOut to rout[seg], and
-// k_finish_pairs finishes the pair later.
+// keys.  seg < 0: the whole pair, one task, finished by the same warp.  seg >=
+// 0: part of a pair as band ranges, one task each: range r, number seg + r,
+// holds the band blocks whose first stream starts in [slo + r step, slo + (r +
+// 1) step) up to shi, both ends moved forward to the next band start; its
+// candidates go to the range store, its PairOut to rout[seg + r], and
+// k_finish_pairs finishes the pair later.  The ranges are not written out:
+// a launch has hundreds of thousands, and laying them out on the host and
+// copying them and their outcomes took longer than many of its alignments.
 struct PairTask {
   int comp, a, b, self, entry_bepos, seg;
-  int64_t lo, hi, slo, shi;
+  int64_t lo, hi, slo, shi, step;
+  int64_t tasks() const { return seg < 0 ? 1 : (shi - slo + step - 1) / step; }
 };
 
 // Per task.  For a range task nsurv is its candidate count and rec_off the
@@ -32,10 +36,12 @@ struct PairOut {
   int64_t waves, cells;  // wave steps of its Local_Alignment calls, and their diagonals
 };
 
-// A pair run in ranges: its ranges, in order, are range_idx[first ..
-// first + nseg).
+// A pair run in ranges: its ranges, in order, are three runs of range numbers
+// (a self pair's parts below, on and above the diagonal; one run otherwise).
+// Without `emit` only the ranges' calls and last bepos are combined.
 struct FinishTask {
-  int comp, a, b, entry_bepos, first, nseg;
+  int comp, a, b, entry_bepos, emit;
+  int first[3], nseg[3];
 };
 
 // One surviving alignment; trace bytes (uint8 pairs: diffs, b-delta per
@@ -73,8 +79,9 @@ struct CallMemo {
 };
 
 struct AlignLaunch {
-  const PairTask *tasks;
-  int ntasks;
+  const PairTask *tasks;   // nitems of them
+  const unsigned *tfirst;  // the number of each one's first task, then ntasks
+  int nitems, ntasks;
   unsigned *next_task;
   unsigned *smflag;   // k_align_pairs: SM_FLAGS flags, zero at launch (null: off)
   // SM cycles the launch's warps spent in Local_Alignment [0] and in the
@@ -118,7 +125,6 @@ struct AlignLaunch {
   int64_t ltrace_cap;
   const FinishTask *ftasks;          // k_finish_pairs
   int nftasks;
-  const int *range_idx;
   uint8_t *cand_bytes;
   unsigned long long *cand_next;
   int64_t cand_cap;

@@ -128,7 +128,7 @@ struct pga_ctx {
   DBuf pk, poff, pwords;
   DBuf numf, numr, soff, tasks, task_next, pout, wave, points, cells, cell_next, ovl, perm, cand,
       cand_next, recs, rec_next, outb, out_next, pflag, pidx, pstart, pab, rng_ovl, rng_next, ftasks, fout,
-      ridx, rout, selfb, pstart2, pab2, small, shist, fo_dev, binfo[2], plive[2];
+      rout, selfb, pstart2, pab2, small, shist, fo_dev, binfo[2], plive[2];
   // survivors in la_sort order on the device (srecs, their traces in strace,
   // toff rewritten to offsets there), and their host copy, made when read
   DBuf srecs, slen, strace, skeys, skeys2, lhist, lscan;
@@ -245,7 +245,7 @@ bool shed_align_buffers(pga_ctx *ctx) {
   DBuf *bufs[] = {&ctx->numf, &ctx->numr, &ctx->pk, &ctx->wave, &ctx->points, &ctx->cells, &ctx->ovl, &ctx->perm,
                   &ctx->cand, &ctx->recs, &ctx->outb, &ctx->rng_ovl, &ctx->tasks, &ctx->pout, &ctx->pflag,
                   &ctx->pidx, &ctx->pstart, &ctx->pab, &ctx->pstart2, &ctx->pab2, &ctx->small, &ctx->ftasks,
-                  &ctx->fout, &ctx->ridx, &ctx->rout, &ctx->lreq, &ctx->lpath, &ctx->ltoff, &ctx->ltrace,
+                  &ctx->fout, &ctx->rout, &ctx->lreq, &ctx->lpath, &ctx->ltoff, &ctx->ltrace,
                   &ctx->binfo[0], &ctx->binfo[1], &ctx->plive[0], &ctx->plive[1], &ctx->skeys, &ctx->skeys2,
                   &ctx->lhist, &ctx->lscan, &ctx->memo_hits, &ctx->mlog_key, &ctx->mlog_val, &ctx->mlog_toff,
                   &ctx->mlog_trace, &ctx->mlog_ctr};
@@ -747,44 +747,52 @@ void fo_ranges(int n, const std::vector<int64_t> &clen_pos, int64_t npost, const
   }
 }
 
-// What one launch runs: tasks (whole pairs or band ranges, any order) and
-// then the pairs to finish from their ranges (k_finish_pairs), each listing
-// its range numbers, in order, at ridx[first .. first + nseg).
+// What one launch runs: pairs or parts of pairs (their tasks in this order),
+// then the pairs to finish from their ranges (k_finish_pairs).
 struct LaunchPlan {
   std::vector<PairTask> tasks;
   std::vector<FinishTask> fins;
-  std::vector<int> ridx;
 };
 
-// Runs a plan: the warps take the tasks in plan order.  tout: one
-// PairOut per task (plan order), fout: one per finished pair; rout_h (one
-// per range number) is refreshed.  Pebbles live for one launch; candidate
+// Runs a plan: the warps take the tasks in plan order.  tout: one PairOut per
+// whole pair (at its place in the plan), fout: one per finish task; *cycles
+// grows by the launch's task cycles.  Pebbles live for one launch; candidate
 // traces, range candidates and survivors accumulate over the launches of one
 // pga_align.  A pool that overflows is grown (keeping what earlier launches
 // left in it) and the launch runs again from the same counters.
 int align_launch(pga_ctx *ctx, AlignLaunch &L, const LaunchPlan &plan, std::vector<PairOut> &tout,
-                 std::vector<PairOut> &fout, std::vector<PairOut> &rout_h, long long *max_cycles,
-                 int64_t *max_task_calls) {
-  const size_t nt = plan.tasks.size(), nf = plan.fins.size();
-  tout.assign(nt, PairOut{});
+                 std::vector<PairOut> &fout, long long *cycles, long long *max_cycles, int64_t *max_task_calls) {
+  const size_t ni = plan.tasks.size(), nf = plan.fins.size();
+  tout.assign(ni, PairOut{});
   fout.assign(nf, PairOut{});
-  if (nt == 0 && nf == 0 && L.nsmall == 0) return PGA_OK;
-  const std::vector<PairTask> &sorted = plan.tasks;  // the warps take them in this order
-  if (nt) {
-    ENSURE(ctx->tasks, sizeof(PairTask) * nt);
-    ENSURE(ctx->pout, sizeof(PairOut) * nt);
-    CK(cudaMemcpyAsync(ctx->tasks.p, sorted.data(), sizeof(PairTask) * nt, cudaMemcpyHostToDevice, ctx->st));
+  std::vector<unsigned> tfirst(ni + 1);
+  int64_t nt = 0;
+  bool whole = false;
+  for (size_t i = 0; i < ni; i++) {
+    tfirst[i] = (unsigned)nt;
+    nt += plan.tasks[i].tasks();
+    whole |= plan.tasks[i].seg < 0;
   }
+  tfirst[ni] = (unsigned)nt;
+  if (nt + L.nsmall >= (int64_t)0x7fffffff)
+    return fail(ctx, PGA_ERR_LIMIT, "%lld alignment tasks: at most 2^31 supported", (long long)(nt + L.nsmall));
+  if (nt == 0 && nf == 0 && L.nsmall == 0) return PGA_OK;
+  if (nt) {
+    ENSURE(ctx->tasks, sizeof(PairTask) * ni + sizeof(unsigned) * (ni + 1));
+    ENSURE(ctx->pout, sizeof(PairOut) * ni);
+    unsigned *dfirst = (unsigned *)(P<PairTask>(ctx->tasks) + ni);
+    CK(cudaMemcpyAsync(ctx->tasks.p, plan.tasks.data(), sizeof(PairTask) * ni, cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaMemcpyAsync(dfirst, tfirst.data(), sizeof(unsigned) * (ni + 1), cudaMemcpyHostToDevice, ctx->st));
+    L.tasks = P<PairTask>(ctx->tasks);
+    L.tfirst = dfirst;
+  }
+  L.nitems = (int)ni;
+  L.ntasks = (int)nt;
   if (nf) {
     ENSURE(ctx->ftasks, sizeof(FinishTask) * nf);
     ENSURE(ctx->fout, sizeof(PairOut) * nf);
-    ENSURE(ctx->ridx, sizeof(int) * (plan.ridx.size() + 1));
     CK(cudaMemcpyAsync(ctx->ftasks.p, plan.fins.data(), sizeof(FinishTask) * nf, cudaMemcpyHostToDevice, ctx->st));
-    if (!plan.ridx.empty())
-      CK(cudaMemcpyAsync(ctx->ridx.p, plan.ridx.data(), sizeof(int) * plan.ridx.size(), cudaMemcpyHostToDevice,
-                         ctx->st));
   }
-  std::vector<PairOut> ro(nt);
   const int grid = (int)((L.nwarps * 32 + ALIGN_THREADS - 1) / ALIGN_THREADS);
   const unsigned long long base[4] = {ctx->cand_used, ctx->rng_used, ctx->rec_used, ctx->out_used};
   for (int attempt = 0;; attempt++) {
@@ -806,36 +814,31 @@ int align_launch(pga_ctx *ctx, AlignLaunch &L, const LaunchPlan &plan, std::vect
     CK(cudaMemcpyAsync(ctx->rec_next.p, &ctx->counters[2], 8, cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(ctx->out_next.p, &ctx->counters[3], 8, cudaMemcpyHostToDevice, ctx->st));
     L.rout = P<PairOut>(ctx->rout);
-    if (L.nsmall > 0) {
-      // the device-planned pairs' reductions: sred[6] (first failing task) starts at ~0
-      CK(cudaMemsetAsync(L.sred, 0, sizeof(unsigned long long) * (8 + 2 * (size_t)ctx->ncontig), ctx->st));
-      CK(cudaMemsetAsync(L.sred + 6, 0xff, sizeof(unsigned long long), ctx->st));
-    }
+    // the tasks' reductions ([6], the first failing task, starts at ~0) and the
+    // device-planned pairs' order keys
+    CK(cudaMemsetAsync(L.sred, 0, sizeof(unsigned long long) * (8 + (L.nsmall > 0 ? 2 * (size_t)ctx->ncontig : 0)),
+                       ctx->st));
+    CK(cudaMemsetAsync(L.sred + 6, 0xff, sizeof(unsigned long long), ctx->st));
+    unsigned long long sred[8] = {0, 0, 0, 0, 0, 0, ~0ull, 0};
     if (nt || L.nsmall > 0) {
-      L.tasks = P<PairTask>(ctx->tasks);
-      L.ntasks = (int)nt;
       L.pout = P<PairOut>(ctx->pout);
       launch_align(L, grid, ctx->st);
       LAUNCHED(1);
       CK(cudaGetLastError());
-      if (nt) CK(cudaMemcpyAsync(ro.data(), ctx->pout.p, sizeof(PairOut) * nt, cudaMemcpyDeviceToHost, ctx->st));
+      if (whole)
+        CK(cudaMemcpyAsync(tout.data(), ctx->pout.p, sizeof(PairOut) * ni, cudaMemcpyDeviceToHost, ctx->st));
+      CK(cudaMemcpyAsync(sred, L.sred, sizeof(sred), cudaMemcpyDeviceToHost, ctx->st));
     }
-    unsigned long long sred[8] = {0, 0, 0, 0, 0, 0, ~0ull, 0};
-    if (L.nsmall > 0) CK(cudaMemcpyAsync(sred, L.sred, sizeof(sred), cudaMemcpyDeviceToHost, ctx->st));
     if (nf) {
       AlignLaunch F = L;
       F.ftasks = P<FinishTask>(ctx->ftasks);
       F.nftasks = (int)nf;
-      F.range_idx = P<int>(ctx->ridx);
       F.pout = P<PairOut>(ctx->fout);
       launch_finish(F, grid, ctx->st);
       LAUNCHED(1);
       CK(cudaGetLastError());
       CK(cudaMemcpyAsync(fout.data(), ctx->fout.p, sizeof(PairOut) * nf, cudaMemcpyDeviceToHost, ctx->st));
     }
-    if (!rout_h.empty())
-      CK(cudaMemcpyAsync(rout_h.data(), ctx->rout.p, sizeof(PairOut) * rout_h.size(), cudaMemcpyDeviceToHost,
-                         ctx->st));
     unsigned long long used[4] = {0, 0, 0, 0}, prof[2] = {0, 0};
     CK(cudaMemcpyAsync(prof, L.prof, 16, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(&used[0], ctx->cand_next.p, 8, cudaMemcpyDeviceToHost, ctx->st));
@@ -843,12 +846,7 @@ int align_launch(pga_ctx *ctx, AlignLaunch &L, const LaunchPlan &plan, std::vect
     CK(cudaMemcpyAsync(&used[2], ctx->rec_next.p, 8, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(&used[3], ctx->out_next.p, 8, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
-    int errs = (int)sred[3], bad = -1, badf = -1;
-    for (size_t k = 0; k < nt; k++)
-      if (ro[k].err) {
-        errs |= ro[k].err;
-        if (bad < 0) bad = (int)k;
-      }
+    int errs = (int)sred[3], badf = -1;
     for (size_t f = 0; f < nf; f++)
       if (fout[f].err) {
         errs |= fout[f].err;
@@ -861,6 +859,14 @@ int align_launch(pga_ctx *ctx, AlignLaunch &L, const LaunchPlan &plan, std::vect
       ctx->rng_used = used[1];
       ctx->rec_used = used[2];
       ctx->out_used = used[3];
+      ctx->align_work[0] += (int64_t)sred[4];
+      ctx->align_work[1] += (int64_t)sred[5];
+      ctx->align_work[3] += nt + L.nsmall;
+      *cycles += (long long)sred[1];
+      if ((long long)(sred[2] >> 16) > *max_cycles) {
+        *max_cycles = (long long)(sred[2] >> 16);
+        *max_task_calls = (int64_t)(sred[2] & 0xffff);
+      }
       break;
     }
     // grow what overflowed and run the launch again
@@ -908,50 +914,19 @@ int align_launch(pga_ctx *ctx, AlignLaunch &L, const LaunchPlan &plan, std::vect
       if (r) return r;
     }
     if (!grown) {
+      if (sred[3] && sred[6] < (unsigned long long)nt) {
+        const PairTask &t =
+            plan.tasks[std::upper_bound(tfirst.begin(), tfirst.end(), (unsigned)sred[6]) - tfirst.begin() - 1];
+        return fail(ctx, PGA_ERR_LIMIT, "alignment of pair (%d,%d,%s) overflowed its work space (err 0x%llx)", t.a,
+                    t.b, t.comp ? "C" : "N", sred[3]);
+      }
       if (sred[3])
         return fail(ctx, PGA_ERR_LIMIT, "alignment of a contig pair overflowed its work space (err 0x%llx)", sred[3]);
-      if (bad >= 0)
-        return fail(ctx, PGA_ERR_LIMIT, "alignment of pair (%d,%d,%s) overflowed its work space (err 0x%x)",
-                    sorted[bad].a, sorted[bad].b, sorted[bad].comp ? "C" : "N", ro[bad].err);
       return fail(ctx, PGA_ERR_LIMIT, "alignment of pair (%d,%d,%s) overflowed its work space (err 0x%x)",
                   plan.fins[badf].a, plan.fins[badf].b, plan.fins[badf].comp ? "C" : "N", fout[badf].err);
     }
   }
-  for (size_t k = 0; k < nt; k++) {
-    tout[k] = ro[k];
-    ctx->align_work[0] += ro[k].waves;
-    ctx->align_work[1] += ro[k].cells;
-    ctx->align_work[3] += 1;
-    if (ro[k].cycles > *max_cycles) {
-      *max_cycles = ro[k].cycles;
-      *max_task_calls = ro[k].calls;
-    }
-  }
-  if (L.nsmall > 0) {
-    unsigned long long sred[8];
-    CK(cudaMemcpyAsync(sred, L.sred, sizeof(sred), cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    ctx->align_work[0] += (int64_t)sred[4];
-    ctx->align_work[1] += (int64_t)sred[5];
-    ctx->align_work[3] += L.nsmall;
-    if ((long long)(sred[2] >> 16) > *max_cycles) {
-      *max_cycles = (long long)(sred[2] >> 16);
-      *max_task_calls = (int64_t)(sred[2] & 0xffff);
-    }
-  }
   return PGA_OK;
-}
-
-// Calls and exit bepos of a pair run as ranges: the sum, and the last range
-// (in order) that called, else `entry`.
-void combine_ranges(const std::vector<PairOut> &rout_h, const std::vector<int> &ids, int *calls, int *exit_bepos,
-                    int entry) {
-  *calls = 0;
-  *exit_bepos = entry;
-  for (int id : ids) {
-    *calls += rout_h[id].calls;
-    if (rout_h[id].calls > 0) *exit_bepos = rout_h[id].exit_bepos;
-  }
 }
 
 // NUMERIC (with sentinels) and 2-bit packed copies of every contig, the base
@@ -1332,6 +1307,7 @@ int run_align(pga_ctx *ctx) {
       t.hi = h3[3 * q + 1];
       t.slo = t.lo;
       t.shi = t.hi;
+      t.step = 0;
       pairs[comp].push_back(t);
     }
   }
@@ -1427,25 +1403,29 @@ int run_align(pga_ctx *ctx) {
     CK(cudaStreamSynchronize(ctx->st));
   }
   int nranges = 0;
-  // ranges of about RS seeds covering seeds [x0, x1) of pair t (x1 a band start)
-  auto add_ranges = [&](const PairTask &t, int64_t x0, int64_t x1, std::vector<int> &ids,
-                        std::vector<PairTask> &dst) {
-    const int64_t step = RS > 0 ? RS : x1 - x0;
-    for (int64_t x = x0; x < x1; x += step) {
-      PairTask r = t;
-      r.entry_bepos = 0;
-      r.seg = nranges++;
-      r.slo = x;
-      r.shi = std::min(x1, x + step);
-      ids.push_back(r.seg);
-      dst.push_back(r);
-    }
-  };
   LaunchPlan P1;
+  // ranges of about RS seeds covering seeds [x0, x1) of pair t (x1 a band
+  // start): their first number and count
+  struct Ranges {
+    int first = 0, n = 0;
+  };
+  auto add_ranges = [&](const PairTask &t, int64_t x0, int64_t x1) {
+    Ranges g;
+    if (x1 <= x0) return g;
+    PairTask r = t;
+    r.entry_bepos = 0;
+    r.seg = g.first = nranges;
+    r.slo = x0;
+    r.shi = x1;
+    r.step = RS;
+    nranges += g.n = (int)r.tasks();
+    P1.tasks.push_back(r);
+    return g;
+  };
   std::vector<int> first_task(first.size(), -1), first_fin(first.size(), -1);
-  std::vector<std::vector<int>> first_ids(first.size());
   struct SelfPlan {
-    std::vector<int> pre, post;
+    Ranges pre, post;
+    int fin = -1;   // finish tasks combining pre, then post
     int diag = -1;  // range number of the middle part (RS > 0)
     bool whole = false;
   };
@@ -1464,22 +1444,14 @@ int run_align(pga_ctx *ctx) {
   std::stable_sort(src.begin(), src.end(), [](const std::pair<int64_t, int> &x, const std::pair<int64_t, int> &y) {
     return x.first > y.first;
   });
-  {
-    size_t est = 2 * (size_t)nself + 1;
-    for (const auto &s : src) est += RS > 0 ? (size_t)(s.first / RS + 2) : 1;
-    P1.tasks.reserve(est);
-    P1.ridx.reserve(est);
-  }
   for (const auto &s : src) {
     if (s.second >= 0) {
       const size_t i = (size_t)s.second;
       PairTask t = first[i];
       if (RS > 0 && t.hi - t.lo > RS) {
-        add_ranges(t, t.lo, t.hi, first_ids[i], P1.tasks);
-        FinishTask f{t.comp, t.a, t.b, 0, (int)P1.ridx.size(), (int)first_ids[i].size()};
-        P1.ridx.insert(P1.ridx.end(), first_ids[i].begin(), first_ids[i].end());
+        const Ranges g = add_ranges(t, t.lo, t.hi);
         first_fin[i] = (int)P1.fins.size();
-        P1.fins.push_back(f);
+        P1.fins.push_back(FinishTask{t.comp, t.a, t.b, 0, 1, {g.first, 0, 0}, {g.n, 0, 0}});
       } else {
         first_task[i] = (int)P1.tasks.size();
         P1.tasks.push_back(t);
@@ -1488,8 +1460,11 @@ int run_align(pga_ctx *ctx) {
       const int q = -1 - s.second;
       const PairTask &t = pairs[0][self_idx[q]];
       const int64_t x1 = t.lo + x12[2 * q], x2 = t.lo + x12[2 * q + 1];
-      add_ranges(t, t.lo, x1, sp[q].pre, P1.tasks);
-      add_ranges(t, x2, t.hi, sp[q].post, P1.tasks);
+      sp[q].pre = add_ranges(t, t.lo, x1);
+      sp[q].post = add_ranges(t, x2, t.hi);
+      sp[q].fin = (int)P1.fins.size();
+      P1.fins.push_back(FinishTask{0, t.a, t.b, 0, 0, {sp[q].pre.first, 0, 0}, {sp[q].pre.n, 0, 0}});
+      P1.fins.push_back(FinishTask{0, t.a, t.b, 0, 0, {sp[q].post.first, 0, 0}, {sp[q].post.n, 0, 0}});
     }
   }
   for (int q = 0; q < nself; q++) {
@@ -1505,17 +1480,18 @@ int run_align(pga_ctx *ctx) {
       d.seg = sp[q].diag = nranges++;
       d.slo = x1;
       d.shi = x2;
+      d.step = x2 - x1;
       diag_task[q] = d;
     }
   }
   ENSURE(ctx->rout, sizeof(PairOut) * (size_t)(nranges + 1));
-  std::vector<PairOut> rout_h(nranges);
+  L.rout = P<PairOut>(ctx->rout);
 
   const double t_launch = now_ms();
   long long maxcyc = 0, sumcyc = 0;
   int64_t maxcalls = 0, calls = 0;
   std::vector<PairOut> tout, fout;
-  int r = align_launch(ctx, L, P1, tout, fout, rout_h, &maxcyc, &maxcalls);
+  int r = align_launch(ctx, L, P1, tout, fout, &sumcyc, &maxcyc, &maxcalls);
   if (r) return r;
   // the device-planned pairs: totals and, per order position, FastGA's
   // order keys of the N pairs among them
@@ -1527,7 +1503,6 @@ int run_align(pga_ctx *ctx) {
     CK(cudaMemcpyAsync(fo.data(), L.fo_last, sizeof(unsigned long long) * 2 * nc, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     calls += (int64_t)red[0];
-    sumcyc += (long long)red[1];
     for (int x = 0; x < nc; x++) {
       Lk[x] = (int64_t)fo[x];
       ebest[x] = (int64_t)fo[nc + x];
@@ -1536,17 +1511,17 @@ int run_align(pga_ctx *ctx) {
   L.nsmall = 0;  // the later launches run host-planned tasks only
   std::vector<PairOut> out1(first.size());
   for (size_t i = 0; i < first.size(); i++) {
-    if (first_task[i] >= 0) {
-      out1[i] = tout[first_task[i]];
-    } else {
-      out1[i] = fout[first_fin[i]];
-      long long c = 0;
-      for (int id : first_ids[i]) c += rout_h[id].cycles;
-      out1[i].cycles = c + fout[first_fin[i]].cycles;
-    }
+    out1[i] = first_task[i] >= 0 ? tout[first_task[i]] : fout[first_fin[i]];
+    if (first_task[i] < 0) sumcyc += out1[i].cycles;
     calls += out1[i].calls;
-    sumcyc += out1[i].cycles;
   }
+  // the self pairs' outer parts: calls and last bepos
+  std::vector<PairOut> pre(nself, PairOut{}), post(nself, PairOut{});
+  for (int q = 0; q < nself; q++)
+    if (sp[q].fin >= 0) {
+      pre[q] = fout[sp[q].fin];
+      post[q] = fout[sp[q].fin + 1];
+    }
 
   const double t_self = now_ms();
   // 6. self pairs: entry values by FastGA's order (src/fastga_order.c)
@@ -1588,41 +1563,30 @@ int run_align(pga_ctx *ctx) {
     std::vector<int64_t> S(nc, 0);  // 0 none, 1 pending, 2 no call, 3+bepos called
     std::vector<int> val(nself, 0), state(nself, 0);  // 0 undetermined, 1 known
     std::vector<char> done(nself, 0);
-    // the ranges of self pair q in order, with its middle part's
-    auto self_ids = [&](int q) {
-      std::vector<int> ids = sp[q].pre;
-      if (sp[q].diag >= 0) ids.push_back(sp[q].diag);
-      ids.insert(ids.end(), sp[q].post.begin(), sp[q].post.end());
-      return ids;
+    // self pair q from its ranges, its middle part's among them
+    auto self_fin = [&](int q, int entry) {
+      const PairTask &t = pairs[0][self_idx[q]];
+      return FinishTask{0, t.a, t.b, entry, 1, {sp[q].pre.first, sp[q].diag, sp[q].post.first},
+                        {sp[q].pre.n, sp[q].diag >= 0 ? 1 : 0, sp[q].post.n}};
     };
     LaunchPlan pending;  // self pairs to finish in the next launch
-    std::vector<int> pending_q;
     for (int q = 0; q < nself; q++) {
       const PairTask &t = pairs[0][self_idx[q]];
       int x = F.pos[t.a];
       S[x] = 1;
-      if (!sp[q].whole) {
-        int pc, pe;
-        combine_ranges(rout_h, sp[q].pre, &pc, &pe, 0);
-        if (pc > 0 || sp[q].diag < 0) {
-          // entered after a call of its own, or with no middle part: its
-          // result does not depend on the order's value
-          val[q] = pe;
-          state[q] = 1;
-          if (sp[q].diag < 0) {
-            std::vector<int> ids = self_ids(q);
-            int c, e;
-            combine_ranges(rout_h, ids, &c, &e, 0);
-            S[x] = c > 0 ? 3 + (int64_t)e : 2;
-            calls += c;
-            for (int id : ids) sumcyc += rout_h[id].cycles;
-            done[q] = 1;
-            FinishTask f{0, t.a, t.b, 0, (int)pending.ridx.size(), (int)ids.size()};
-            pending.ridx.insert(pending.ridx.end(), ids.begin(), ids.end());
-            pending.fins.push_back(f);
-          }
-          continue;
+      if (!sp[q].whole && (pre[q].calls > 0 || sp[q].diag < 0)) {
+        // entered after a call of its own, or with no middle part: its
+        // result does not depend on the order's value
+        val[q] = pre[q].exit_bepos;
+        state[q] = 1;
+        if (sp[q].diag < 0) {
+          const int c = pre[q].calls + post[q].calls;
+          S[x] = c > 0 ? 3 + (int64_t)(post[q].calls > 0 ? post[q].exit_bepos : pre[q].exit_bepos) : 2;
+          calls += c;
+          done[q] = 1;
+          pending.fins.push_back(self_fin(q, 0));
         }
+        continue;
       }
       // nearest earlier partner that made a call (src/fastga_order_core.c:147-166)
       const bool found = ebest[x] != 0;
@@ -1636,7 +1600,7 @@ int run_align(pga_ctx *ctx) {
     while (true) {
       LaunchPlan plan = pending;
       pending = LaunchPlan();
-      std::vector<int> bq;
+      std::vector<int> bq, fin_of;
       for (int q = 0; q < nself; q++) {
         if (done[q]) continue;
         if (!state[q]) {
@@ -1671,32 +1635,21 @@ int run_align(pga_ctx *ctx) {
         plan.tasks.push_back(d);
         bq.push_back(q);
         if (!sp[q].whole) {
-          std::vector<int> ids = self_ids(q);
-          FinishTask f{0, d.a, d.b, 0, (int)plan.ridx.size(), (int)ids.size()};
-          plan.ridx.insert(plan.ridx.end(), ids.begin(), ids.end());
-          plan.fins.push_back(f);
-        }
+          fin_of.push_back((int)plan.fins.size());
+          plan.fins.push_back(self_fin(q, val[q]));
+        } else
+          fin_of.push_back(-1);
       }
       if (plan.tasks.empty() && plan.fins.empty()) break;
       if (!plan.tasks.empty()) nrounds++;
-      r = align_launch(ctx, L, plan, tout, fout, rout_h, &maxcyc, &maxcalls);
+      r = align_launch(ctx, L, plan, tout, fout, &sumcyc, &maxcyc, &maxcalls);
       if (r) return r;
       for (size_t i = 0; i < bq.size(); i++) {
         const int q = bq[i];
         done[q] = 1;
-        int x = F.pos[pairs[0][self_idx[q]].a];
-        int c, e;
-        if (sp[q].whole) {
-          c = tout[i].calls;
-          e = tout[i].exit_bepos;
-          sumcyc += tout[i].cycles;
-        } else {
-          std::vector<int> ids = self_ids(q);
-          combine_ranges(rout_h, ids, &c, &e, val[q]);
-          for (int id : ids) sumcyc += rout_h[id].cycles;
-        }
-        S[x] = c > 0 ? 3 + (int64_t)e : 2;
-        calls += c;
+        const PairOut &o = fin_of[i] < 0 ? tout[i] : fout[fin_of[i]];
+        S[F.pos[pairs[0][self_idx[q]].a]] = o.calls > 0 ? 3 + (int64_t)o.exit_bepos : 2;
+        calls += o.calls;
       }
     }
     for (int q = 0; q < nself; q++)
@@ -1774,7 +1727,7 @@ void pga_ctx_destroy(pga_ctx *ctx) {
                    &ctx->wave, &ctx->points, &ctx->cells, &ctx->cell_next, &ctx->ovl, &ctx->perm, &ctx->cand,
                    &ctx->cand_next, &ctx->recs, &ctx->rec_next, &ctx->outb, &ctx->out_next, &ctx->pflag,
                    &ctx->pidx, &ctx->pstart, &ctx->pab, &ctx->rng_ovl, &ctx->rng_next, &ctx->ftasks,
-                   &ctx->fout, &ctx->ridx, &ctx->rout, &ctx->selfb, &ctx->lreq, &ctx->lpath, &ctx->ltoff,
+                   &ctx->fout, &ctx->rout, &ctx->selfb, &ctx->lreq, &ctx->lpath, &ctx->ltoff,
                    &ctx->ltrace, &ctx->lnext, &ctx->pstart2, &ctx->pab2, &ctx->small, &ctx->shist, &ctx->fo_dev,
                    &ctx->srecs, &ctx->slen, &ctx->strace, &ctx->skeys, &ctx->skeys2, &ctx->lhist, &ctx->lscan,
                    &ctx->memo_hits, &ctx->mlog_key, &ctx->mlog_val, &ctx->mlog_toff, &ctx->mlog_trace,
