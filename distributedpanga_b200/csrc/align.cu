@@ -68,15 +68,134 @@ struct KeySeeds {
   __device__ int64_t band(int64_t i) const { return (int64_t)key_bits(k[i], L.off_band, L.off_j - L.off_band); }
   __device__ int lcp(int64_t i) const { return (int)key_bits(k[i], 0, 6); }
   __device__ int dlow(int64_t i) const { return (int)key_bits(k[i], L.off_dlow, 6); }
-  __device__ int64_t band_end(int64_t i, int64_t b) const {
+  // First index >= x in [x, hi) whose band differs from its predecessor's
+  // (x itself when x == 0), else hi; warp-wide.  Bands never decrease within
+  // a pair, so this is the first index whose band exceeds band(x-1): a search
+  // that probes 32 points per step (ballot) and ends with one linear step of
+  // 32, so neither a range that starts inside a long band nor a block that
+  // holds one walks its seeds.
+  __device__ int64_t next_band_start(int64_t x, int64_t hi) const {
+    if (x <= 0) return 0;
+    if (x >= hi) return hi;
     const int lane = threadIdx.x & 31;
-    for (int64_t base = i; base < n; base += 32) {
-      int64_t j = base + lane;
-      bool stop = j < n && band(j) != b;
-      unsigned msk = __ballot_sync(FULL, stop);
-      if (msk) return base + __ffs(msk) - 1;
+    const int64_t b = band(x - 1);
+    int64_t lo = x, h = hi;  // the answer lies in [lo, h], h meaning none below h
+    while (h - lo > 32) {
+      const int64_t span = h - lo;
+      const int64_t p = lo + (span * (lane + 1)) / 33;  // increasing in lane, inside [lo, h)
+      const unsigned m = __ballot_sync(FULL, band(p) > b);
+      if (m) {
+        const int f = __ffs(m) - 1;
+        const int64_t pf = lo + (span * (f + 1)) / 33;
+        const int64_t before = f > 0 ? lo + (span * f) / 33 : lo - 1;  // last probe known not past b
+        lo = before + 1;
+        h = pf;  // band(pf) > b: the answer is at most pf
+        if (h - lo <= 32) {
+          const int64_t q = lo + lane;
+          const unsigned m2 = __ballot_sync(FULL, q < h && band(q) > b);
+          return m2 ? lo + __ffs(m2) - 1 : h;
+        }
+      } else {
+        lo = lo + (span * 32) / 33 + 1;
+      }
     }
-    return n;
+    const int64_t q = lo + lane;
+    const unsigned m = __ballot_sync(FULL, q < h && band(q) > b);
+    return m ? lo + __ffs(m) - 1 : h;
+  }
+  // The first index >= i past band b, which i is in.
+  __device__ int64_t band_end(int64_t i, int64_t b) const {
+    const int64_t j = i + (threadIdx.x & 31);
+    const unsigned msk = __ballot_sync(FULL, j < n && band(j) != b);
+    return msk ? i + __ffs(msk) - 1 : next_band_start(i + 32, n);
+  }
+
+  // Takes up to 32 * FOLLOW seeds of one stream into the open chain (highest
+  // end P) if each starts less than CHAIN_BREAK past the one before, and those
+  // of the other stream up to the last of them; false if neither stream's next
+  // ones do.  The long diagonal of two contigs is one chain of up to millions
+  // of seeds, scanned by one warp: 32 at a time through the merge below took
+  // longer than aligning it.
+  static constexpr int FOLLOW = 8;
+  __device__ __forceinline__ uint32_t anti32(U128 key) const {  // below 2^32: contigs are below 2^31
+    return (uint32_t)key_bits(key, L.off_anti, L.off_band - L.off_anti);
+  }
+  __device__ bool follow(int64_t &s, int64_t m, int64_t &t, int64_t e, int64_t &P, int &mix, int &dgmin,
+                         int &dgmax) const {
+    const int lane = threadIdx.x & 31;
+    for (int lead = 1; lead <= 2; lead++) {  // the stream followed
+      int64_t &x = lead == 1 ? s : t;
+      const int64_t end = lead == 1 ? m : e;
+      if (end - x < 32) continue;
+      const int n = (int)min(end - x, (int64_t)(32 * FOLLOW));
+      uint32_t a[FOLLOW];
+      int l2[FOLLOW], dg[FOLLOW];
+#pragma unroll
+      for (int j = 0; j < FOLLOW; j++) {
+        a[j] = 0;
+        l2[j] = dg[j] = 0;
+        if (32 * j + lane < n) {
+          const U128 key = k[x + 32 * j + lane];
+          a[j] = anti32(key);
+          l2[j] = (int)key_bits(key, 0, 6) << 1;
+          dg[j] = (int)key_bits(key, L.off_dlow, 6);
+        }
+      }
+      const uint32_t a0 = __shfl_sync(FULL, a[0], 0);
+      bool ok = (int64_t)a0 < P + CHAIN_BREAK;
+      int lo = 2 * BUCK_WIDTH, hi = -1;
+      uint32_t far = 0;  // furthest end, from a0
+#pragma unroll
+      for (int j = 0; j < FOLLOW; j++) {
+        const uint32_t up = __shfl_up_sync(FULL, a[j], 1);
+        const uint32_t before = j > 0 ? __shfl_sync(FULL, a[j - 1], 31) : a0;
+        if (32 * j + lane < n) {
+          ok = ok && a[j] - (lane > 0 ? up : before) < (uint32_t)CHAIN_BREAK;
+          lo = min(lo, dg[j]);
+          hi = max(hi, dg[j]);
+          far = max(far, a[j] - a0 + (uint32_t)l2[j]);
+        }
+      }
+      if (!__all_sync(FULL, ok)) continue;
+      uint32_t last = 0;
+#pragma unroll
+      for (int j = 0; j < FOLLOW; j++)
+        if (32 * j < n) last = __shfl_sync(FULL, a[j], min(n - 32 * j, 32) - 1);
+      const int add = lead == 1 ? 0 : BUCK_WIDTH;
+      dgmin = min(dgmin, __reduce_min_sync(FULL, lo) + add);
+      dgmax = max(dgmax, __reduce_max_sync(FULL, hi) + add);
+      P = max(P, (int64_t)a0 + __reduce_max_sync(FULL, far));
+      mix |= lead;
+      x += n;
+      // the other stream's seeds up to the last
+      int64_t &y = lead == 1 ? t : s;
+      const int64_t yend = lead == 1 ? e : m;
+      const int yadd = lead == 1 ? BUCK_WIDTH : 0;
+      while (y < yend) {
+        uint32_t b = 0xffffffffu;
+        int bl = 0, bd = 0;
+        const bool in = y + lane < yend;
+        if (in) {
+          const U128 key = k[y + lane];
+          b = anti32(key);
+          bl = (int)key_bits(key, 0, 6) << 1;
+          bd = (int)key_bits(key, L.off_dlow, 6) + yadd;
+        }
+        const unsigned take = __ballot_sync(FULL, in && b <= last);  // sorted: the first ones
+        const int c = __popc(take);
+        if (c > 0) {
+          const bool mine = lane < c;
+          dgmin = min(dgmin, __reduce_min_sync(FULL, mine ? bd : I32MAX));
+          dgmax = max(dgmax, __reduce_max_sync(FULL, mine ? bd : -1));
+          P = max(P, (int64_t)last + __reduce_max_sync(FULL, mine ? (int)(b - last) + bl : -I32MAX));
+          mix |= 3 - lead;
+          y += c;
+        }
+        if (c < 32) break;
+      }
+      return true;
+    }
+    return false;
   }
 
   // The chains of the block [b, m) + [m, e) exactly as scan_block_scalar
@@ -94,9 +213,18 @@ struct KeySeeds {
     int64_t P = -CHAIN_BREAK;  // highest chain end so far
     bool open = false;         // a chain is open (the first seed always opens one)
     int64_t cov = 0, alow = 0;
-    int mix = 0, dgmin = 0, dgmax = 0;
+    int mix = 0, dgmin = 0, dgmax = 0, rest = 0;
     int64_t s = b, t = m;
     while (s < m || t < e) {
+      // A chain past the hit test's coverage needs only its ends and the
+      // extremes of its diagonals: while one stream's seeds follow each other
+      // within CHAIN_BREAK they are all the chain's, and so is what the other
+      // stream has between them.
+      if (open && cov >= CHAIN_MIN && rest-- <= 0) {
+        rest = 0;
+        if (follow(s, m, t, e, P, mix, dgmin, dgmax)) continue;
+        rest = 8;  // steps before the next try
+      }
       int64_t i1 = s + lane, i2 = t + lane;
       int64_t a1 = MAX_I64, a2 = MAX_I64;
       int l1 = 0, l2 = 0, d1 = 0, d2 = 0;
@@ -187,12 +315,185 @@ struct KeySeeds {
   }
 };
 
-template <bool BLOCKS>
+// Slot of a call's inputs in the target's record of its own calls, -1 if it
+// is not there.
+__device__ int64_t record_slot(const CallMemo &M, const uint32_t *k) {
+  const uint64_t mask = (uint64_t)M.cap - 1;
+  for (uint64_t s = memo_hash(k) & mask, probe = 0; probe <= mask; probe++, s = (s + 1) & mask) {
+    const uint32_t *q = M.key + MEMO_KEY * s;
+    if (q[0] == MEMO_EMPTY) return -1;
+    bool same = true;
+    for (int i = 0; i < MEMO_KEY; i++) same &= q[i] == k[i];
+    if (same) return (int64_t)s;
+  }
+  return -1;
+}
+
+__device__ __forceinline__ void call_key(uint32_t *k, int a, int b, bool comp, int low, int hgh, int anti, int lbord,
+                                         int hbord) {
+  k[0] = (uint32_t)a | ((uint32_t)b << 15) | ((uint32_t)comp << 30);
+  k[1] = (uint32_t)low;
+  k[2] = (uint32_t)hgh;
+  k[3] = (uint32_t)anti;
+  k[4] = (uint32_t)lbord;
+  k[5] = (uint32_t)hbord;
+}
+
+namespace aln {
+// What a task's scout pass reads: its seeds, how chains become calls, and the
+// call the task is at.
+struct TaskChains {
+  KeySeeds S;
+  const uint16_t *info;
+  const CallMemo *M;
+  int a, b;
+  bool comp;
+  int64_t bmxpos, doffset, aoffset;
+  int64_t blo, bhi;
+  int low, hgh, anti;
+};
+}  // namespace aln
+
+// The sink of a scout pass: what ChainSink would call first for a chain,
+// queued, and the starts along it.
+struct ScoutSink {
+  const TaskChains &T;
+  const ShareTable &X;
+  int64_t cdiag;
+  int isnew;
+  int64_t alast;
+  __device__ int chain(int64_t cov, int mix, int dgmin, int dgmax, int64_t alow, int64_t ahgh) {
+    if (!(cov >= CHAIN_MIN && (mix != 1 || isnew))) return 0;
+    const int lane = threadIdx.x & 31;
+    dgmin += (int)(cdiag << BUCK_SHIFT);
+    dgmax += (int)(cdiag << BUCK_SHIFT);
+    if (T.comp) {
+      dgmin += (int)T.doffset;
+      dgmax += (int)T.doffset;
+      alow += T.aoffset;
+      ahgh += T.aoffset;
+    } else {
+      dgmin -= (int)T.bmxpos;
+      dgmax -= (int)T.bmxpos;
+    }
+    if (ahgh <= -1) return 0;
+    if (alow < -1) alow = -1;
+    ahgh -= BUCK_ANTI;
+    int64_t amid = alow + BUCK_ANTI;
+    if (amid > ahgh) {
+      amid = ahgh;
+      if (amid + dgmin < 0) {
+        dgmin = (int)-amid;
+        if (dgmin > dgmax) return 0;
+      }
+    }
+    uint32_t k[MEMO_KEY];
+    call_key(k, T.a, T.b, T.comp, dgmin, dgmax, (int)amid, -1, -1);
+    if (T.M->cap > 0 && T.a < T.M->nt && T.b < T.M->nt && record_slot(*T.M, k) >= 0) return 0;
+    // the call itself, then starts half a line or more past the chain's start
+    const bool call = !(dgmin == T.low && dgmax == T.hgh && (int)amid == T.anti);
+    const int64_t first = (alow + SHARE_LINE - 1) / SHARE_LINE;
+    const int n = (int)max((ahgh + SHARE_LINE / 2) / SHARE_LINE - first, (int64_t)0) + (call ? 1 : 0);
+    if (n == 0 || *(volatile unsigned *)X.qtail >= (unsigned)X.qcap) return 0;
+    unsigned base = 0;
+    if (lane == 0) base = atomicAdd(X.qtail, (unsigned)n);
+    base = __shfl_sync(FULL, base, 0);
+    for (int i = lane; i < n && base + i < (unsigned)X.qcap; i += 32) {
+      Scout &q = X.scouts[base + i];
+      const int j = i - (call ? 1 : 0);
+      q.a = T.a;
+      q.b = T.b;
+      q.comp = T.comp;
+      q.low = dgmin;
+      q.hgh = dgmax;
+      q.anti = j < 0 ? (int)amid : (int)((first + j) * SHARE_LINE + SHARE_LINE / 2);
+      q.call = j < 0;
+      __threadfence();
+      *(volatile int *)&q.state = SCOUT_READY;
+      if (j >= 0) continue;
+      const unsigned long long key = memo_hash(k) | 1;
+      unsigned at = (unsigned)(key >> 24) & X.cmask;
+      for (int probe = 0; probe < SHARE_PROBES; probe++, at = (at + 1) & X.cmask)
+        if (atomicCAS(&X.ckeys[at], 0ull, key) == 0) {
+          *(volatile int *)&X.cvals[at] = (int)(base + i);
+          break;
+        }
+    }
+    __syncwarp();
+    return 0;
+  }
+};
+
+template <class Sink>
+__device__ int scan_blocks(const KeySeeds &S, const uint16_t *info, int64_t blo, int64_t bhi, Sink &K);
+
+namespace aln {
+__device__ __noinline__ void scout_if_free(WarpWork &W) {
+  const TaskChains &T = *W.task;
+  if (*(volatile const unsigned *)W.share->next_task < W.share->ntasks) return;
+  W.task = nullptr;
+  ScoutSink K{T, *W.share, 0, 0, -1};
+  scan_blocks(T.S, T.info, T.blo, T.bhi, K);
+}
+}  // namespace aln
+
+template <bool BLOCKS, bool SHARE>
 struct WarpAligner {
   WarpWork &W;
   const AlignSpec &spec;
   const CallMemo &M;
   int a, b;  // the pair's contigs (A's and B's)
+  TaskChains *chains;  // the task's (null: it queues no scouts)
+
+  // A call another warp ran or runs ahead of this one: its result, if it
+  // comes.  One still queued is taken off the queue and left to the caller.
+  __device__ bool take_call(const uint32_t *k, bool acomp, Path &P) {
+    const ShareTable &X = *W.share;
+    const int lane = threadIdx.x & 31;
+    int got = -1;
+    if (lane == 0) {
+      const unsigned long long key = memo_hash(k) | 1;
+      unsigned at = (unsigned)(key >> 24) & X.cmask;
+      for (int probe = 0; probe < SHARE_PROBES; probe++, at = (at + 1) & X.cmask) {
+        const unsigned long long q = *(volatile unsigned long long *)&X.ckeys[at];
+        if (q == 0) break;
+        if (q != key) continue;
+        const int v = *(volatile int *)&X.cvals[at];
+        if (v < 0) break;
+        Scout &c = X.scouts[v];
+        __threadfence();
+        if (__ldcg(&c.a) != a || __ldcg(&c.b) != b || __ldcg(&c.comp) != (int)acomp ||
+            __ldcg(&c.low) != (int)k[1] || __ldcg(&c.hgh) != (int)k[2] || __ldcg(&c.anti) != (int)k[3])
+          continue;
+        int state = atomicCAS(&c.state, SCOUT_READY, SCOUT_VOID);
+        for (int poll = 0; poll < SHARE_POLLS && state == SCOUT_RUNS; poll++) {
+          __nanosleep(500);
+          state = *(volatile int *)&c.state;
+        }
+        if (state == SCOUT_DONE) got = v;
+        break;
+      }
+    }
+    got = __shfl_sync(FULL, got, 0);
+    if (got < 0) return false;
+    __threadfence();
+    const Scout &c = X.scouts[got];
+    const int tlen = __ldcg(&c.tlen);
+    if (tlen > W.point_cap) return false;
+    const int64_t off = __ldcg(&c.off);
+    uint32_t *pt = reinterpret_cast<uint32_t *>(W.points);
+    for (int i = lane; i < tlen / 2; i += 32) pt[i] = __ldcg(&X.list[off + i]);
+    __syncwarp();
+    P.abpos = __ldcg(&c.abpos);
+    P.aepos = __ldcg(&c.aepos);
+    P.bbpos = __ldcg(&c.bbpos);
+    P.bepos = __ldcg(&c.bepos);
+    P.diffs = __ldcg(&c.diffs);
+    P.tlen = tlen;
+    P.trace_off = 0;
+    return true;
+  }
+
   __device__ int call(const Seq &A, const Seq &B, bool acomp, Path &P, int low, int hgh, int anti, int lbord,
                       int hbord) {
     const long long t0 = clock64();
@@ -200,22 +501,12 @@ struct WarpAligner {
     // a call on two target contigs: its recorded result, if the target's run made it
     const bool keyed = (M.cap > 0 || M.lkey) && a < M.nt && b < M.nt;
     uint32_t k[MEMO_KEY];
-    k[0] = (uint32_t)a | ((uint32_t)b << 15) | ((uint32_t)acomp << 30);
-    k[1] = (uint32_t)low;
-    k[2] = (uint32_t)hgh;
-    k[3] = (uint32_t)anti;
-    k[4] = (uint32_t)lbord;
-    k[5] = (uint32_t)hbord;
+    call_key(k, a, b, acomp, low, hgh, anti, lbord, hbord);
     if (keyed && M.cap > 0) {
-      const uint64_t mask = (uint64_t)M.cap - 1;
-      for (uint64_t s = memo_hash(k) & mask, probe = 0; probe <= mask; probe++, s = (s + 1) & mask) {
-        const uint32_t *q = M.key + MEMO_KEY * s;
-        if (q[0] == MEMO_EMPTY) break;
-        bool same = true;
-        for (int i = 0; i < MEMO_KEY; i++) same &= q[i] == k[i];
-        if (!same) continue;
+      const int64_t s = record_slot(M, k);
+      // (a result that does not fit is computed below, which reports the overflow)
+      if (s >= 0 && M.val[MEMO_VAL * s + 5] <= W.point_cap) {
         const int32_t *v = M.val + MEMO_VAL * s;
-        if (v[5] > W.point_cap) break;  // computed below, which reports the overflow
         const uint8_t *tr = M.trace + M.toff[s];
         for (int i = lane; i < v[5]; i += 32) W.points[i] = tr[i];
         __syncwarp();
@@ -231,7 +522,19 @@ struct WarpAligner {
         return 0;
       }
     }
-    const int r = local_alignment_w<BLOCKS>(W, spec, A, B, acomp, P, low, hgh, anti, lbord, hbord);
+    W.pair = k[0];
+    int r = 0;
+    bool taken = false;
+    if (SHARE && chains) {
+      if (!W.task) taken = take_call(k, acomp, P);
+      else {
+        chains->low = low;
+        chains->hgh = hgh;
+        chains->anti = anti;
+        scout_if_free(W);
+      }
+    }
+    if (!taken) r = local_alignment_w<BLOCKS, SHARE>(W, spec, A, B, acomp, P, low, hgh, anti, lbord, hbord);
     if (keyed && M.lkey && r == 0) {
       // the target's own run: append the call to the log
       unsigned long long e = 0, tb = 0;
@@ -295,6 +598,9 @@ __device__ WarpWork warp_work(const AlignLaunch &P, int64_t wid) {
   W.smflag = P.smflag;
   W.long_waves = P.smflag ? P.long_waves : 0;
   W.flagged = 0;
+  W.share = P.share;
+  W.pair = 0;
+  W.task = nullptr;
   W.la_cycles = 0;
   return W;
 }
@@ -327,40 +633,6 @@ __device__ OvlArena warp_arena(const AlignLaunch &P, int64_t wid) {
   return O;
 }
 
-// First index >= x in [x, hi) whose band differs from its predecessor's
-// (x itself when x == 0), else hi; warp-wide.  Bands never decrease within
-// a pair, so this is the first index whose band exceeds band(x-1): a search
-// that probes 32 points per step (ballot) and ends with one linear step of
-// 32, so a range that starts inside a long band does not walk its seeds.
-__device__ int64_t next_band_start(const KeySeeds &S, int64_t x, int64_t hi, int lane) {
-  if (x <= 0) return 0;
-  if (x >= hi) return hi;
-  const int64_t b = S.band(x - 1);
-  int64_t lo = x, h = hi;  // the answer lies in [lo, h], h meaning none below h
-  while (h - lo > 32) {
-    const int64_t span = h - lo;
-    const int64_t p = lo + (span * (lane + 1)) / 33;  // increasing in lane, inside [lo, h)
-    const unsigned m = __ballot_sync(FULL, S.band(p) > b);
-    if (m) {
-      const int f = __ffs(m) - 1;
-      const int64_t pf = lo + (span * (f + 1)) / 33;
-      const int64_t before = f > 0 ? lo + (span * f) / 33 : lo - 1;  // last probe known not past b
-      lo = before + 1;
-      h = pf;  // band(pf) > b: the answer is at most pf
-      if (h - lo <= 32) {
-        const int64_t q = lo + lane;
-        const unsigned m2 = __ballot_sync(FULL, q < h && S.band(q) > b);
-        return m2 ? lo + __ffs(m2) - 1 : h;
-      }
-    } else {
-      lo = lo + (span * 32) / 33 + 1;
-    }
-  }
-  const int64_t q = lo + lane;
-  const unsigned m = __ballot_sync(FULL, q < h && S.band(q) > b);
-  return m ? lo + __ffs(m) - 1 : h;
-}
-
 // align_pair (align_core.cuh) for a pair's seeds on the device: the same
 // band blocks in the same order, with the same chains and calls, but the
 // blocks come from the per-seed band info, 32 seeds per step, and a block
@@ -370,29 +642,24 @@ __device__ int64_t next_band_start(const KeySeeds &S, int64_t x, int64_t hi, int
 // Block (c, c+1) starting at band c's first seed b is scanned when band c
 // is new (the band below it is not c-1) or band c+1 follows it, as in
 // align_pair; blocks start in [blo, bhi).
-template <class Aligner>
-__device__ int align_pair_dev(const KeySeeds &S, const uint16_t *info, bool comp, bool self, const Seq &A,
-                              const Seq &B, int64_t amxpos, int64_t maxdag, Aligner &AL, Path &path, OvlArena &O,
-                              PairResult &R, int lane, int64_t blo, int64_t bhi) {
+template <class Sink>
+__device__ int scan_blocks(const KeySeeds &S, const uint16_t *info, int64_t blo, int64_t bhi, Sink &K) {
+  const int lane = threadIdx.x & 31;
   const int64_t n = S.n;
-  R.calls = 0;
-  R.nhit = 0;
-  R.nlas = 0;
-  R.exit_bepos = path.bepos;
-  O.nov = 0;
-  if (bhi < 0 || bhi > n) bhi = n;
-  if (blo < 0) blo = 0;
-  if (blo >= bhi) return 0;
-  ChainSink<Aligner> K{comp, self, A, B, AL, path, O, R, lane, 32, amxpos, (int64_t)A.len + B.len,
-                           (int64_t)A.len - maxdag, (int64_t)A.len - amxpos, 0, 0, -1};
   int64_t pend = -1;  // the last band start seen, its block not yet decided
   int pend_sum = 0;
   bool pend_new = false;
   bool done = false;
+  int empty = 0;  // steps since the last band start
   for (int64_t base = blo; base < n && !done; base += 32) {
     const int64_t i = base + lane;
     const uint16_t v = i < n ? info[i] : 0;
     unsigned starts = __ballot_sync(FULL, (v & BI_START) != 0);
+    empty = starts ? 0 : empty + 1;
+    if (empty == 4) {  // a long band: on to the next one's start
+      base = S.next_band_start(base + 32, n) - 32;
+      empty = 0;
+    }
     while (starts) {
       const int l = __ffs(starts) - 1;
       starts &= starts - 1;
@@ -424,6 +691,24 @@ __device__ int align_pair_dev(const KeySeeds &S, const uint16_t *info, bool comp
     K.alast = -1;
     if (S.scan_block(pend, n, n, K)) return 1;
   }
+  return 0;
+}
+
+template <class Aligner>
+__device__ int align_pair_dev(const KeySeeds &S, const uint16_t *info, bool comp, bool self, const Seq &A,
+                              const Seq &B, int64_t amxpos, int64_t maxdag, Aligner &AL, Path &path, OvlArena &O,
+                              PairResult &R, int lane, int64_t blo, int64_t bhi) {
+  R.calls = 0;
+  R.nhit = 0;
+  R.nlas = 0;
+  R.exit_bepos = path.bepos;
+  O.nov = 0;
+  if (bhi < 0 || bhi > S.n) bhi = S.n;
+  if (blo < 0) blo = 0;
+  if (blo >= bhi) return 0;
+  ChainSink<Aligner> K{comp, self, A, B, AL, path, O, R, lane, 32, amxpos, (int64_t)A.len + B.len,
+                           (int64_t)A.len - maxdag, (int64_t)A.len - amxpos, 0, 0, -1};
+  if (scan_blocks(S, info, blo, bhi, K)) return 1;
   R.exit_bepos = path.bepos;
   return 0;
 }
@@ -566,7 +851,82 @@ struct TaskSums {
   }
 };
 
-// The persistent alignment loop, in four builds: MINB = 1 keeps every
+constexpr int IDLE_POLLS = 1 << 16;  // bound of a warp's wait for scouts, a poll every 20 us or so
+
+// The next queued scout, -1 if there is none, -2 if it was not to be run.
+__device__ int take_scout(const ShareTable &X, int lane) {
+  int got = -1;
+  if (lane == 0) {
+    unsigned h = *(volatile unsigned *)X.qhead;
+    while (h < min(*(volatile unsigned *)X.qtail, (unsigned)X.qcap)) {
+      const unsigned old = atomicCAS(X.qhead, h, h + 1);
+      if (old == h) {
+        got = (int)h;
+        break;
+      }
+      h = old;
+    }
+    if (got >= 0) {
+      // ours to run, unless its task has come to it first
+      int state = SCOUT_UNWRITTEN;
+      for (int poll = 0; poll < SHARE_POLLS; poll++) {
+        state = atomicCAS(&X.scouts[got].state, SCOUT_READY, SCOUT_RUNS);
+        if (state != SCOUT_UNWRITTEN) break;
+        __nanosleep(100);
+      }
+      if (state != SCOUT_READY) got = -2;
+    }
+  }
+  got = __shfl_sync(FULL, got, 0);
+  __threadfence();
+  return got;
+}
+
+// A queued call, its result left for its task, or a start grown both ways.
+__device__ void run_scout(const AlignLaunch &P, WarpWork &W, const AlignSpec &spec, Scout &q, int lane) {
+  const int a = __ldcg(&q.a), b = __ldcg(&q.b), comp = __ldcg(&q.comp);
+  const int low = __ldcg(&q.low), hgh = __ldcg(&q.hgh), anti = __ldcg(&q.anti);
+  const Seq A = contig_seq(P, a, true, comp != 0), B = contig_seq(P, b, false, false);
+  W.err = 0;
+  W.task = nullptr;
+  W.pair = (uint32_t)a | ((uint32_t)b << 15) | ((uint32_t)comp << 30);
+  if (!__ldcg(&q.call)) {
+    scout_w(W, spec, A, B, comp != 0, low, hgh, anti);
+    return;
+  }
+  Path path;
+  path.tlen = path.diffs = path.abpos = path.bbpos = path.aepos = path.bepos = 0;
+  path.trace_off = 0;
+  bool done = local_alignment_w<true, true>(W, spec, A, B, comp != 0, path, low, hgh, anti, -1, -1) == 0;
+  const ShareTable &X = *W.share;
+  const int pairs = path.tlen / 2;
+  unsigned long long off = 0;
+  if (done) {
+    if (lane == 0) off = atomicAdd(X.nlist, (unsigned long long)pairs);
+    off = __shfl_sync(FULL, off, 0);
+    done = (int64_t)off + pairs <= X.list_cap;
+  }
+  if (done) {
+    const uint32_t *pt = reinterpret_cast<const uint32_t *>(W.points + path.trace_off);
+    for (int i = lane; i < pairs; i += 32) X.list[off + i] = pt[i];
+    if (lane == 0) {
+      q.abpos = path.abpos;
+      q.aepos = path.aepos;
+      q.bbpos = path.bbpos;
+      q.bepos = path.bepos;
+      q.diffs = path.diffs;
+      q.tlen = path.tlen;
+      q.off = (int64_t)off;
+    }
+  }
+  __threadfence();
+  __syncwarp();
+  if (lane == 0) *(volatile int *)&q.state = done ? SCOUT_DONE : SCOUT_VOID;
+}
+
+// The persistent alignment loop.  SHARE: with the launch's table of shared
+// extensions and its scouts, for launches of long contigs (prepare_share,
+// capi.cu).  MINB = 1 keeps every
 // register a warp's wave loop wants (255, two CTAs per SM), for launches
 // bounded by their longest tasks; MINB = 3, 4 and 5 trade spills for more
 // resident warps (three to five CTAs per SM: 168, 128 or 96 registers), for
@@ -575,17 +935,21 @@ struct TaskSums {
 // register form of the waves of 32 to 124 diagonals (align_warp.cuh, extend).
 // 2 x 200 Mbp repeat-rich, two to five CTAs: 342, 298, 240, 224 ms of pair
 // phase; 2 x 41 kbp: 10.8, 11.1, 14.4, 14.8.
-template <int MINB>
-__global__ void __launch_bounds__(ALIGN_THREADS, MINB) k_align_pairs(AlignLaunch P) {
+template <int MINB, bool SHARE>
+__global__ void __launch_bounds__(ALIGN_THREADS, MINB) k_align_pairs(const __grid_constant__ AlignLaunch P) {
   __shared__ BlockSeed s_block[ALIGN_THREADS / 32][32];
   const int lane = threadIdx.x & 31;
   const int64_t wid = ((int64_t)blockIdx.x * ALIGN_THREADS + threadIdx.x) >> 5;
   if (wid >= P.nwarps) return;
   const AlignSpec spec = launch_spec(P);
   WarpWork W = warp_work(P, wid);
+  W.sm = reinterpret_cast<int *>(s_block[threadIdx.x >> 5]);  // (scan_block holds nothing there while a call runs)
 
   OvlArena O = warp_arena(P, wid);
   TaskSums sums;
+  const unsigned total = (unsigned)P.ntasks + (unsigned)P.nsmall;
+  bool drained = false;
+  int idle = 0;
 
   while (true) {
     unsigned t = 0;
@@ -598,9 +962,29 @@ __global__ void __launch_bounds__(ALIGN_THREADS, MINB) k_align_pairs(AlignLaunch
       f = __shfl_sync(FULL, f, 0);
       if (f) break;
     }
-    if (lane == 0) t = atomicAdd(P.next_task, 1u);
-    t = __shfl_sync(FULL, t, 0);
-    if (t >= (unsigned)P.ntasks + (unsigned)P.nsmall) break;
+    if (SHARE && drained) {
+      const int sc = take_scout(*P.share, lane);
+      if (sc == -2) continue;
+      if (sc >= 0) {
+        run_scout(P, W, spec, P.share->scouts[sc], lane);
+        continue;
+      }
+    }
+    if (!drained) {
+      if (lane == 0) t = atomicAdd(P.next_task, 1u);
+      t = __shfl_sync(FULL, t, 0);
+      drained = t >= total;
+    }
+    if (drained) {
+      // no task left: stay for the scouts of those that still run
+      if (!SHARE || idle == IDLE_POLLS) break;
+      unsigned ended = 0;
+      if (lane == 0) ended = *(volatile unsigned *)P.share->ended;
+      if (__shfl_sync(FULL, ended, 0) >= total) break;
+      idle++;
+      __nanosleep(20000);
+      continue;
+    }
     int item = 0;
     const PairTask tk = t < (unsigned)P.ntasks ? planned_task(P, t, lane, &item)
                                                : small_task(P, P.small[t - P.ntasks]);
@@ -617,12 +1001,15 @@ __global__ void __launch_bounds__(ALIGN_THREADS, MINB) k_align_pairs(AlignLaunch
     path.trace_off = 0;
     int64_t blo = 0, bhi = S.n;
     if (tk.seg >= 0) {
-      blo = next_band_start(S, tk.slo - tk.lo, S.n, lane);
-      bhi = next_band_start(S, tk.shi - tk.lo, S.n, lane);
+      blo = S.next_band_start(tk.slo - tk.lo, S.n);
+      bhi = S.next_band_start(tk.shi - tk.lo, S.n);
     }
     PairResult R;
-    WarpAligner<(MINB <= 3)> AL{W, spec, P.memo, tk.a, tk.b};
     const uint16_t *info = (tk.comp ? P.infoC : P.infoN) + tk.lo;
+    TaskChains TC{S, info, &P.memo, tk.a, tk.b, tk.comp != 0, P.amxpos, (int64_t)A.len - P.maxdag,
+                  (int64_t)A.len - P.amxpos, blo, bhi, 0, 0, 0};
+    W.task = SHARE && !tk.self ? &TC : nullptr;
+    WarpAligner<MINB <= 3, SHARE> AL{W, spec, P.memo, tk.a, tk.b, SHARE && !tk.self ? &TC : nullptr};
     int rc = align_pair_dev(S, info, tk.comp != 0, tk.self != 0, A, B, P.amxpos, P.maxdag, AL, path, O, R, lane,
                             blo, bhi);
     __syncwarp();
@@ -659,9 +1046,12 @@ __global__ void __launch_bounds__(ALIGN_THREADS, MINB) k_align_pairs(AlignLaunch
       sums.add(po, t);
       if (t >= (unsigned)P.ntasks) sums.add_small(P, tk, po);
       else if (tk.seg < 0) P.pout[item] = po;
+      if (SHARE) atomicAdd(P.share->ended, 1u);
     }
     __syncwarp();
   }
+  sums.waves += W.waves;  // of scouts
+  sums.cells += W.cells;
   if (lane == 0) sums.flush(P);
   if (lane == 0 && W.la_cycles > 0) atomicAdd(&P.prof[0], (unsigned long long)W.la_cycles);
 }
@@ -673,7 +1063,7 @@ __global__ void __launch_bounds__(ALIGN_THREADS, MINB) k_align_pairs(AlignLaunch
 // output.  The pair's calls are the ranges' sum and its exit bepos the last
 // range's with a call (the entry value when none called).
 __global__ void __launch_bounds__(ALIGN_THREADS)
-k_finish_pairs(AlignLaunch P) {
+k_finish_pairs(const __grid_constant__ AlignLaunch P) {
   const int lane = threadIdx.x & 31;
   const int64_t wid = ((int64_t)blockIdx.x * ALIGN_THREADS + threadIdx.x) >> 5;
   if (wid >= P.nwarps) return;
@@ -725,12 +1115,15 @@ k_finish_pairs(AlignLaunch P) {
 // (abpos aepos bbpos bepos diffs tlen status) and copies its tlen uint16
 // trace values into a shared pool.
 __global__ void __launch_bounds__(ALIGN_THREADS)
-k_local_batch(AlignLaunch P) {
+k_local_batch(const __grid_constant__ AlignLaunch P) {
   const int lane = threadIdx.x & 31;
   const int64_t wid = ((int64_t)blockIdx.x * ALIGN_THREADS + threadIdx.x) >> 5;
   if (wid >= P.nwarps) return;
   const AlignSpec spec = launch_spec(P);
+  __shared__ int s_walk[ALIGN_THREADS / 32][128];
   WarpWork W = warp_work(P, wid);
+  W.sm = s_walk[threadIdx.x >> 5];
+  W.share = nullptr;  // requests grow alone: their lists need not share paths
   while (true) {
     unsigned long long r = 0;
     if (lane == 0) r = atomicAdd(P.lreq_next, 1ull);
@@ -744,7 +1137,7 @@ k_local_batch(AlignLaunch P) {
     Path path;
     path.tlen = path.diffs = path.abpos = path.bbpos = path.aepos = path.bepos = 0;
     path.trace_off = 0;
-    int status = local_alignment_w<true>(W, spec, A, B, comp, path, q[3], q[4], q[5], q[6], q[7]) ? (W.err | 0x100) : 0;
+    int status = local_alignment_w<true, false>(W, spec, A, B, comp, path, q[3], q[4], q[5], q[6], q[7]) ? (W.err | 0x100) : 0;
     int64_t off = -1;
     if (status == 0 && path.tlen > 0) {
       unsigned long long o = 0;
@@ -926,10 +1319,11 @@ void launch_base_counts(const uint8_t *bps, const int64_t *clen, const int64_t *
 }
 
 void launch_align(const AlignLaunch &P, int grid, cudaStream_t st) {
-  if (P.min_blocks == 5) k_align_pairs<5><<<grid, ALIGN_THREADS, 0, st>>>(P);
-  else if (P.min_blocks == 4) k_align_pairs<4><<<grid, ALIGN_THREADS, 0, st>>>(P);
-  else if (P.min_blocks == 3) k_align_pairs<3><<<grid, ALIGN_THREADS, 0, st>>>(P);
-  else k_align_pairs<1><<<grid, ALIGN_THREADS, 0, st>>>(P);
+  if (P.min_blocks == 5) k_align_pairs<5, false><<<grid, ALIGN_THREADS, 0, st>>>(P);
+  else if (P.min_blocks == 4) k_align_pairs<4, false><<<grid, ALIGN_THREADS, 0, st>>>(P);
+  else if (P.min_blocks == 3) k_align_pairs<3, false><<<grid, ALIGN_THREADS, 0, st>>>(P);
+  else if (P.share) k_align_pairs<1, true><<<grid, ALIGN_THREADS, 0, st>>>(P);
+  else k_align_pairs<1, false><<<grid, ALIGN_THREADS, 0, st>>>(P);
 }
 
 void launch_finish(const AlignLaunch &P, int grid, cudaStream_t st) {

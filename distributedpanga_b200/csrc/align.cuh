@@ -3,6 +3,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "align_core.cuh"
+#include "align_share.cuh"
 #include "common.cuh"
 #include "seeds.cuh"
 #include "memo.h"
@@ -88,6 +89,7 @@ struct AlignLaunch {
   // pairs' finishing step [1], zero at launch
   unsigned long long *prof;
   CallMemo memo;
+  const aln::ShareTable *share;  // shared extensions (null: off)
   int long_waves;     // a wave loop past this many waves flags its SM
   const U128 *keysN, *keysC;
   // per seed of each unit: band start (bit 15), previous band of the pair

@@ -39,6 +39,7 @@
 #pragma once
 #include <stdint.h>
 #include "align_core.cuh"
+#include "align_share.cuh"
 
 namespace pga {
 namespace aln {
@@ -58,6 +59,14 @@ struct __align__(16) RingCell {
   int HA, HM;
 };
 
+__device__ __forceinline__ uint32_t mix32(uint32_t h) {
+  h ^= h >> 16;
+  h *= 0x85ebca6bu;
+  h ^= h >> 13;
+  h *= 0xc2b2ae35u;
+  return h ^ (h >> 16);
+}
+
 struct WarpWork {
   RingCell *C[2];  // waves by diagonal & (vcap - 1), in growth coordinates
   int *V[2];
@@ -73,9 +82,16 @@ struct WarpWork {
   int long_waves;        // waves of one wave loop that make a call long (0: never)
   int flagged;           // this warp has flagged its SM
   long long la_cycles;   // SM cycles spent in Local_Alignment calls (lane-uniform)
+  int *sm;                  // 128 words of this warp's shared memory
+  const ShareTable *share;  // null: extensions are not shared
+  unsigned pair;            // the call's contigs and orientation, for the table's keys
+  const struct TaskChains *task;  // the task's chains, until its scouts are queued (null: none are)
 };
 
 constexpr int PEBBLE_CHUNK = 4096;
+
+// Queues the scouts of the warp's task if warps are free for them (align.cu).
+__device__ void scout_if_free(WarpWork &W);
 
 // Reserve `cnt` consecutive pebbles for the warp (lane-uniform call).
 __device__ __forceinline__ int64_t warp_pebbles(WarpWork &W, int cnt) {
@@ -164,6 +180,7 @@ struct Wave {
   int low, hgh, dif, cur;
   int besta, bestx, lasta, trima, trimx, trimd, trimha;
   int more;
+  int line;  // the antidiagonal narrow_waves stops at
 };
 
 // Snake along diagonal k from x in rounds of 16 * N bases: stops at the first
@@ -215,7 +232,7 @@ struct TrimTest {
 // The trace marks the lanes' snakes passed: one pebble each unless the path
 // has it already (hm).  next / end: the warp's pebble chunk.  Returns false
 // when the pool is full.
-__device__ __forceinline__ bool drop_pebbles(const WarpWork &W, const Wave &E, bool act, int k, int x, int dif, int &ha,
+__device__ __forceinline__ bool drop_pebbles(const PebblePool &pool, const Wave &E, bool act, int k, int x, int dif, int &ha,
                                              int &hm, int &nak, int &next, int &end) {
   const int lane = threadIdx.x & 31;
   bool cross = act && x >= nak;
@@ -225,16 +242,16 @@ __device__ __forceinline__ bool drop_pebbles(const WarpWork &W, const Wave &E, b
     const int cnt = __popc(mb);
     if (next + cnt > end) {
       unsigned long long base = 0;
-      if (lane == 0) base = atomicAdd(W.pool.next, (unsigned long long)PEBBLE_CHUNK);
+      if (lane == 0) base = atomicAdd(pool.next, (unsigned long long)PEBBLE_CHUNK);
       base = __shfl_sync(FULL, base, 0);
       // pebble numbers are int
-      if ((int64_t)base + PEBBLE_CHUNK > min(W.pool.cap, (int64_t)I32MAX)) return false;
+      if ((int64_t)base + PEBBLE_CHUNK > min(pool.cap, (int64_t)I32MAX)) return false;
       next = (int)base;
       end = next + PEBBLE_CHUNK;
     }
     if (mk) {
       const int s = next + __popc(mb & ((1u << lane) - 1u));
-      *reinterpret_cast<int4 *>(W.pool.cells + s) = make_int4(ha, E.sg * k, dif, E.sg * nak);
+      *reinterpret_cast<int4 *>(pool.cells + s) = make_int4(ha, E.sg * k, dif, E.sg * nak);
       ha = s;
       hm = nak;
     }
@@ -299,6 +316,125 @@ __device__ __forceinline__ int can_grow(const Wave &S, int besta) {
   return S.limB - besta + S.bestx != 0 && S.limA - S.bestx != 0 ? 1 : 0;
 }
 
+// What an extension shares: its record and last entry (-1: none), and the
+// entry it joined (-1: none), with its best diagonal's head pebble there (the
+// path most likely comes through that one).
+struct Sharing {
+  int rec, last, joined, guess;
+  int from;   // the extension's first antidiagonal
+  bool full;  // no room for more entries
+};
+
+// The first multiple of SHARE_LINE above antidiagonal a.
+__device__ __forceinline__ int next_line(int a) { return (a & ~(SHARE_LINE - 1)) + SHARE_LINE; }
+
+// A narrow wave, in the ring, whose best crossed a line (`way`: the pair,
+// orientation and direction): joins the extension whose wave there was the
+// same (returned), or enters it.
+__device__ __noinline__ bool cross_line(const WarpWork &W, const Wave &wave, unsigned way, Sharing &io) {
+  const ShareTable &X = *W.share;
+  Sharing *S = &io;
+  const int lane = threadIdx.x & 31;
+  const int low = wave.low, hgh = wave.hgh, besta = wave.besta, bestx = wave.bestx, lasta = wave.lasta;
+  const int dif = wave.dif, next = (int)W.chunk_next;
+  if (besta - S->from < SHARE_MIN) return false;
+  const int k = low + ((lane - low) & 31), vi = k & (W.vcap - 1);
+  const bool live = k <= hgh;
+  int V = NO_WAVE, HA = -1, HM = 0, NA = 0;
+  uint64_t T = 0;
+  if (live) {
+    const RingCell c = W.C[wave.cur][vi];
+    V = W.V[wave.cur][vi];
+    NA = W.NA[vi];
+    T = c.T;
+    HA = c.HA;
+    HM = c.HM;
+  }
+  // which diagonals have the same head pebble: the first lane with this one's
+  const int pat = __ffs(__match_any_sync(FULL, live ? HA : -2 - lane)) - 1;
+  // the state's key
+  const uint32_t tl = (uint32_t)T, th = (uint32_t)(T >> 32) & HIST_HI;
+  const uint32_t a = mix32(V + 0x9e3779b9u * (lane + 1)) + mix32(tl ^ 0x7f4a7c15u), b = mix32(th + HM) + mix32(NA ^ tl ^ pat << 16);
+  const uint32_t h1 = __reduce_xor_sync(FULL, live ? mix32(a + 31 * b) : 0);
+  const uint32_t h2 = __reduce_add_sync(FULL, live ? mix32(b ^ (a * 0x27d4eb2fu)) : 0);
+  const uint32_t u = mix32(besta + mix32(lasta + mix32(bestx + mix32(way))));
+  const unsigned long long key = ((unsigned long long)mix32(h1 + u) << 32 | mix32(h2 ^ (u + mix32(low + 37 * hgh)))) | 1;
+  int val = -2;
+  unsigned at = 0;
+  if (lane == 0) {
+    at = (unsigned)(key >> 20) & X.mask;
+    for (int probe = 0; probe < SHARE_PROBES; probe++, at = (at + 1) & X.mask) {
+      const unsigned long long old = atomicCAS(&X.keys[at], 0ull, key);
+      if (old == 0) {
+        val = -3;  // ours to write
+        break;
+      }
+      if (old == key) {
+        for (int poll = 0; poll < SHARE_POLLS && (val = *(volatile int *)&X.vals[at]) == -1; poll++) __nanosleep(100);
+        break;
+      }
+    }
+  }
+  val = __shfl_sync(FULL, val, 0);
+  if (val == -3) {
+    int e = -1, r = S->rec;
+    if (lane == 0) {
+      e = (int)min(atomicAdd(X.nentry, 1u), (unsigned)X.entry_cap);
+      if (e < X.entry_cap && r < 0) r = (int)min(atomicAdd(X.nrec, 1u), (unsigned)X.rec_cap);
+      if (e >= X.entry_cap || r >= X.rec_cap) {
+        e = -1;
+        *(volatile int *)&X.vals[at] = -2;
+      }
+    }
+    e = __shfl_sync(FULL, e, 0);
+    r = __shfl_sync(FULL, r, 0);
+    if (e < 0) {
+      S->full = true;
+      return false;
+    }
+    ShareEntry &E = X.entries[e];
+    if (lane == 0) {
+      if (S->rec < 0) X.recs[r].status = 0;
+      E.rec = r;
+      E.prev = S->last;
+      E.low = low;
+      E.hgh = hgh;
+      E.besta = besta;
+      E.bestx = bestx;
+      E.lasta = lasta;
+      E.dif = dif;
+      E.mark = next;
+      E.way = way;
+      E.kind = SHARE_NONE;
+    }
+    E.V[lane] = V;
+    E.HA[lane] = live ? HA : -1;
+    E.HM[lane] = HM;
+    E.pat[lane] = pat;
+    E.NA[lane] = NA;
+    E.T[lane] = T;
+    S->rec = r;
+    S->last = e;
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) *(volatile int *)&X.vals[at] = e;
+    return false;
+  }
+  if (val < 0) return false;
+  const ShareEntry &E = X.entries[val];
+  __threadfence();
+  bool same = __ldcg(&E.way) == way && __ldcg(&E.low) == low && __ldcg(&E.hgh) == hgh && __ldcg(&E.besta) == besta &&
+              __ldcg(&E.bestx) == bestx && __ldcg(&E.lasta) == lasta;
+  if (live)
+    same = same && __ldcg(&E.V[lane]) == V && __ldcg(&E.HM[lane]) == HM && __ldcg(&E.NA[lane]) == NA &&
+           __ldcg(&E.pat[lane]) == pat &&
+           ((__ldcg(&E.T[lane]) ^ T) & ((1ull << 61) - 1)) == 0;
+  if (!__all_sync(FULL, same)) return false;
+  S->joined = val;
+  S->guess = __shfl_sync(FULL, HA, (2 * bestx - besta) & 31);
+  return true;
+}
+
 // ---------------------------------------------------------------------------
 // Narrow waves, at most 31 diagonals: diagonal k lives in lane k mod 32, its
 // state in registers, the previous wave's neighbours come by shuffle.  The
@@ -312,21 +448,24 @@ __device__ __forceinline__ int can_grow(const Wave &S, int besta) {
 // that step's sequence words are on their way, before the loop's end
 // conditions are tested and anything of the new wave is kept.
 //
-// Runs until the loop ends, the next wave does not fit, or the wave count
-// reaches `stop`.  Returns 1 when the pebble pool is full.
+// Runs until the loop ends, the next wave does not fit, the best crosses
+// `line`, or the wave count reaches `stop`.  Returns 1 when the pebble pool is
+// full.
 // ---------------------------------------------------------------------------
 constexpr int NARROW = 31;
 constexpr int PAST_MAX = (1 << 26) - 1;  // a best further past than this takes the general record search
 
-__device__ __forceinline__ int narrow_waves(WarpWork &W, Wave &io, int stop) {
+__device__ __noinline__ int narrow_waves(WarpWork &W, Wave &io, int stop) {
   const int lane = threadIdx.x & 31;
   const int lup = (lane + 1) & 31, ldn = (lane - 1) & 31;
   Wave S = io;
+  const PebblePool pool = W.pool;
   const TrimTest trim(S.dscore);
   const int vmask = W.vcap - 1;
   int next = (int)W.chunk_next, end = (int)W.chunk_end;
   int ncells = 0;
   int low = S.low, hgh = S.hgh, dif = S.dif, besta = S.besta, lasta = S.lasta;
+  const int line = S.line;
 
   // the last wave: lane's diagonal kw (if live), its furthest x, what came with it
   int V = NO_WAVE, HA = -1, HM = 0, NA = 0, X = 0, kw = low + ((lane - low) & 31);
@@ -344,7 +483,7 @@ __device__ __forceinline__ int narrow_waves(WarpWork &W, Wave &io, int stop) {
   }
   // the last wave's pebbles and record; once done, doing it again changes nothing
   auto settle = [&]() {
-    if (!drop_pebbles(W, S, live, kw, X, dif, HA, HM, NA, next, end)) return false;
+    if (!drop_pebbles(pool, S, live, kw, X, dif, HA, HM, NA, next, end)) return false;
     const int L = kr & 31;
     const uint64_t t = __shfl_sync(FULL, T, L);
     const int hr = __shfl_sync(FULL, HA, L);
@@ -389,7 +528,7 @@ __device__ __forceinline__ int narrow_waves(WarpWork &W, Wave &io, int stop) {
       full = true;
       break;
     }
-    if (!(S.more && lasta >= besta - TRIM_MLAG && low <= hgh && wide < NARROW && dif < stop)) break;
+    if (!(S.more && lasta >= besta - TRIM_MLAG && low <= hgh && wide < NARROW && dif < stop && besta < line)) break;
     dif += 1;
     ncells += wide + 1;
 
@@ -406,9 +545,13 @@ __device__ __forceinline__ int narrow_waves(WarpWork &W, Wave &io, int stop) {
     int run = 0;
     if (go) {
       run = match_loaded<4>(a, (ia & 15) << 1, b, (ib & 15) << 1);
-      for (int r = run; r == 64 && run < mx; run += r) {
-        const int qa = ia + run, qb = ib + run;
-        r = match_words<4>(S.pa + (qa >> 4), (qa & 15) << 1, S.pb + (qb >> 4), (qb & 15) << 1);
+      if (run == 64) {
+        int r;
+        do {
+          const int qa = min(ia + run, ia + mx), qb = min(ib + run, ib + mx);
+          r = match_words<2>(S.pa + (qa >> 4), (qa & 15) << 1, S.pb + (qb >> 4), (qb & 15) << 1);
+          run += r;
+        } while (r == 32 && run < mx);
       }
       run = min(run, mx);
     }
@@ -427,24 +570,19 @@ __device__ __forceinline__ int narrow_waves(WarpWork &W, Wave &io, int stop) {
     kr = nlow + (key & 31);
     low = nlow;
     hgh = nhgh;
-    if (hits || key >= (PAST_MAX << 5)) {
-      if (key >= (PAST_MAX << 5)) {
-        rc = __reduce_max_sync(FULL, act ? c : NO_WAVE);
-        kr = __reduce_max_sync(FULL, act && c == rc ? k : NO_WAVE);
-      }
-      if (hits) {
-        // snakes that reached a sequence's end clip the window
-        if (!settle()) {
-          full = true;
-          break;
-        }
-        const bool hit = hits >> lane & 1, hb = met_b(S, x, k, go);
-        const int ka = __reduce_min_sync(FULL, hit && !hb ? k : I32MAX);
-        const int kb = __reduce_max_sync(FULL, hit && hb ? k : NO_WAVE);
-        S.more = can_grow(S, rc);
-        if (ka != I32MAX) hgh = ka - 1;
-        if (kb != NO_WAVE) low = kb + 1;
-      }
+    if (key >= (PAST_MAX << 5)) {
+      rc = __reduce_max_sync(FULL, act ? c : NO_WAVE);
+      kr = __reduce_max_sync(FULL, act && c == rc ? k : NO_WAVE);
+    }
+    if (hits) {
+      // snakes that reached a sequence's end clip the window
+      const bool hit = hits >> lane & 1, hb = met_b(S, x, k, go);
+      const int ka = __reduce_min_sync(FULL, hit && !hb ? k : I32MAX);
+      const int kb = __reduce_max_sync(FULL, hit && hb ? k : NO_WAVE);
+      if (rc > besta) S.bestx = (rc + kr) >> 1;
+      S.more = can_grow(S, rc);
+      if (ka != I32MAX) hgh = ka - 1;
+      if (kb != NO_WAVE) low = kb + 1;
     }
     besta = rc;
     // WAVE_LAG pruning from either end, between the clipped ends
@@ -503,12 +641,13 @@ __device__ __forceinline__ T pick(const T (&v)[J], int j) {
 }
 
 template <int J>
-__device__ __forceinline__ int block_waves(WarpWork &W, Wave &io, int stop) {
+__device__ __noinline__ int block_waves(WarpWork &W, Wave &io, int stop) {
   constexpr int LG = J == 2 ? 1 : 2;
   static_assert(J == 1 << LG, "J is 2 or 4");
   const int lane = threadIdx.x & 31;
   const int lup = (lane + 1) & 31, ldn = (lane - 1) & 31;
   Wave S = io;
+  const PebblePool pool = W.pool;
   const TrimTest trim(S.dscore);
   const int vmask = W.vcap - 1;
   int next = (int)W.chunk_next, end = (int)W.chunk_end;
@@ -617,9 +756,19 @@ __device__ __forceinline__ int block_waves(WarpWork &W, Wave &io, int stop) {
       if (act[j]) key = max(key, (past << 7) + (k - nlow));
     }
     if (__any_sync(FULL, cross)) {
+#pragma unroll 1
+      for (int j = 0; j < J; j++) {  // (one copy of the loop: few diagonals cross a mark)
+        int ha = pick<J>(HA, j), hm = pick<J>(HM, j), nak = pick<J>(NA, j);
+        const int k = kw + j;
+        full |= !drop_pebbles(pool, S, k >= nlow && k <= nhgh, k, pick<J>(x, j), dif, ha, hm, nak, next, end);
 #pragma unroll
-      for (int j = 0; j < J; j++)
-        full |= !drop_pebbles(W, S, act[j], kw + j, x[j], dif, HA[j], HM[j], NA[j], next, end);
+        for (int q = 0; q < J; q++)
+          if (q == j) {
+            HA[q] = ha;
+            HM[q] = hm;
+            NA[q] = nak;
+          }
+      }
       if (full) break;
     }
 
@@ -740,7 +889,7 @@ __device__ __forceinline__ int block_waves(WarpWork &W, Wave &io, int stop) {
 // diagonals per pass from the highest down.  Runs until the loop ends, the
 // window has at most `least` diagonals, or the wave count reaches `stop`.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int wide_waves(WarpWork &W, Wave &io, int stop, int least) {
+__device__ __noinline__ int wide_waves(WarpWork &W, Wave &io, int stop, int least) {
   const int lane = threadIdx.x & 31;
   Wave S = io;
   const TrimTest trim(S.dscore);
@@ -800,7 +949,7 @@ __device__ __forceinline__ int wide_waves(WarpWork &W, Wave &io, int stop, int l
       const uint64_t b = hist_step(t0, run);
       x += run;
       c = (x << 1) - k;
-      if (!drop_pebbles(W, S, act, k, x, S.dif, ha, hm, nak, next, end)) {
+      if (!drop_pebbles(W.pool, S, act, k, x, S.dif, ha, hm, nak, next, end)) {
         err = ALN_ERR_CELLS;
         break;
       }
@@ -860,17 +1009,241 @@ __device__ __forceinline__ int wide_waves(WarpWork &W, Wave &io, int stop, int l
   return 0;
 }
 
+// A trace being walked back from its tip: intervals (diffs, b-delta) in the
+// free end of the trace buffer, last first -- forward ones down from the
+// buffer's top, reverse ones up from its bottom.
+struct TraceWalk {
+  bool fwd, inner;   // inner: the reverse path of a call whose forward path has a trace
+  int sg, mida, tspace, aoff;
+  int64_t room;      // intervals the free end holds
+  int64_t base, lim; // the extension's first pebble, and a bound of its pebbles
+  int64_t n;         // intervals so far
+  int last;          // the extension's entries not yet crossed, going back
+  int start;         // the diagonal the path starts on
+  // the interval of a reverse path that ends inside the forward path's first
+  // one, which it extends
+  int jd, jb;
+
+  __device__ __forceinline__ uint32_t *slot(const WarpWork &W, int64_t i) const {
+    return reinterpret_cast<uint32_t *>(W.points) + (fwd ? (W.point_cap >> 1) - 1 - i : i);
+  }
+  __device__ __forceinline__ void put(const WarpWork &W, int dd, int db) {
+    if ((threadIdx.x & 31) == 0 && n < room) *slot(W, n) = (uint32_t)(uint16_t)dd | (uint32_t)(uint16_t)db << 16;
+    n += 1;
+  }
+  // the b position a pebble stands for; the start pebble stands at its
+  // antidiagonal's going forward
+  __device__ __forceinline__ int bpos(int4 q) const { return fwd && q.x < 0 ? (mida - q.y) >> 1 : q.w - q.y; }
+  __device__ __forceinline__ bool inside(int4 q) const { return !fwd && q.x < 0 && q.w % tspace != aoff; }
+
+  // The end past the last mark: an interval of its own, or part of the one
+  // before (left in dd, db).
+  __device__ __forceinline__ void tip(const WarpWork &W, int4 q, int trimx, int trimy, int trimd, int &dd, int &db) {
+    const int qb = bpos(q);
+    dd = trimd - q.z;
+    db = sg * (trimy - qb);
+    if (inside(q) || qb + q.y != trimx) {
+      if (inside(q) && inner) {
+        jd = dd;
+        jb = db;
+      } else
+        put(W, dd, db);
+      dd = db = 0;
+    } else if (qb == trimy)
+      dd = db = 0;
+    else if (!fwd && q.x < 0) {
+      jd = dd;
+      jb = db;
+    }
+  }
+};
+
+// How the path crosses the lines of the entries that pebble `head` is older
+// than: p is the first pebble after them (kind PEBBLE), or the path's head is
+// from before (HEAD; NONE where that leaves no trace to share).
+__device__ __noinline__ void cross_entries(const WarpWork &W, TraceWalk &T, int head, int kind, int4 p) {
+  const int lane = threadIdx.x & 31;
+  while (T.last >= 0) {
+    ShareEntry &O = W.share->entries[T.last];
+    if (head >= __ldcg(&O.mark)) return;
+    const unsigned eq = __ballot_sync(FULL, __ldcg(&O.HA[lane]) == head);
+    if (lane == 0) {
+      O.kind = eq ? kind : SHARE_NONE;
+      O.lane = __ffs(eq) - 1;
+      O.after = (int)T.n;
+      O.pdiag = p.y;
+      O.pdiff = p.z;
+      O.pmark = p.w;
+    }
+    T.last = __ldcg(&O.prev);
+  }
+}
+
+// The walk from pebble values q (its slot's successor is q.x) to the path's
+// start.  A path's pebbles lie a dozen or so slots apart, so the pointers of
+// the 128 slots up to the next one come into shared memory at once (the block
+// below it already on its way), one lane per pebble found there takes its
+// interval, and only the hops within a block are a chain: a warp's load per
+// pebble took 360 ns each.  dd, db: what the first interval has already.
+// Returns an error code.
+template <bool SHARE>
+__device__ __noinline__ int walk_back(const WarpWork &W, TraceWalk &io, int4 q, int dd, int db) {
+  constexpr int SPAN = 128;
+  const int lane = threadIdx.x & 31;
+  const int4 *cl = reinterpret_cast<const int4 *>(W.pool.cells);  // ptr, diag, diff, mark
+  int *sm = W.sm;
+  TraceWalk T = io;
+  int near = I32MAX, err = 0, ahead[SPAN / 32];
+  int64_t steps = 0;
+  int mark = SHARE && T.last >= 0 ? __ldcg(&W.share->entries[T.last].mark) : -1;
+  while (q.x >= 0) {
+    const int h = q.x;
+    if (h < T.base || steps > T.lim || T.n > T.room) {
+      err = T.n > T.room ? ALN_ERR_POINTS : ALN_ERR_CELLS;
+      break;
+    }
+    if (SHARE && h < mark) {
+      io = T;
+      cross_entries(W, io, h, SHARE_PEBBLE, q);
+      T.last = io.last;
+      mark = T.last >= 0 ? __ldcg(&W.share->entries[T.last].mark) : -1;
+    }
+    const bool have = near != I32MAX && h >= near - SPAN && h < near;
+    near = have ? near - SPAN : h - (SPAN - 1);
+    if (!have) {
+#pragma unroll
+      for (int j = 0; j < SPAN / 32; j++) ahead[j] = cl[max(near + 32 * j + lane, 0)].x;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < SPAN / 32; j++) sm[32 * j + lane] = ahead[j];
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < SPAN / 32; j++) ahead[j] = cl[max(near - SPAN + 32 * j + lane, 0)].x;
+    // the path's pebbles in the block, before the next entry's line
+    const int least = max(max(near, mark), 0);
+    int cnt = 0, slot = h;
+    for (int cur = h; cnt < 32 && cur >= least; cnt++) {
+      slot = lane == cnt ? cur : slot;
+      cur = sm[cur - near];
+    }
+    const bool in = lane < cnt;
+    const int4 p = cl[slot];
+    const int pb = T.bpos(p);
+    int by = __shfl_up_sync(FULL, pb, 1), bz = __shfl_up_sync(FULL, p.z, 1);
+    if (lane == 0) {
+      by = T.bpos(q);
+      bz = q.z;
+    }
+    const int vd = bz - p.z + (lane == 0 ? dd : 0), vb = T.sg * (by - pb) + (lane == 0 ? db : 0);
+    const bool ends = T.inner && T.inside(p);  // (the start: the last pebble at most)
+    if (in && !ends && T.n + lane < T.room)
+      *T.slot(W, T.n + lane) = (uint32_t)(uint16_t)vd | (uint32_t)(uint16_t)vb << 16;
+    const unsigned e = __ballot_sync(FULL, in && ends);
+    if (e) {
+      T.jd = __shfl_sync(FULL, vd, cnt - 1);
+      T.jb = __shfl_sync(FULL, vb, cnt - 1);
+    }
+    T.n += cnt - (e ? 1 : 0);
+    steps += cnt;
+    dd = db = 0;
+    q.x = __shfl_sync(FULL, p.x, cnt - 1);
+    q.y = __shfl_sync(FULL, p.y, cnt - 1);
+    q.z = __shfl_sync(FULL, p.z, cnt - 1);
+    q.w = __shfl_sync(FULL, p.w, cnt - 1);
+  }
+  T.start = q.y;
+  io = T;
+  return err ? err : (T.n > T.room ? ALN_ERR_POINTS : 0);
+}
+
+// Publishes an extension that stopped: its first n own intervals (the walk's)
+// and, filled by the caller on lane 0, the rest of its record.  Returns whether
+// the list had room.
+__device__ __forceinline__ bool publish(const WarpWork &W, const TraceWalk &T, int rec, int status) {
+  const ShareTable &X = *W.share;
+  const int lane = threadIdx.x & 31;
+  ShareRec &R = X.recs[rec];
+  unsigned long long off = 0;
+  if (lane == 0) off = atomicAdd(X.nlist, (unsigned long long)T.n);
+  off = __shfl_sync(FULL, off, 0);
+  const bool fits = (int64_t)off + T.n <= X.list_cap;
+  __syncwarp();
+  if (fits)
+    for (int64_t i = lane; i < T.n; i += 32) X.list[off + i] = *T.slot(W, i);
+  if (lane == 0) {
+    R.own = (int)T.n;
+    R.off = (int64_t)off;
+  }
+  __threadfence();
+  __syncwarp();
+  if (lane == 0) *(volatile int *)&R.status = fits ? status : SHARE_FAILED;
+  return fits;
+}
+
+// A joined extension's path past its join: the extensions on the way to the
+// tip, their parts of the trace from the tip on into the walk's buffer.
+// Returns the first pebble after the join's line (x unset) in this
+// extension's wave numbers (its wave `dif` joined entry e0), what the interval
+// from there has already (dd, db), and the tip; false if there is no room.
+// way: W.vcap places, for the entries on the way.
+__device__ __noinline__ bool gather_path(const WarpWork &W, TraceWalk &T, int *way, int e0, int dif, int4 &q, int &dd,
+                                         int &db, int &tipx, int &tipy, int &tipd) {
+  const ShareTable &X = *W.share;
+  const int lane = threadIdx.x & 31;
+  int m = 0, status = SHARE_JOINED;
+  for (int e = e0; status == SHARE_JOINED; m++) {
+    if (m >= W.vcap) return false;
+    if (lane == 0) way[m] = e;
+    const ShareRec &R = X.recs[__ldcg(&X.entries[e].rec)];
+    status = __ldcg(&R.status);
+    if (status == SHARE_FAILED) return false;
+    if (status == SHARE_DONE) {
+      tipx = __ldcg(&R.tipx);
+      tipy = __ldcg(&R.tipy);
+      tipd = __ldcg(&R.tipd);
+    } else
+      e = __ldcg(&R.entry);
+  }
+  __syncwarp();
+  dd = db = 0;
+  for (int i = m - 1; i >= 0; i--) {
+    const ShareEntry &E = X.entries[way[i]];
+    const ShareRec &R = X.recs[__ldcg(&E.rec)];  // the owner; q, tipd are in its wave numbers from here
+    if (i < m - 1) {
+      // from the pebble after the line it joined on to its head there
+      const int4 head = make_int4(0, __ldcg(&R.hdiag), __ldcg(&R.hdiff), __ldcg(&R.hmark));
+      T.put(W, dd + q.z - head.z, db + T.sg * (T.bpos(q) - T.bpos(head)));
+      dd = db = 0;
+    }
+    const int after = __ldcg(&E.after);
+    const int64_t off = __ldcg(&R.off);
+    if (T.n + after > T.room) return false;
+    for (int k = lane; k < after; k += 32) *T.slot(W, T.n + k) = __ldcg(&X.list[off + k]);
+    T.n += after;
+    q = make_int4(0, __ldcg(&E.pdiag), __ldcg(&E.pdiff), __ldcg(&E.pmark));
+    if (i == m - 1 && after == 0) T.tip(W, q, tipx, tipy, tipd, dd, db);
+    // on to the joiner's wave numbers
+    const int delta = (i > 0 ? __ldcg(&X.recs[__ldcg(&X.entries[way[i - 1]].rec)].dif) : dif) - __ldcg(&E.dif);
+    q.z += delta;
+    tipd += delta;
+  }
+  __syncwarp();
+  return T.n <= T.room;
+}
+
 // forward_wave (fwd) or reverse_wave of a path, out of line: one copy of the
 // code serves both directions and every call.  `start` is the forward wave's
 // lowest diagonal on entry and, on return, the diagonal the path starts on.
+// A scout's trace is left out (its own intervals go to the share's list).
 // BLOCKS: waves of 32 to 124 diagonals run in registers (block_waves), for
 // launches bounded by their longest calls (2 x 41 kbp: pair phase 10.8 ms
 // against 14.9 through memory); without, they too run as passes
 // (wide_waves), for launches bounded by throughput, where the smaller loop
 // and its registers pay (2 x 200 Mbp repeat-rich: 224 ms against 278).
 // Returns 1 on a work-space overflow (W.err set).
-template <bool BLOCKS>
-__device__ __noinline__ int extend(const bool fwd, WarpWork &W, const AlignSpec &spec, const Seq &A, const Seq &B,
+template <bool BLOCKS, bool SHARE>
+__device__ __noinline__ int extend(const bool fwd, const bool scout, WarpWork &W, const AlignSpec &spec, const Seq &A, const Seq &B,
                                    Path &P, int &start, int maxd, int mida, int minp, int maxp, int aoff) {
   const int lane = threadIdx.x & 31;
   const int tspace = spec.trace_space;
@@ -899,6 +1272,13 @@ __device__ __noinline__ int extend(const bool fwd, WarpWork &W, const AlignSpec 
   S.besta = S.lasta = S.trima = S.sg * mida;
   S.bestx = S.trimx = S.sg * ((mida + maxd) >> 1);
   S.trimd = S.trimha = 0;
+  Sharing sh;
+  sh.rec = sh.last = sh.joined = -1;
+  sh.guess = 0;
+  sh.from = S.besta;
+  sh.full = false;
+  // (a border would be part of the state: such calls grow alone)
+  S.line = SHARE && minp == -I32MAX && maxp == I32MAX ? next_line(S.besta) : I32MAX;
   S.more = 1;
   int64_t call_base = -1;  // this call's first pebble: the reference's cells[0]
 
@@ -966,12 +1346,30 @@ __device__ __noinline__ int extend(const bool fwd, WarpWork &W, const AlignSpec 
     if (kb != NO_WAVE) S.low = kb + 1;
   }
 
+  // an extension that fails lets those that joined it go on alone
+  auto give_up = [&]() {
+    if (SHARE && sh.rec >= 0 && lane == 0) *(volatile int *)&W.share->recs[sh.rec].status = SHARE_FAILED;
+    return 1;
+  };
+  const int64_t t0 = P.trace_off;
+  TraceWalk T;
+  T.fwd = fwd;
+  T.inner = !fwd && P.tlen != 0;
+  T.sg = S.sg;
+  T.mida = mida;
+  T.tspace = tspace;
+  T.aoff = aoff;
+  T.room = (fwd ? W.point_cap - t0 : t0) >> 1;
+  T.base = call_base;
+  const int4 *cl = reinterpret_cast<const int4 *>(cells);
+  int trimx, trimy, trimd;
   const int max_waves = A.len + B.len + 1024;
+grow:
   while (S.more && S.lasta >= S.besta - TRIM_MLAG) {
     // no wave to grow from, or more waves than bases: neither ends by itself
     if (S.hgh < S.low || S.dif > max_waves) {
       W.err |= ALN_ERR_VCAP;
-      return 1;
+      return give_up();
     }
     int stop = max_waves + 1;
     if (W.long_waves > 0 && !W.flagged) {
@@ -989,73 +1387,148 @@ __device__ __noinline__ int extend(const bool fwd, WarpWork &W, const AlignSpec 
     }
     const int width = S.hgh - S.low + 1 + (S.low > S.minp ? 1 : 0) + (S.hgh < S.maxp ? 1 : 0);
     int r;
+    if (SHARE && S.besta >= S.line && width <= NARROW) {
+      S.line = next_line(S.besta);
+      if (W.task) scout_if_free(W);
+      if (cross_line(W, S, W.pair | (fwd ? 1u << 31 : 0u), sh)) break;
+      if (sh.full) S.line = I32MAX;
+    }
     if (width <= NARROW) r = narrow_waves(W, S, stop);
     else if (BLOCKS && width <= BLOCK * NARROW) r = block_waves<BLOCK>(W, S, stop);
     else r = wide_waves(W, S, stop, BLOCKS ? BLOCK * NARROW - 8 : BLOCK_OUT);
-    if (r) return 1;
+    if (r) return give_up();
   }
   __syncwarp();
 
-  // Trace-back, from the path's tip to its start: one pebble per step, read
-  // whole.  Lane 0 writes each interval's (diffs, b-delta) to the free end of
-  // the trace buffer; the warp then moves them next to the path's start.
-  const int trimx = S.sg * S.trimx, trimy = S.sg * S.trima - trimx, trimd = S.trimd, h = S.trimha;
-  const int64_t t0 = P.trace_off;
-  const int64_t room = (fwd ? W.point_cap - t0 : t0) >> 1;  // intervals the free end holds
-  const int64_t lim = W.chunk_next - call_base + 1;
-  const int4 *cl = reinterpret_cast<const int4 *>(cells);  // ptr, diag, diff, mark
-  int64_t n = 0;
-  // forward intervals come last first, down from the buffer's top; reverse
-  // ones first first, up from its bottom
-  auto put = [&](int dd, int db) {
-    n += 1;
-    if (lane == 0 && n <= room) {
-      uint16_t *o = W.points + (fwd ? W.point_cap - 2 * n : 2 * (n - 1));
-      o[0] = (uint16_t)dd;
-      o[1] = (uint16_t)db;
+  // Trace-back, from the path's tip to its start.
+  T.lim = W.chunk_next - call_base + 1;
+  T.n = 0;
+  T.jd = T.jb = 0;
+  T.last = -1;
+  int err = 0;
+  bool joined = false;
+  if (SHARE && sh.joined >= 0) {
+    const ShareTable &X = *W.share;
+    const ShareEntry &E = X.entries[sh.joined];
+    ShareRec &R = X.recs[__ldcg(&E.rec)];
+    const bool walks = sh.rec >= 0 || (scout && fwd);
+    if (walks) {
+      // this extension's part, as it most likely is, while the owner's is on its way
+      T.last = sh.last;
+      err = walk_back<SHARE>(W, T, cl[sh.guess], 0, 0);
+      if (err) {
+        W.err |= err;
+        return give_up();
+      }
     }
-  };
-  // the interval of a reverse path that ends inside the forward path's first one
-  auto join = [&](int dd, int db) {
-    if (lane == 0) {
-      uint16_t *o = W.points + t0;
-      o[0] = (uint16_t)(o[0] + dd);
-      o[1] = (uint16_t)(o[1] + db);
+    if (scout && sh.rec < 0) {  // nothing behind it for others
+      start = T.start;
+      return 0;
     }
-  };
-  int4 q = cl[h];
-  bool first = q.x < 0;
-  int qb = fwd && first ? (mida - q.y) >> 1 : q.w - q.y;
-  int dd = trimd - q.z, db = S.sg * (trimy - qb);  // past the last mark
-  const bool inside = !fwd && first && q.w % tspace != aoff;
-  if (inside || qb + q.y != trimx) {
-    if (inside && P.tlen != 0) join(dd, db);
-    else put(dd, db);
-    dd = db = 0;
-  } else if (qb == trimy)
-    dd = db = 0;
-  else if (first && !fwd)
-    join(dd, db);
-  int steps = 0;
-  while (!first) {
-    if (q.x < call_base || ++steps > lim || n > room) {
-      W.err |= n > room ? ALN_ERR_POINTS : ALN_ERR_CELLS;
-      return 1;
+    int status = 0;
+    if (lane == 0)
+      for (int poll = 0; poll < SHARE_POLLS && (status = *(volatile int *)&R.status) == 0; poll++) __nanosleep(200);
+    status = __shfl_sync(FULL, status, 0);
+    __threadfence();
+    const int kind = __ldcg(&E.kind);
+    if (status == 0 || status == SHARE_FAILED || kind == SHARE_NONE) {
+      // go on alone (what was entered so far stays with the record, which fails)
+      give_up();
+      sh.rec = sh.last = sh.joined = -1;
+      goto grow;
     }
-    const int4 p = cl[q.x];
-    first = p.x < 0;
-    const int pb = fwd && first ? (mida - p.y) >> 1 : p.w - p.y;
-    dd += q.z - p.z;
-    db += S.sg * (qb - pb);
-    if (!fwd && first && P.tlen != 0 && p.w % tspace != aoff) join(dd, db);
-    else put(dd, db);
-    dd = db = 0;
-    q = p;
-    qb = pb;
+    const int dif = S.dif - __ldcg(&E.dif), kc = S.low + ((__ldcg(&E.lane) - S.low) & 31);
+    const int head = W.C[S.cur][kc & vmask].HA;
+    if (status == SHARE_DONE && __ldcg(&R.tipd) <= __ldcg(&E.dif)) {
+      // the owner found nothing past this wave: the tip is this extension's own
+    } else if (kind == SHARE_HEAD) {
+      // the owner's tip is before the next mark
+      S.trimx = S.sg * __ldcg(&R.tipx);
+      S.trima = S.trimx + S.sg * __ldcg(&R.tipy);
+      S.trimd = __ldcg(&R.tipd) + dif;
+      S.trimha = head;
+    } else {
+      joined = true;
+      if (walks && head != sh.guess) {
+        T.n = 0;
+        T.jd = T.jb = 0;
+        T.last = sh.last;
+        err = walk_back<SHARE>(W, T, cl[head], 0, 0);
+      }
+      bool listed = false;
+      if (sh.rec >= 0 && !err) {
+        ShareRec &O = X.recs[sh.rec];
+        if (lane == 0) {
+          const int4 q = cl[head];
+          O.entry = sh.joined;
+          O.dif = S.dif;
+          O.hdiag = q.y;
+          O.hdiff = q.z;
+          O.hmark = q.w;
+        }
+        listed = publish(W, T, sh.rec, SHARE_JOINED);
+      }
+      if (!scout && !err) {
+        // the parts past the join, then this extension's own
+        const int64_t own = T.n;
+        int4 q;
+        int dd, db;
+        T.n = 0;
+        if (!gather_path(W, T, W.V[S.cur ^ 1], sh.joined, S.dif, q, dd, db, trimx, trimy, trimd)) {
+          sh.rec = sh.last = sh.joined = -1;  // (its record stands)
+          goto grow;
+        }
+        q.x = head;
+        T.last = -1;
+        if (listed) {
+          const int4 p = cl[head];
+          T.put(W, dd + q.z - p.z, db + T.sg * (T.bpos(q) - T.bpos(p)));
+          const int64_t off = __ldcg(&X.recs[sh.rec].off);
+          if (T.n + own > T.room) err = ALN_ERR_POINTS;
+          else
+            for (int64_t i = lane; i < own; i += 32) *T.slot(W, T.n + i) = __ldcg(&X.list[off + i]);
+          T.n += own;
+        } else
+          err = walk_back<SHARE>(W, T, q, dd, db);
+      }
+    }
   }
-  if (n > room) {
-    W.err |= ALN_ERR_POINTS;
-    return 1;
+  if (!joined) {
+    T.n = 0;
+    T.jd = T.jb = 0;
+    T.last = SHARE ? sh.last : -1;
+    trimx = S.sg * S.trimx;
+    trimy = S.sg * S.trima - trimx;
+    trimd = S.trimd;
+    const int4 q = cl[S.trimha];
+    if (SHARE && T.last >= 0) cross_entries(W, T, S.trimha, SHARE_HEAD, q);
+    int dd, db;
+    T.tip(W, q, trimx, trimy, trimd, dd, db);
+    err = walk_back<SHARE>(W, T, q, dd, db);
+    if (SHARE && sh.rec >= 0 && !err) {
+      if (lane == 0) {
+        ShareRec &O = W.share->recs[sh.rec];
+        O.tipx = trimx;
+        O.tipy = trimy;
+        O.tipd = trimd;
+      }
+      publish(W, T, sh.rec, SHARE_DONE);
+    }
+  }
+  if (err) {
+    W.err |= err;
+    return joined ? 1 : give_up();
+  }
+  __syncwarp();
+  const int64_t n = T.n;
+  if (scout) {
+    start = T.start;
+    return 0;
+  }
+  if ((T.jd | T.jb) && lane == 0) {
+    uint16_t *o = W.points + t0;
+    o[0] = (uint16_t)(o[0] + T.jd);
+    o[1] = (uint16_t)(o[1] + T.jb);
   }
   __syncwarp();
   {
@@ -1072,7 +1545,7 @@ __device__ __noinline__ int extend(const bool fwd, WarpWork &W, const AlignSpec 
     }
   }
   if (fwd) {
-    start = q.y;
+    start = T.start;
     P.aepos = trimx;
     P.bepos = trimy;
     P.diffs = trimd;
@@ -1120,7 +1593,7 @@ __device__ __forceinline__ void path_to_forward(uint16_t *trace, const Seq &A, c
 // start, a reverse re-run counts its differences afresh).  With `acomp` A is
 // the complemented contig and the path comes back in forward coordinates.
 // Returns 1 on a work-space overflow (W.err says which).
-template <bool BLOCKS>
+template <bool BLOCKS, bool SHARE>
 __device__ __forceinline__ int local_alignment_w(WarpWork &W, const AlignSpec &spec, const Seq &A, const Seq &B,
                                                  bool acomp, Path &P, int low, int hgh, int anti, int lbord,
                                                  int hbord) {
@@ -1136,9 +1609,9 @@ __device__ __forceinline__ int local_alignment_w(WarpWork &W, const AlignSpec &s
   const int aoff = acomp ? A.len % spec.trace_space : 0;
 
   int from = low;
-  if (extend<BLOCKS>(true, W, spec, A, B, P, from, hgh, anti, minp, maxp, aoff)) return 1;
+  if (extend<BLOCKS, SHARE>(true, false, W, spec, A, B, P, from, hgh, anti, minp, maxp, aoff)) return 1;
   const bool fwd_away = (P.aepos + P.bepos) - anti >= DUB_TRIM;
-  if (extend<BLOCKS>(false, W, spec, A, B, P, from, from, anti, minp, maxp, aoff)) return 1;
+  if (extend<BLOCKS, SHARE>(false, false, W, spec, A, B, P, from, from, anti, minp, maxp, aoff)) return 1;
   const bool rev_away = anti - (P.abpos + P.bbpos) >= DUB_TRIM;
 
   if (!fwd_away && !rev_away) {
@@ -1148,16 +1621,32 @@ __device__ __forceinline__ int local_alignment_w(WarpWork &W, const AlignSpec &s
   } else if (!fwd_away) {
     from = P.abpos - P.bbpos;
     P.tlen = 0;
-    if (extend<BLOCKS>(true, W, spec, A, B, P, from, from, P.abpos + P.bbpos, minp, maxp, aoff)) return 1;
+    if (extend<BLOCKS, SHARE>(true, false, W, spec, A, B, P, from, from, P.abpos + P.bbpos, minp, maxp, aoff)) return 1;
   } else if (!rev_away) {
     from = P.aepos - P.bepos;
     const int at = P.aepos + P.bepos;
     P.tlen = 0;
     P.diffs = 0;
-    if (extend<BLOCKS>(false, W, spec, A, B, P, from, from, at, minp, maxp, aoff)) return 1;
+    if (extend<BLOCKS, SHARE>(false, false, W, spec, A, B, P, from, from, at, minp, maxp, aoff)) return 1;
   }
   if (acomp) path_to_forward(W.points + P.trace_off, A, B, P);
   return 0;
+}
+
+// A scout: a call's two extensions for those that join them.  What it cannot
+// do (a full pool) its joiners do themselves.
+__device__ __forceinline__ void scout_w(WarpWork &W, const AlignSpec &spec, const Seq &A, const Seq &B, bool acomp,
+                                        int low, int hgh, int anti) {
+  Path P;
+  P.tlen = P.diffs = P.abpos = P.bbpos = P.aepos = P.bepos = 0;
+  P.trace_off = 2 * (A.len / spec.trace_space + 2);
+  if (2 * (int64_t)P.trace_off > W.point_cap) return;
+  while (((anti - hgh) >> 1) < 0) hgh -= 1;
+  const int aoff = acomp ? A.len % spec.trace_space : 0;
+  int from = low;
+  if (hgh < low || extend<true, true>(true, true, W, spec, A, B, P, from, hgh, anti, -I32MAX, I32MAX, aoff)) return;
+  P.tlen = 0;
+  extend<true, true>(false, true, W, spec, A, B, P, from, from, anti, -I32MAX, I32MAX, aoff);
 }
 
 }  // namespace aln

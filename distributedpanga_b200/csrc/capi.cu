@@ -116,6 +116,7 @@ struct pga_ctx {
   int64_t cap_calls = 0, cap_bytes = 0;
   // the scoring tables of the last alignment
   int ave_path_host = 0, dscore_host = 0;
+  aln::ShareTable share_host;  // of the last alignment's shared extensions
   int diag_passes[2] = {0, 0};
   SeedKeyLayout lay[2];
   bool have_diag[2] = {false, false};
@@ -128,7 +129,7 @@ struct pga_ctx {
   DBuf pk, poff, pwords;
   DBuf numf, numr, soff, tasks, task_next, pout, wave, points, cells, cell_next, ovl, perm, cand,
       cand_next, recs, rec_next, outb, out_next, pflag, pidx, pstart, pab, rng_ovl, rng_next, ftasks, fout,
-      rout, selfb, pstart2, pab2, small, shist, fo_dev, binfo[2], plive[2];
+      rout, share_tab, share_ent, share_list, selfb, pstart2, pab2, small, shist, fo_dev, binfo[2], plive[2];
   // survivors in la_sort order on the device (srecs, their traces in strace,
   // toff rewritten to offsets there), and their host copy, made when read
   DBuf srecs, slen, strace, skeys, skeys2, lhist, lscan;
@@ -245,7 +246,8 @@ bool shed_align_buffers(pga_ctx *ctx) {
   DBuf *bufs[] = {&ctx->numf, &ctx->numr, &ctx->pk, &ctx->wave, &ctx->points, &ctx->cells, &ctx->ovl, &ctx->perm,
                   &ctx->cand, &ctx->recs, &ctx->outb, &ctx->rng_ovl, &ctx->tasks, &ctx->pout, &ctx->pflag,
                   &ctx->pidx, &ctx->pstart, &ctx->pab, &ctx->pstart2, &ctx->pab2, &ctx->small, &ctx->ftasks,
-                  &ctx->fout, &ctx->rout, &ctx->lreq, &ctx->lpath, &ctx->ltoff, &ctx->ltrace,
+                  &ctx->fout, &ctx->rout, &ctx->share_tab, &ctx->share_ent, &ctx->share_list, &ctx->lreq, &ctx->lpath,
+                  &ctx->ltoff, &ctx->ltrace,
                   &ctx->binfo[0], &ctx->binfo[1], &ctx->plive[0], &ctx->plive[1], &ctx->skeys, &ctx->skeys2,
                   &ctx->lhist, &ctx->lscan, &ctx->memo_hits, &ctx->mlog_key, &ctx->mlog_val, &ctx->mlog_toff,
                   &ctx->mlog_trace, &ctx->mlog_ctr};
@@ -754,6 +756,83 @@ struct LaunchPlan {
   std::vector<FinishTask> fins;
 };
 
+// The launch's table of shared extensions (align_share.cuh), and its pools:
+// an entry per 2,048 bases (a path makes one per 16,384 in each direction and
+// strand), 512 intervals and a scout per entry, tables twice that; where a pool
+// is full, calls grow alone, and without the memory for them all do.
+//
+// A launch shares its extensions if its contigs are several lines long and
+// most of its tasks are parts of pairs: what is shared is the path that many
+// band blocks of one pair lead to.  Pair phase shared and alone, longest
+// contig, parts and whole pairs: 2 x 2 Mbp in one-copy contigs 4.0 and 17.2 ms
+// (493 kbp, 9,348 and 6); 2 x 23 Mbp 24 and 31 (13.2 Mbp, 187,177 and 116);
+// 2 x 100 Mbp 84 and 129 (19.1 Mbp, 478,652 and 177); but 17 x 2.5 Mbp 14.6 and
+// 12.4 (250 kbp, 684 and 58,910), 2 x 20 Mbp repeat-rich 60 and 57 (10 kbp,
+// 98,578 and 90,791): the larger loop costs, and whole pairs repeat no path.
+constexpr int64_t SHARE_CONTIG = 4 * aln::SHARE_LINE;
+
+void prepare_share(pga_ctx *ctx, AlignLaunch &L, int64_t nt) {
+  L.share = nullptr;
+  if (L.min_blocks != 2 || ctx->maxctg < SHARE_CONTIG || nt < L.nsmall) return;
+  int64_t seqtot = 0;
+  for (int c = 0; c < ctx->ncontig; c++) seqtot += ctx->clen[c];
+  int lg = 12;
+  while (lg < 19 && ((int64_t)1 << lg) * 2048 < seqtot) lg++;
+  const size_t ne = (size_t)1 << lg;
+  // the table itself, its counters at 192, then its arrays
+  size_t end = 256;
+  auto room = [&](size_t bytes) {
+    const size_t at = end;
+    end += (bytes + 15) & ~(size_t)15;
+    return at;
+  };
+  const size_t keys = room(sizeof(unsigned long long) * 2 * ne), vals = room(sizeof(int) * 2 * ne),
+               recs = room(sizeof(aln::ShareRec) * ne), scouts = room(sizeof(aln::Scout) * ne),
+               ckeys = room(sizeof(unsigned long long) * 2 * ne), cvals = room(sizeof(int) * 2 * ne);
+  // (only out of plenty: the pools that grow in a rerun come first)
+  const size_t need = end + (sizeof(aln::ShareEntry) + sizeof(uint32_t) * 512) * ne;
+  size_t free_b = 0, total_b = 0;
+  const bool have = ctx->share_tab.cap >= end && ctx->share_ent.cap >= sizeof(aln::ShareEntry) * ne &&
+                    ctx->share_list.cap >= sizeof(uint32_t) * 512 * ne;
+  if (!have && (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess ||
+      free_b + ctx->arena.free_bytes() + ctx->share_tab.cap + ctx->share_ent.cap + ctx->share_list.cap < 4 * need)) {
+    cudaGetLastError();
+    return;
+  }
+  char err[sizeof(ctx->err)];
+  memcpy(err, ctx->err, sizeof(err));
+  if (ensure(ctx, ctx->share_tab, end) != PGA_OK || ensure(ctx, ctx->share_ent, sizeof(aln::ShareEntry) * ne) != PGA_OK ||
+      ensure(ctx, ctx->share_list, sizeof(uint32_t) * 512 * ne) != PGA_OK) {
+    cudaGetLastError();
+    memcpy(ctx->err, err, sizeof(err));
+    return;
+  }
+  uint8_t *base = P<uint8_t>(ctx->share_tab);
+  aln::ShareTable X{};
+  unsigned *counters = (unsigned *)(base + 192);
+  X.nentry = counters;
+  X.nrec = counters + 1;
+  X.nlist = (unsigned long long *)(counters + 2);
+  X.qhead = counters + 4;
+  X.qtail = counters + 5;
+  X.ended = counters + 6;
+  X.next_task = P<unsigned>(ctx->task_next);
+  X.keys = (unsigned long long *)(base + keys);
+  X.vals = (int *)(base + vals);
+  X.recs = (aln::ShareRec *)(base + recs);
+  X.scouts = (aln::Scout *)(base + scouts);
+  X.ckeys = (unsigned long long *)(base + ckeys);
+  X.cvals = (int *)(base + cvals);
+  X.mask = X.cmask = (unsigned)(2 * ne - 1);
+  X.entries = P<aln::ShareEntry>(ctx->share_ent);
+  X.list = P<uint32_t>(ctx->share_list);
+  X.entry_cap = X.rec_cap = X.qcap = (int)ne;
+  X.list_cap = (int64_t)(512 * ne);
+  static_assert(sizeof(aln::ShareTable) <= 192, "the counters follow the table");
+  ctx->share_host = X;
+  L.share = (const aln::ShareTable *)base;
+}
+
 // Runs a plan: the warps take the tasks in plan order.  tout: one PairOut per
 // whole pair (at its place in the plan), fout: one per finish task; *cycles
 // grows by the launch's task cycles.  Pebbles live for one launch; candidate
@@ -777,6 +856,7 @@ int align_launch(pga_ctx *ctx, AlignLaunch &L, const LaunchPlan &plan, std::vect
   if (nt + L.nsmall >= (int64_t)0x7fffffff)
     return fail(ctx, PGA_ERR_LIMIT, "%lld alignment tasks: at most 2^31 supported", (long long)(nt + L.nsmall));
   if (nt == 0 && nf == 0 && L.nsmall == 0) return PGA_OK;
+  prepare_share(ctx, L, nt);
   if (nt) {
     ENSURE(ctx->tasks, sizeof(PairTask) * ni + sizeof(unsigned) * (ni + 1));
     ENSURE(ctx->pout, sizeof(PairOut) * ni);
@@ -809,6 +889,18 @@ int align_launch(pga_ctx *ctx, AlignLaunch &L, const LaunchPlan &plan, std::vect
     // idle warps that still have queue work
     L.long_waves = ctx->long_waves >= 0 ? ctx->long_waves : (L.min_blocks >= 3 ? 0 : LONG_WAVES_AUTO);
     CK(cudaMemsetAsync(ctx->cell_next.p, 0, 8, ctx->st));
+    if (L.share) {
+      // the shared extensions: no entry, no record (their pebbles go with the launch)
+      aln::ShareTable &X = ctx->share_host;
+      X.ntasks = (unsigned)(nt + L.nsmall);
+      CK(cudaMemcpyAsync(ctx->share_tab.p, &X, sizeof(X), cudaMemcpyHostToDevice, ctx->st));
+      CK(cudaMemsetAsync(X.keys, 0, sizeof(unsigned long long) * ((size_t)X.mask + 1), ctx->st));
+      CK(cudaMemsetAsync(X.vals, 0xff, sizeof(int) * ((size_t)X.mask + 1), ctx->st));
+      CK(cudaMemsetAsync(X.nentry, 0, 64, ctx->st));
+      CK(cudaMemsetAsync(X.scouts, 0, sizeof(aln::Scout) * (size_t)X.qcap, ctx->st));
+      CK(cudaMemsetAsync(X.ckeys, 0, sizeof(unsigned long long) * ((size_t)X.cmask + 1), ctx->st));
+      CK(cudaMemsetAsync(X.cvals, 0xff, sizeof(int) * ((size_t)X.cmask + 1), ctx->st));
+    }
     CK(cudaMemcpyAsync(ctx->cand_next.p, &ctx->counters[0], 8, cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(ctx->rng_next.p, &ctx->counters[1], 8, cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(ctx->rec_next.p, &ctx->counters[2], 8, cudaMemcpyHostToDevice, ctx->st));
@@ -1727,7 +1819,7 @@ void pga_ctx_destroy(pga_ctx *ctx) {
                    &ctx->wave, &ctx->points, &ctx->cells, &ctx->cell_next, &ctx->ovl, &ctx->perm, &ctx->cand,
                    &ctx->cand_next, &ctx->recs, &ctx->rec_next, &ctx->outb, &ctx->out_next, &ctx->pflag,
                    &ctx->pidx, &ctx->pstart, &ctx->pab, &ctx->rng_ovl, &ctx->rng_next, &ctx->ftasks,
-                   &ctx->fout, &ctx->rout, &ctx->selfb, &ctx->lreq, &ctx->lpath, &ctx->ltoff,
+                   &ctx->fout, &ctx->rout, &ctx->share_tab, &ctx->share_ent, &ctx->share_list, &ctx->selfb, &ctx->lreq, &ctx->lpath, &ctx->ltoff,
                    &ctx->ltrace, &ctx->lnext, &ctx->pstart2, &ctx->pab2, &ctx->small, &ctx->shist, &ctx->fo_dev,
                    &ctx->srecs, &ctx->slen, &ctx->strace, &ctx->skeys, &ctx->skeys2, &ctx->lhist, &ctx->lscan,
                    &ctx->memo_hits, &ctx->mlog_key, &ctx->mlog_val, &ctx->mlog_toff, &ctx->mlog_trace,
