@@ -14,6 +14,7 @@
 #include "index.cuh"
 #include "merge.cuh"
 #include "diag_sort.cuh"
+#include "hostcopy.h"
 #include "radix.cuh"
 #include "scan.cuh"
 #include "seeds.cuh"
@@ -116,6 +117,8 @@ struct pga_ctx {
   int64_t cap_calls = 0, cap_bytes = 0;
   // the scoring tables of the last alignment
   int ave_path_host = 0, dscore_host = 0;
+  HostCopier copier;
+  bool trace_valid = false;        // h_trace holds the last alignment's traces
   aln::ShareTable share_host;  // of the last alignment's shared extensions
   int diag_passes[2] = {0, 0};
   SeedKeyLayout lay[2];
@@ -313,6 +316,14 @@ int grow_keep(pga_ctx *ctx, DBuf &b, size_t bytes, size_t keep) {
   return PGA_OK;
 }
 
+// Copies between a caller's memory and the device, in stream order (hostcopy.h).
+cudaError_t copy_out(pga_ctx *ctx, void *host, const void *dev, size_t bytes) {
+  return ctx->copier.copy(ctx->device, const_cast<void *>(dev), host, bytes, true, ctx->st);
+}
+cudaError_t copy_in(pga_ctx *ctx, void *dev, const void *host, size_t bytes) {
+  return ctx->copier.copy(ctx->device, dev, const_cast<void *>(host), bytes, false, ctx->st);
+}
+
 #define ENSURE(b, bytes)                      \
   do {                                        \
     int _r = ensure(ctx, (b), (bytes));       \
@@ -495,7 +506,7 @@ int index_from_host(pga_ctx *ctx, const uint8_t *records, int64_t count, int pos
   ENSURE(ctx->hist, sizeof(uint32_t) * (NPREFIX + 1));
   ENSURE(ctx->start, sizeof(uint32_t) * (NPREFIX + 1));
   if (count > 0) {
-    CK(cudaMemcpyAsync(ctx->io.p, records, (size_t)count * rs, cudaMemcpyHostToDevice, ctx->st));
+    CK(copy_in(ctx, ctx->io.p, records, (size_t)count * rs));
     k_records_in<<<grid_for(count, 256), 256, 0, ctx->st>>>(P<uint8_t>(ctx->io), count, posb, ctgb, P<Rec>(ctx->rec2), nullptr);
     LAUNCHED(1);
   }
@@ -661,7 +672,7 @@ int copy_diag(pga_ctx *ctx, int comp, int ncontig, uint8_t *out, int64_t *panel_
                                                                  P<int64_t>(ctx->panel[comp]));
   LAUNCHED(1);
   CK(cudaGetLastError());
-  if (out && n > 0) CK(cudaMemcpyAsync(out, ctx->io.p, (size_t)n * sw, cudaMemcpyDeviceToHost, ctx->st));
+  if (out && n > 0) CK(copy_out(ctx, out, ctx->io.p, (size_t)n * sw));
   if (panel_off)
     CK(cudaMemcpyAsync(panel_off, ctx->panel[comp].p, sizeof(int64_t) * (ncontig + 1), cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
@@ -677,7 +688,7 @@ int copy_seeds(pga_ctx *ctx, int comp, uint8_t *out, int64_t *buck) {
       k_seeds_out<<<grid_for(n, 256), 256, 0, ctx->st>>>(P<Seed>(ctx->seed[comp]), n, ctx->posb, ctx->ctgb,
                                                          P<uint8_t>(ctx->io));
       LAUNCHED(1);
-      CK(cudaMemcpyAsync(out, ctx->io.p, (size_t)n * sb, cudaMemcpyDeviceToHost, ctx->st));
+      CK(copy_out(ctx, out, ctx->io.p, (size_t)n * sb));
     }
   }
   if (buck) {
@@ -1228,27 +1239,36 @@ int la_sort_device(pga_ctx *ctx, int64_t n, int64_t nbytes) {
   return PGA_OK;
 }
 
-// The host copy of the last alignment's results (made on first read).
-int host_alignments(pga_ctx *ctx) {
+// The host copy of the last alignment's records (made on first read).
+int host_records(pga_ctx *ctx) {
   if (ctx->host_valid) return PGA_OK;
   const int64_t n = ctx->nalign;
   ctx->h_recs.resize(n);
   ctx->h_toff.assign(n + 1, 0);
   ctx->h_trace.clear();
   if (n > 0) {
-    CK(cudaMemcpyAsync(ctx->h_recs.data(), ctx->srecs.p, sizeof(AlnRec) * n, cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_out(ctx, ctx->h_recs.data(), ctx->srecs.p, sizeof(AlnRec) * n));
     CK(cudaStreamSynchronize(ctx->st));
     // the survivors' traces lie back to back from offset 0
     const int64_t total = ctx->h_recs[n - 1].toff + ctx->h_recs[n - 1].tlen;
     if (total < 0 || total > ctx->ntrace) return fail(ctx, PGA_ERR_CUDA, "alignment traces out of range");
-    ctx->h_trace.resize(total);
-    if (total > 0)
-      CK(cudaMemcpyAsync(ctx->h_trace.data(), ctx->strace.p, total, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
     for (int64_t i = 0; i < n; i++) ctx->h_toff[i] = ctx->h_recs[i].toff;
     ctx->h_toff[n] = total;
   }
   ctx->host_valid = true;
+  ctx->trace_valid = false;
+  return PGA_OK;
+}
+
+// The host copy of its records and traces.
+int host_alignments(pga_ctx *ctx) {
+  const int r = host_records(ctx);
+  if (r || ctx->trace_valid) return r;
+  const int64_t total = ctx->h_toff.back();
+  ctx->h_trace.resize(total);
+  if (total > 0) CK(copy_out(ctx, ctx->h_trace.data(), ctx->strace.p, total));
+  CK(cudaStreamSynchronize(ctx->st));
+  ctx->trace_valid = true;
   return PGA_OK;
 }
 
@@ -1815,6 +1835,7 @@ void pga_ctx_destroy(pga_ctx *ctx) {
   if (!ctx) return;
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->st);
+  ctx->copier.release();
   DBuf *abufs[] = {&ctx->pk, &ctx->poff, &ctx->pwords, &ctx->numf, &ctx->numr, &ctx->soff, &ctx->tasks, &ctx->task_next, &ctx->pout, &ctx->binfo[0], &ctx->binfo[1], &ctx->plive[0], &ctx->plive[1],
                    &ctx->wave, &ctx->points, &ctx->cells, &ctx->cell_next, &ctx->ovl, &ctx->perm, &ctx->cand,
                    &ctx->cand_next, &ctx->recs, &ctx->rec_next, &ctx->outb, &ctx->out_next, &ctx->pflag,
@@ -1961,7 +1982,7 @@ int pga_gdb_load(pga_ctx *ctx, const uint8_t *bps, int64_t bps_bytes, int nconti
   ENSURE(ctx->bps, (size_t)bps_bytes + 16);
   ENSURE(ctx->dclen, sizeof(int64_t) * (ncontig + 1));
   ENSURE(ctx->dboff, sizeof(int64_t) * (ncontig + 1));
-  if (bps_bytes > 0) CK(cudaMemcpyAsync(ctx->bps.p, bps, bps_bytes, cudaMemcpyHostToDevice, ctx->st));
+  if (bps_bytes > 0) CK(copy_in(ctx, ctx->bps.p, bps, bps_bytes));
   if (ncontig > 0) {
     CK(cudaMemcpyAsync(ctx->dclen.p, clen, sizeof(int64_t) * ncontig, cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(ctx->dboff.p, boff, sizeof(int64_t) * ncontig, cudaMemcpyHostToDevice, ctx->st));
@@ -2159,7 +2180,7 @@ int pga_gdb_ingest_fasta(pga_ctx *ctx, const char *text, int64_t nbytes, int nth
     if (!e) CK(cudaEventCreate(&e));
   ENSURE(ctx->fa_text, (size_t)nbytes + 64);
   CK(cudaEventRecord(ctx->fa_ev[0], ctx->st));
-  CK(cudaMemcpyAsync(ctx->fa_text.p, text, nbytes, cudaMemcpyHostToDevice, ctx->st));
+  CK(copy_in(ctx, ctx->fa_text.p, text, nbytes));
   CK(cudaMemsetAsync(P<uint8_t>(ctx->fa_text) + nbytes, 0, 64, ctx->st));
   CK(cudaEventRecord(ctx->fa_ev[1], ctx->st));
   int r = ingest_device(ctx, nbytes, nthr, sizes6);
@@ -2184,7 +2205,7 @@ int pga_gdb_copy(pga_ctx *ctx, uint8_t *bps, int64_t *contigs4, int64_t *scaffol
   if (!ctx || !ctx->have_scaffolds) return PGA_ERR_ARG;
   CK(cudaSetDevice(ctx->device));
   if (bps && ctx->bps_bytes > 0) {
-    CK(cudaMemcpyAsync(bps, ctx->bps.p, ctx->bps_bytes, cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_out(ctx, bps, ctx->bps.p, ctx->bps_bytes));
     CK(cudaStreamSynchronize(ctx->st));
   }
   if (contigs4)
@@ -2299,7 +2320,7 @@ int pga_extract_to_records(pga_ctx *ctx, int num_workers, int worker_id, uint8_t
     k_records_out<<<grid_for(total_rec, 256), 256, 0, ctx->st>>>(P<Rec>(ctx->rec2), nullptr, total_rec, ctx->posb,
                                                                   ctx->ctgb, P<uint8_t>(ctx->io));
     LAUNCHED(1);
-    cudaError_t e = cudaMemcpyAsync(h, ctx->io.p, bytes, cudaMemcpyDeviceToHost, ctx->st);
+    cudaError_t e = copy_out(ctx, h, ctx->io.p, bytes);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->st);
     if (e != cudaSuccess) {
       free(h);
@@ -2325,7 +2346,7 @@ int pga_sort_records(pga_ctx *ctx, uint8_t *records, int64_t count, int posb, in
                                                               ctgb, P<uint8_t>(ctx->io));
     LAUNCHED(2);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(records, ctx->io.p, (size_t)count * rs, cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_out(ctx, records, ctx->io.p, (size_t)count * rs));
   }
   CK(cudaStreamSynchronize(ctx->st));
   ctx->have_index = false;
@@ -2343,7 +2364,7 @@ int pga_recalc_lcps(pga_ctx *ctx, uint8_t *records, int64_t count, int posb, int
   ENSURE(ctx->io, (size_t)count * rs + 16);
   ENSURE(ctx->rec, sizeof(Rec) * (size_t)count + 16);
   ENSURE(ctx->lcp, (size_t)count + 16);
-  CK(cudaMemcpyAsync(ctx->io.p, records, (size_t)count * rs, cudaMemcpyHostToDevice, ctx->st));
+  CK(copy_in(ctx, ctx->io.p, records, (size_t)count * rs));
   k_records_in<<<grid_for(count, 256), 256, 0, ctx->st>>>(P<uint8_t>(ctx->io), count, posb, ctgb, P<Rec>(ctx->rec),
                                                            P<uint8_t>(ctx->lcp));
   k_lcp<<<grid_for(count, 256), 256, 0, ctx->st>>>(P<Rec>(ctx->rec), count, P<uint8_t>(ctx->lcp));
@@ -2351,7 +2372,7 @@ int pga_recalc_lcps(pga_ctx *ctx, uint8_t *records, int64_t count, int posb, int
                                                             P<uint8_t>(ctx->io));
   LAUNCHED(3);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(records, ctx->io.p, (size_t)count * rs, cudaMemcpyDeviceToHost, ctx->st));
+  CK(copy_out(ctx, records, ctx->io.p, (size_t)count * rs));
   CK(cudaStreamSynchronize(ctx->st));
   ctx->have_index = false;
   return PGA_OK;
@@ -2377,7 +2398,7 @@ int pga_build_kmer_adapter(pga_ctx *ctx, const uint8_t *records, int64_t count, 
   // The records are already sorted: their prefixes' histogram scan gives the table.
   CK(cudaMemsetAsync(ctx->hist.p, 0, sizeof(uint32_t) * NPREFIX, ctx->st));
   if (count > 0) {
-    CK(cudaMemcpyAsync(ctx->io.p, records, (size_t)count * rs, cudaMemcpyHostToDevice, ctx->st));
+    CK(copy_in(ctx, ctx->io.p, records, (size_t)count * rs));
     k_records_in<<<grid_for(count, 256), 256, 0, ctx->st>>>(P<uint8_t>(ctx->io), count, posb, ctgb, P<Rec>(ctx->rec), P<uint8_t>(ctx->lcp));
     k_prefix_hist<<<grid_for(count, 256), 256, 0, ctx->st>>>(P<Rec>(ctx->rec), count, P<uint32_t>(ctx->hist));
     LAUNCHED(2);
@@ -2400,8 +2421,8 @@ int pga_build_kmer_adapter(pga_ctx *ctx, const uint8_t *records, int64_t count, 
                                                      P<uint32_t>(ctx->maxrun));
   LAUNCHED(1);
   CK(cudaGetLastError());
-  if (count > 0) CK(cudaMemcpyAsync(entries, ctx->ent.p, (size_t)count * eb, cudaMemcpyDeviceToHost, ctx->st));
-  CK(cudaMemcpyAsync(cum, ctx->cum.p, sizeof(int64_t) * NPREFIX, cudaMemcpyDeviceToHost, ctx->st));
+  if (count > 0) CK(copy_out(ctx, entries, ctx->ent.p, (size_t)count * eb));
+  CK(copy_out(ctx, cum, ctx->cum.p, sizeof(int64_t) * NPREFIX));
   uint32_t mr = 0;
   CK(cudaMemcpyAsync(&mr, ctx->maxrun.p, 4, cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
@@ -2428,8 +2449,8 @@ int pga_self_adaptamer_merge(pga_ctx *ctx, const uint8_t *entries, const int64_t
   ENSURE(ctx->cum, sizeof(int64_t) * NPREFIX);
   ENSURE(ctx->rec, sizeof(Rec) * (size_t)count + 16);
   ENSURE(ctx->lcp, (size_t)count + 16);
-  if (count > 0) CK(cudaMemcpyAsync(ctx->io.p, entries, (size_t)count * eb, cudaMemcpyHostToDevice, ctx->st));
-  CK(cudaMemcpyAsync(ctx->cum.p, cum, sizeof(int64_t) * NPREFIX, cudaMemcpyHostToDevice, ctx->st));
+  if (count > 0) CK(copy_in(ctx, ctx->io.p, entries, (size_t)count * eb));
+  CK(copy_in(ctx, ctx->cum.p, cum, sizeof(int64_t) * NPREFIX));
   k_entries_in<<<NPREFIX / 256, 256, 0, ctx->st>>>(P<uint8_t>(ctx->io), P<int64_t>(ctx->cum), count, posb, ctgb,
                                                    P<Rec>(ctx->rec), P<uint8_t>(ctx->lcp));
   LAUNCHED(1);
@@ -2483,7 +2504,7 @@ int pga_reimport_sort(pga_ctx *ctx, const uint8_t *seeds, int64_t len, int posb,
   ENSURE(ctx->io, (size_t)len + 16);
   ENSURE(ctx->seed[comp], sizeof(Seed) * (size_t)n + 16);
   if (n > 0) {
-    CK(cudaMemcpyAsync(ctx->io.p, seeds, (size_t)n * sb, cudaMemcpyHostToDevice, ctx->st));
+    CK(copy_in(ctx, ctx->io.p, seeds, (size_t)n * sb));
     k_seeds_in<<<grid_for(n, 256), 256, 0, ctx->st>>>(P<uint8_t>(ctx->io), n, posb, ctgb, P<Seed>(ctx->seed[comp]));
     LAUNCHED(1);
   }
@@ -2925,7 +2946,7 @@ int pga_index_copy_records(pga_ctx *ctx, uint8_t *records) {
                                                          ctx->ctgb, P<uint8_t>(ctx->io));
     LAUNCHED(1);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(records, ctx->io.p, (size_t)n * ctx->rsize, cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_out(ctx, records, ctx->io.p, (size_t)n * ctx->rsize));
   }
   CK(cudaStreamSynchronize(ctx->st));
   return PGA_OK;
@@ -2935,8 +2956,8 @@ int pga_index_copy_entries(pga_ctx *ctx, uint8_t *entries, int64_t *cum, int64_t
   if (!ctx || !ctx->have_index || !ctx->have_entries) return PGA_ERR_ARG;
   int eb = 9 + ctx->posb + ctx->ctgb;
   if (entries && ctx->nrec > 0)
-    CK(cudaMemcpyAsync(entries, ctx->ent.p, (size_t)ctx->nrec * eb, cudaMemcpyDeviceToHost, ctx->st));
-  if (cum) CK(cudaMemcpyAsync(cum, ctx->cum.p, sizeof(int64_t) * NPREFIX, cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_out(ctx, entries, ctx->ent.p, (size_t)ctx->nrec * eb));
+  if (cum) CK(copy_out(ctx, cum, ctx->cum.p, sizeof(int64_t) * NPREFIX));
   CK(cudaStreamSynchronize(ctx->st));
   if (largest) *largest = ctx->largest;
   return PGA_OK;
@@ -2980,7 +3001,7 @@ int pga_seeds_load(pga_ctx *ctx, int comp, const uint8_t *seeds, int64_t len) {
   ENSURE(ctx->io, (size_t)len + 16);
   ENSURE(ctx->seed[comp], sizeof(Seed) * (size_t)n + 16);
   if (n > 0) {
-    CK(cudaMemcpyAsync(ctx->io.p, seeds, (size_t)len, cudaMemcpyHostToDevice, ctx->st));
+    CK(copy_in(ctx, ctx->io.p, seeds, (size_t)len));
     k_seeds_in<<<grid_for(n, 256), 256, 0, ctx->st>>>(P<uint8_t>(ctx->io), n, ctx->posb, ctx->ctgb,
                                                        P<Seed>(ctx->seed[comp]));
     LAUNCHED(1);
@@ -3047,7 +3068,7 @@ int pga_align(pga_ctx *ctx, int64_t *nalign) {
 int pga_align_copy(pga_ctx *ctx, int32_t *recs9, int64_t *trace_off, uint8_t *trace) {
   if (!ctx || !ctx->have_align) return PGA_ERR_ARG;
   CK(cudaSetDevice(ctx->device));
-  int r = host_alignments(ctx);
+  int r = host_records(ctx);
   if (r) return r;
   int64_t n = (int64_t)ctx->h_recs.size();
   for (int64_t i = 0; i < n; i++) {
@@ -3059,7 +3080,12 @@ int pga_align_copy(pga_ctx *ctx, int32_t *recs9, int64_t *trace_off, uint8_t *tr
     }
   }
   if (trace_off) memcpy(trace_off, ctx->h_toff.data(), sizeof(int64_t) * (n + 1));
-  if (trace && !ctx->h_trace.empty()) memcpy(trace, ctx->h_trace.data(), ctx->h_trace.size());
+  if (trace && ctx->trace_valid) {
+    if (!ctx->h_trace.empty()) memcpy(trace, ctx->h_trace.data(), ctx->h_trace.size());
+  } else if (trace && ctx->h_toff[n] > 0) {
+    CK(copy_out(ctx, trace, ctx->strace.p, ctx->h_toff[n]));
+    CK(cudaStreamSynchronize(ctx->st));
+  }
   return PGA_OK;
 }
 

@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import weakref
 
 import numpy as np
 
@@ -136,13 +137,16 @@ def _ptr(a: np.ndarray):
 
 
 def _take(L, p, nbytes: int) -> np.ndarray:
-    """Copy a malloc'd C buffer into numpy and free it."""
-    out = np.empty(nbytes, dtype=np.uint8)
-    if nbytes:
-        C.memmove(out.ctypes.data, p, nbytes)
-    if p:
-        L.free_ptr(C.cast(p, vp))
-    return out
+    """A malloc'd C buffer as a numpy array, which frees it when it goes."""
+    if not p:
+        return np.empty(0, dtype=np.uint8)
+    raw = C.cast(p, vp)
+    if not nbytes:
+        L.free_ptr(raw)
+        return np.empty(0, dtype=np.uint8)
+    mem = (C.c_uint8 * nbytes).from_address(raw.value)
+    weakref.finalize(mem, L.free_ptr, raw).atexit = False
+    return np.frombuffer(mem, dtype=np.uint8)
 
 
 # pga_stage_times' slots
