@@ -79,7 +79,9 @@ struct KeySeeds {
     if (x >= hi) return hi;
     const int lane = threadIdx.x & 31;
     const int64_t b = band(x - 1);
-    int64_t lo = x, h = hi;  // the answer lies in [lo, h], h meaning none below h
+    const unsigned near = __ballot_sync(FULL, x + lane < hi && band(x + lane) > b);  // as it mostly is
+    if (near) return x + __ffs(near) - 1;
+    int64_t lo = min(x + 32, hi), h = hi;  // the answer lies in [lo, h], h meaning none below h
     while (h - lo > 32) {
       const int64_t span = h - lo;
       const int64_t p = lo + (span * (lane + 1)) / 33;  // increasing in lane, inside [lo, h)
@@ -315,6 +317,21 @@ struct KeySeeds {
   }
 };
 
+// v[j] for a j that is the same in all lanes, without local memory
+__device__ __forceinline__ uint16_t pick4(const uint16_t (&v)[4], int j) {
+  return j < 2 ? (j == 0 ? v[0] : v[1]) : (j == 2 ? v[2] : v[3]);
+}
+
+// scan_block out of line: the scan's registers are then not live around the
+// wave loops.  The build for launches bounded by their longest calls is the
+// faster for it (2 x 41 kbp: pair phase 10.9 -> 10.3 ms, 2 x 20 Mbp repeat-rich
+// 59.1 -> 57.6); the others' many short scans are the slower (2 x 200 Mbp
+// repeat-rich 194 -> 206, 2 x 100 Mbp 85 -> 89).
+template <class Sink>
+__device__ __noinline__ int scan_block_out(const KeySeeds &S, int64_t b, int64_t m, int64_t e, Sink &K) {
+  return S.scan_block(b, m, e, K);
+}
+
 // Slot of a call's inputs in the target's record of its own calls, -1 if it
 // is not there.
 __device__ int64_t record_slot(const CallMemo &M, const uint32_t *k) {
@@ -424,7 +441,7 @@ struct ScoutSink {
   }
 };
 
-template <class Sink>
+template <bool OUT, class Sink>
 __device__ int scan_blocks(const KeySeeds &S, const uint16_t *info, int64_t blo, int64_t bhi, Sink &K);
 
 namespace aln {
@@ -433,7 +450,7 @@ __device__ __noinline__ void scout_if_free(WarpWork &W) {
   if (*(volatile const unsigned *)W.share->next_task < W.share->ntasks) return;
   W.task = nullptr;
   ScoutSink K{T, *W.share, 0, 0, -1};
-  scan_blocks(T.S, T.info, T.blo, T.bhi, K);
+  scan_blocks<false>(T.S, T.info, T.blo, T.bhi, K);
 }
 }  // namespace aln
 
@@ -642,59 +659,73 @@ __device__ OvlArena warp_arena(const AlignLaunch &P, int64_t wid) {
 // Block (c, c+1) starting at band c's first seed b is scanned when band c
 // is new (the band below it is not c-1) or band c+1 follows it, as in
 // align_pair; blocks start in [blo, bhi).
-template <class Sink>
+//
+// Most bands hold a chance seed or two and no block of theirs is scanned, so
+// the decision is taken for 32 seeds' bands at once, a lane each, and only the
+// blocks to scan are walked; four groups' infos are read together.  One band
+// start at a time, 60 + 4 Mbp spent 27 of its warps' 31 G cycles here.
+template <bool OUT, class Sink>
 __device__ int scan_blocks(const KeySeeds &S, const uint16_t *info, int64_t blo, int64_t bhi, Sink &K) {
+  constexpr int AHEAD = 4;
   const int lane = threadIdx.x & 31;
   const int64_t n = S.n;
+  // the block of the band that starts at b with info v, the next band (info vn) starting at e
+  auto worth = [](uint16_t v, uint16_t vn) {
+    const bool aux = (vn & BI_ADJ) != 0;  // band c+1 follows band c
+    return ((v & BI_ADJ) == 0 || aux) && (v & 0xff) + (aux ? (vn & 0xff) : 0) >= CHAIN_MIN;
+  };
   int64_t pend = -1;  // the last band start seen, its block not yet decided
-  int pend_sum = 0;
-  bool pend_new = false;
-  bool done = false;
-  int empty = 0;  // steps since the last band start
-  for (int64_t base = blo; base < n && !done; base += 32) {
-    const int64_t i = base + lane;
-    const uint16_t v = i < n ? info[i] : 0;
-    unsigned starts = __ballot_sync(FULL, (v & BI_START) != 0);
-    empty = starts ? 0 : empty + 1;
-    if (empty == 4) {  // a long band: on to the next one's start
-      base = S.next_band_start(base + 32, n) - 32;
-      empty = 0;
+  uint16_t pend_v = 0;
+  int empty = 0;  // groups since the last band start
+  for (int64_t base = blo;; base += 32 * AHEAD) {
+    uint16_t vs[AHEAD];
+#pragma unroll
+    for (int j = 0; j < AHEAD; j++) {
+      const int64_t i = base + 32 * j + lane;
+      vs[j] = i < n ? info[i] : 0;
     }
-    while (starts) {
-      const int l = __ffs(starts) - 1;
-      starts &= starts - 1;
-      const int64_t b = base + l;
-      const uint16_t vb = __shfl_sync(FULL, v, l);
-      if (pend >= 0) {
-        const bool aux = (vb & BI_ADJ) != 0;  // band c+1 follows band c
-        if ((pend_new || aux) && pend_sum + (aux ? (vb & 0xff) : 0) >= CHAIN_MIN) {
-          const int64_t e = aux ? S.band_end(b, S.band(b)) : b;
-          K.cdiag = S.band(pend);
-          K.isnew = pend_new ? 1 : 0;
-          K.alast = -1;
-          if (S.scan_block(pend, b, e, K)) return 1;
-        }
-        pend = -1;
-      }
-      if (b >= bhi) {
-        done = true;
+#pragma unroll 1  // (one copy of what follows)
+    for (int j = 0; j < AHEAD; j++) {
+      const int64_t g = min(base + 32 * j, n);
+      const uint16_t v = pick4(vs, j);
+      // (past the pair's last seed: as if a band no other follows started there)
+      const unsigned starts = g < n ? __ballot_sync(FULL, (v & BI_START) != 0) : 1u;
+      if (!starts) {
+        if (++empty < 4) continue;
+        // a long band: on to the next one's start
+        empty = 0;
+        base = S.next_band_start(g + 32, n) - 32 * AHEAD;
         break;
       }
-      pend = b;
-      pend_sum = vb & 0xff;
-      pend_new = (vb & BI_ADJ) == 0;
+      empty = 0;
+      // the band before this group's first, then the group's own but its last
+      const uint16_t vf = __shfl_sync(FULL, v, __ffs(starts) - 1);
+      bool before = pend >= 0 && worth(pend_v, vf);
+      const unsigned above = starts & ~((2u << lane) - 1u);
+      const uint16_t vn = __shfl_sync(FULL, v, (__ffs(above) - 1) & 31);
+      unsigned take = __ballot_sync(FULL, (v & BI_START) != 0 && above != 0 && g + lane < bhi && worth(v, vn));
+      while (before || take) {
+        const int l = before ? -1 : __ffs(take) - 1;
+        const int next = __ffs(before ? starts : starts & ~((2u << l) - 1u)) - 1;
+        const uint16_t vl = __shfl_sync(FULL, v, l & 31), ve = __shfl_sync(FULL, v, next);
+        const int64_t b = before ? pend : g + l, m = g + next;
+        K.cdiag = S.band(b);
+        K.isnew = ((before ? pend_v : vl) & BI_ADJ) == 0 ? 1 : 0;
+        K.alast = -1;
+        const int64_t e = (ve & BI_ADJ) != 0 ? S.band_end(m, S.band(m)) : m;
+        if (OUT ? scan_block_out(S, b, m, e, K) : S.scan_block(b, m, e, K)) return 1;
+        if (before) before = false;
+        else take &= take - 1;
+      }
+      const int last = 31 - __clz(starts);
+      if (g + last >= bhi) return 0;
+      pend = g + last;
+      pend_v = __shfl_sync(FULL, v, last);
     }
   }
-  if (pend >= 0 && pend_new && pend_sum >= CHAIN_MIN) {  // the pair's last band: no band after it
-    K.cdiag = S.band(pend);
-    K.isnew = 1;
-    K.alast = -1;
-    if (S.scan_block(pend, n, n, K)) return 1;
-  }
-  return 0;
 }
 
-template <class Aligner>
+template <bool OUT, class Aligner>
 __device__ int align_pair_dev(const KeySeeds &S, const uint16_t *info, bool comp, bool self, const Seq &A,
                               const Seq &B, int64_t amxpos, int64_t maxdag, Aligner &AL, Path &path, OvlArena &O,
                               PairResult &R, int lane, int64_t blo, int64_t bhi) {
@@ -708,7 +739,7 @@ __device__ int align_pair_dev(const KeySeeds &S, const uint16_t *info, bool comp
   if (blo >= bhi) return 0;
   ChainSink<Aligner> K{comp, self, A, B, AL, path, O, R, lane, 32, amxpos, (int64_t)A.len + B.len,
                            (int64_t)A.len - maxdag, (int64_t)A.len - amxpos, 0, 0, -1};
-  if (scan_blocks(S, info, blo, bhi, K)) return 1;
+  if (scan_blocks<OUT>(S, info, blo, bhi, K)) return 1;
   R.exit_bepos = path.bepos;
   return 0;
 }
@@ -1010,7 +1041,7 @@ __global__ void __launch_bounds__(ALIGN_THREADS, MINB) k_align_pairs(const __gri
                   (int64_t)A.len - P.amxpos, blo, bhi, 0, 0, 0};
     W.task = SHARE && !tk.self ? &TC : nullptr;
     WarpAligner<MINB <= 3, SHARE> AL{W, spec, P.memo, tk.a, tk.b, SHARE && !tk.self ? &TC : nullptr};
-    int rc = align_pair_dev(S, info, tk.comp != 0, tk.self != 0, A, B, P.amxpos, P.maxdag, AL, path, O, R, lane,
+    int rc = align_pair_dev<MINB == 1 && !SHARE>(S, info, tk.comp != 0, tk.self != 0, A, B, P.amxpos, P.maxdag, AL, path, O, R, lane,
                             blo, bhi);
     __syncwarp();
     PairOut po;

@@ -1594,7 +1594,7 @@ __device__ __forceinline__ void path_to_forward(uint16_t *trace, const Seq &A, c
 // the complemented contig and the path comes back in forward coordinates.
 // Returns 1 on a work-space overflow (W.err says which).
 template <bool BLOCKS, bool SHARE>
-__device__ __forceinline__ int local_alignment_w(WarpWork &W, const AlignSpec &spec, const Seq &A, const Seq &B,
+__device__ __noinline__ int local_alignment_w(WarpWork &W, const AlignSpec &spec, const Seq &A, const Seq &B,
                                                  bool acomp, Path &P, int low, int hgh, int anti, int lbord,
                                                  int hbord) {
   const int maxtp = 2 * (A.len / spec.trace_space + 2);  // trace points the longest path can have
