@@ -236,6 +236,7 @@ __device__ __forceinline__ bool drop_pebbles(const PebblePool &pool, const Wave 
                                              int &hm, int &nak, int &next, int &end) {
   const int lane = threadIdx.x & 31;
   bool cross = act && x >= nak;
+#pragma unroll 1
   do {
     const bool mk = cross && hm < nak;
     const uint32_t mb = __ballot_sync(FULL, mk);
@@ -451,10 +452,16 @@ __device__ __noinline__ bool cross_line(const WarpWork &W, const Wave &wave, uns
 // Runs until the loop ends, the next wave does not fit, the best crosses
 // `line`, or the wave count reaches `stop`.  Returns 1 when the pebble pool is
 // full.
+//
+// R: 16 * R bases are compared per round.  64 where the loop's length counts
+// (a second round's words are another trip to the cache); 32 in the builds
+// with many resident warps, whose limit is fetching their instructions
+// (2 x 200 Mbp repeat-rich: pair phase 201 -> 196 ms).
 // ---------------------------------------------------------------------------
 constexpr int NARROW = 31;
 constexpr int PAST_MAX = (1 << 26) - 1;  // a best further past than this takes the general record search
 
+template <int R>
 __device__ __noinline__ int narrow_waves(WarpWork &W, Wave &io, int stop) {
   const int lane = threadIdx.x & 31;
   const int lup = (lane + 1) & 31, ldn = (lane - 1) & 31;
@@ -483,7 +490,7 @@ __device__ __noinline__ int narrow_waves(WarpWork &W, Wave &io, int stop) {
   }
   // the last wave's pebbles and record; once done, doing it again changes nothing
   auto settle = [&]() {
-    if (!drop_pebbles(pool, S, live, kw, X, dif, HA, HM, NA, next, end)) return false;
+    if (__any_sync(FULL, live && X >= NA) && !drop_pebbles(pool, S, live, kw, X, dif, HA, HM, NA, next, end)) return false;
     const int L = kr & 31;
     const uint64_t t = __shfl_sync(FULL, T, L);
     const int hr = __shfl_sync(FULL, HA, L);
@@ -514,11 +521,11 @@ __device__ __noinline__ int narrow_waves(WarpWork &W, Wave &io, int stop) {
     const int mx = min(S.limA - x, S.limB - x + k);
     const int ia = x + S.offA, ib = x - k + S.offB;
     const bool go = act && (mx | ia | ib) >= 0;
-    uint32_t a[5], b[5];
+    uint32_t a[R + 1], b[R + 1];
     {
       const uint32_t *qa = S.pa + (go ? ia >> 4 : 0), *qb = S.pb + (go ? ib >> 4 : 0);
 #pragma unroll
-      for (int i = 0; i < 5; i++) {
+      for (int i = 0; i <= R; i++) {
         a[i] = __ldg(qa + i);
         b[i] = __ldg(qb + i);
       }
@@ -544,8 +551,8 @@ __device__ __noinline__ int narrow_waves(WarpWork &W, Wave &io, int stop) {
     // snakes, 64 bases per round
     int run = 0;
     if (go) {
-      run = match_loaded<4>(a, (ia & 15) << 1, b, (ib & 15) << 1);
-      if (run == 64) {
+      run = match_loaded<R>(a, (ia & 15) << 1, b, (ib & 15) << 1);
+      if (run == 16 * R) {
         int r;
         do {
           const int qa = min(ia + run, ia + mx), qb = min(ib + run, ib + mx);
@@ -943,13 +950,17 @@ __device__ __noinline__ int wide_waves(WarpWork &W, Wave &io, int stop, int leas
         x = (c + k) >> 1;
         mx = min(S.limA - x, S.limB - x + k);
       }
+      // Most snakes of a wide wave end within 16 bases and few of its passes
+      // cross a trace mark: one word per round and pebbles only where there
+      // are some are the fewer instructions (2 x 200 Mbp repeat-rich: pair
+      // phase 196 -> 179 ms, 2 x 41 kbp 10.2 -> 9.3).
       bool go;
-      const int run = snake<2>(S, x, k, act, mx, go);
+      const int run = snake<1>(S, x, k, act, mx, go);
       const bool hit = act && (!go || run == mx);
       const uint64_t b = hist_step(t0, run);
       x += run;
       c = (x << 1) - k;
-      if (!drop_pebbles(W.pool, S, act, k, x, S.dif, ha, hm, nak, next, end)) {
+      if (__any_sync(FULL, act && x >= nak) && !drop_pebbles(W.pool, S, act, k, x, S.dif, ha, hm, nak, next, end)) {
         err = ALN_ERR_CELLS;
         break;
       }
@@ -1393,7 +1404,7 @@ grow:
       if (cross_line(W, S, W.pair | (fwd ? 1u << 31 : 0u), sh)) break;
       if (sh.full) S.line = I32MAX;
     }
-    if (width <= NARROW) r = narrow_waves(W, S, stop);
+    if (width <= NARROW) r = narrow_waves<BLOCKS ? 4 : 2>(W, S, stop);
     else if (BLOCKS && width <= BLOCK * NARROW) r = block_waves<BLOCK>(W, S, stop);
     else r = wide_waves(W, S, stop, BLOCKS ? BLOCK * NARROW - 8 : BLOCK_OUT);
     if (r) return give_up();
