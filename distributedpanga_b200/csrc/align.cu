@@ -957,15 +957,16 @@ __device__ void run_scout(const AlignLaunch &P, WarpWork &W, const AlignSpec &sp
 
 // The persistent alignment loop.  SHARE: with the launch's table of shared
 // extensions and its scouts, for launches of long contigs (prepare_share,
-// capi.cu).  MINB = 1 keeps every
-// register a warp's wave loop wants (255, two CTAs per SM), for launches
-// bounded by their longest tasks; MINB = 3, 4 and 5 trade spills for more
+// capi.cu).  MINB = 1 keeps every register a warp's wave loop wants (255, two
+// CTAs per SM), for launches bounded by their longest tasks (sharing with
+// three or four: 2 x 100 Mbp 100 and 102 ms of pair phase instead of 85, lone
+// extensions take longer); MINB = 3, 4 and 5 trade spills for more
 // resident warps (three to five CTAs per SM: 168, 128 or 96 registers), for
 // launches bounded by throughput (many pairs with calls), where a wave step's
 // latency is hidden by the other warps of its SM.  The last two leave out the
 // register form of the waves of 32 to 124 diagonals (align_warp.cuh, extend).
-// 2 x 200 Mbp repeat-rich, two to five CTAs: 342, 298, 240, 224 ms of pair
-// phase; 2 x 41 kbp: 10.8, 11.1, 14.4, 14.8.
+// 2 x 200 Mbp repeat-rich, two to five CTAs: 321, 272, 190, 179 ms of pair
+// phase; 2 x 41 kbp: 9.3, 10.3, 11.7, 12.1.
 template <int MINB, bool SHARE>
 __global__ void __launch_bounds__(ALIGN_THREADS, MINB) k_align_pairs(const __grid_constant__ AlignLaunch P) {
   __shared__ BlockSeed s_block[ALIGN_THREADS / 32][32];

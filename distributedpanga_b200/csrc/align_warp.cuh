@@ -1248,10 +1248,10 @@ __device__ __noinline__ bool gather_path(const WarpWork &W, TraceWalk &T, int *w
 // lowest diagonal on entry and, on return, the diagonal the path starts on.
 // A scout's trace is left out (its own intervals go to the share's list).
 // BLOCKS: waves of 32 to 124 diagonals run in registers (block_waves), for
-// launches bounded by their longest calls (2 x 41 kbp: pair phase 10.8 ms
-// against 14.9 through memory); without, they too run as passes
+// launches bounded by their longest calls; without, they too run as passes
 // (wide_waves), for launches bounded by throughput, where the smaller loop
-// and its registers pay (2 x 200 Mbp repeat-rich: 224 ms against 278).
+// and its registers pay (four CTAs per SM, with and without: 2 x 41 kbp 11.4
+// and 13.4 ms of pair phase, 2 x 200 Mbp repeat-rich 260 and 211).
 // Returns 1 on a work-space overflow (W.err set).
 template <bool BLOCKS, bool SHARE>
 __device__ __noinline__ int extend(const bool fwd, const bool scout, WarpWork &W, const AlignSpec &spec, const Seq &A, const Seq &B,

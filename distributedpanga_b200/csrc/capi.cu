@@ -1173,8 +1173,8 @@ int prepare_workspace(pga_ctx *ctx, AlignLaunch &L, int ave_path) {
 
 // Device-planned pairs that can make a call beyond which the alignment launch
 // is bounded by throughput and takes the five-CTA build: 2 x 20 Mbp
-// repeat-rich (0.19 M tasks in all) takes 65 ms of pair phase with two CTAs
-// and 75 with five, 2 x 200 Mbp (1.4 M) 342 and 224.
+// repeat-rich (0.19 M tasks in all) takes 54 ms of pair phase with two CTAs
+// and 60 with five, 2 x 200 Mbp (1.4 M) 321 and 179.
 constexpr int64_t ALIGN_MANY_PAIRS = 1 << 19;
 
 // Frees what the alignment no longer reads once both diagonal sorts are done
