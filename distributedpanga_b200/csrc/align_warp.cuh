@@ -1071,7 +1071,7 @@ struct TraceWalk {
 
 // How the path crosses the lines of the entries that pebble `head` is older
 // than: p is the first pebble after them (kind PEBBLE), or the path's head is
-// from before (HEAD; NONE where that leaves no trace to share).
+// from before (HEAD), or there is no trace to share (NONE).
 __device__ __noinline__ void cross_entries(const WarpWork &W, TraceWalk &T, int head, int kind, int4 p) {
   const int lane = threadIdx.x & 31;
   while (T.last >= 0) {
@@ -1423,10 +1423,20 @@ grow:
     const ShareEntry &E = X.entries[sh.joined];
     ShareRec &R = X.recs[__ldcg(&E.rec)];
     const bool walks = sh.rec >= 0 || (scout && fwd);
-    if (walks) {
-      // this extension's part, as it most likely is, while the owner's is on its way
+    // Its own part, back from head pebble `from`.  An entry that this pebble
+    // is older than has no pebble between its line and the join: what its
+    // joiners would start from lies past the join, so they go on alone.
+    auto walk_own = [&](int from) {
+      T.n = 0;
+      T.jd = T.jb = 0;
       T.last = sh.last;
-      err = walk_back<SHARE>(W, T, cl[sh.guess], 0, 0);
+      const int4 q = cl[from];
+      if (T.last >= 0) cross_entries(W, T, from, SHARE_NONE, q);
+      return walk_back<SHARE>(W, T, q, 0, 0);
+    };
+    if (walks) {
+      // as it most likely is, while the owner's is on its way
+      err = walk_own(sh.guess);
       if (err) {
         W.err |= err;
         return give_up();
@@ -1460,12 +1470,7 @@ grow:
       S.trimha = head;
     } else {
       joined = true;
-      if (walks && head != sh.guess) {
-        T.n = 0;
-        T.jd = T.jb = 0;
-        T.last = sh.last;
-        err = walk_back<SHARE>(W, T, cl[head], 0, 0);
-      }
+      if (walks && head != sh.guess) err = walk_own(head);
       bool listed = false;
       if (sh.rec >= 0 && !err) {
         ShareRec &O = X.recs[sh.rec];
