@@ -1417,7 +1417,7 @@ grow:
   T.jd = T.jb = 0;
   T.last = -1;
   int err = 0;
-  bool joined = false;
+  bool joined = false, closed = false;  // closed: its record, if any, has been published
   if (SHARE && sh.joined >= 0) {
     const ShareTable &X = *W.share;
     const ShareEntry &E = X.entries[sh.joined];
@@ -1483,6 +1483,7 @@ grow:
           O.hmark = q.w;
         }
         listed = publish(W, T, sh.rec, SHARE_JOINED);
+        closed = true;
       }
       if (!scout && !err) {
         // the parts past the join, then this extension's own
@@ -1533,7 +1534,7 @@ grow:
   }
   if (err) {
     W.err |= err;
-    return joined ? 1 : give_up();
+    return closed ? 1 : give_up();
   }
   __syncwarp();
   const int64_t n = T.n;

@@ -65,8 +65,10 @@ struct Table {
 // comp low hgh anti lbord hbord; path7: abpos aepos bbpos bepos diffs tlen err;
 // trace: the results' trace values back to back (trace_cap of them at most).
 // opt: {blocks, share, turns a call runs for before another may (0: to its
-// end), the schedule's seed, entry_cap, rec_cap, list_cap, trace points a call
-// has room for (0: as the device gives)}.  A call has cells_each pebbles of its
+// end), the schedule's seed, entry_cap, rec_cap, list_cap, a call (not 0; -1:
+// none) whose walk back fails: once it has waited for another extension that
+// path crosses on another lane than it did, and the call's pebbles have lost
+// their successors}.  A call has cells_each pebbles of its
 // own, so that a pebble's number tells its call.  stat: {entries, records,
 // entries by kind (none, head, pebble), pebbles named by an entry that are not
 // from after its line, records by status (0 open, done, joined, failed)}.
@@ -86,7 +88,7 @@ extern "C" int warp_host(const uint8_t *seq, int ncontig, const int64_t *len, co
   }
   Table share((int)opt[4], (int)opt[5], opt[6]);
   constexpr int VCAP = 8192;
-  const int64_t room = opt[7] > 0 ? opt[7] : 4 * (maxctg / TSPACE + 4) + 64;
+  const int64_t room = 4 * (maxctg / TSPACE + 4) + 64;
   std::vector<Pebble> cells((size_t)(n * cells_each));
   struct Call {
     std::vector<int> wave = std::vector<int>(11 * VCAP);
@@ -136,6 +138,23 @@ extern "C" int warp_host(const uint8_t *seq, int ncontig, const int64_t *len, co
       C.err[lane] = r ? W.err | 0x100 : 0;
     };
   }
+  bool cut = false;
+  lanes::g_on_wake = [&] {
+    const int64_t k = opt[7];
+    if (cut || k < 0 || lanes::g_warp != &calls[k]->w) return;
+    for (unsigned e = 0; e < share.counters[0]; e++) {
+      ShareEntry &E = share.entries[e];
+      if (E.mark / cells_each == k || E.kind != SHARE_PEBBLE || !share.recs[E.rec].status) continue;
+      for (int l = 0, to = E.lane; l < 32; l++)
+        if (E.HA[l] >= 0 && E.HA[l] != E.HA[to]) {
+          E.lane = l;
+          cut = true;
+          break;
+        }
+    }
+    if (cut)
+      for (int64_t c = k * cells_each; c < (k + 1) * cells_each; c++) cells[c].ptr = min(cells[c].ptr, 0);
+  };
   uint64_t rng = (uint64_t)opt[3] * 0x9e3779b97f4a7c15ull + 1;
   for (int64_t left = n, at = 0; left > 0;) {
     if (opt[2] > 0) {
@@ -152,6 +171,7 @@ extern "C" int warp_host(const uint8_t *seq, int ncontig, const int64_t *len, co
     for (int64_t t = 0; !w.done && (opt[2] == 0 || t < opt[2]); t++) lanes::turn(w);
     if (w.done) left--;
   }
+  lanes::g_on_wake = nullptr;
   int64_t nt = 0;
   for (int64_t i = 0; i < n; i++) {
     const Call &C = *calls[i];

@@ -39,6 +39,8 @@ inline int g_lane = 0;
 inline jmp_buf g_turn;          // the scheduler
 inline ucontext_t g_back;
 
+inline std::function<void()> g_on_wake;  // called when a lane has slept
+
 inline void leave() {
   Warp::Lane &l = g_warp->lane[g_lane];
   if (_setjmp(l.at) == 0) _longjmp(g_turn, 1);
@@ -168,7 +170,10 @@ template <class T> unsigned __match_any_sync(unsigned, T v) {
 }
 inline void __syncwarp() { lanes::gather(0); }
 inline void __threadfence() {}
-inline void __nanosleep(unsigned) { lanes::leave(); }
+inline void __nanosleep(unsigned) {
+  lanes::leave();
+  if (lanes::g_on_wake) lanes::g_on_wake();
+}
 
 inline int __popc(uint32_t v) { return __builtin_popcount(v); }
 inline int __clz(int v) { return v ? __builtin_clz((unsigned)v) : 32; }

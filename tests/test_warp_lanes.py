@@ -41,12 +41,12 @@ class Out:
         self.open, self.done, self.joined, self.failed = (int(v) for v in stat[6:10])
 
 
-def on_lanes(L, cs, req, blocks=True, share=True, turns=0, seed=1, entries=4096, records=4096, listed=1 << 20, room=0,
+def on_lanes(L, cs, req, blocks=True, share=True, turns=0, seed=1, entries=4096, records=4096, listed=1 << 20, cut=-1,
              cells=200_000, freq=EVEN):
     seq = np.concatenate(cs).astype(np.uint8)
     ln = np.array([len(c) for c in cs], np.int64)
     req = np.ascontiguousarray(req, np.int32)
-    opt = np.array([blocks, share, turns, seed, entries, records, listed, room], np.int64)
+    opt = np.array([blocks, share, turns, seed, entries, records, listed, cut], np.int64)
     path, stat = np.zeros((len(req), 7), np.int32), np.zeros(10, np.int64)
     tr = np.zeros(4 * len(req) * (int(ln.max()) // 100 + 4), np.uint16)
     assert L.warp_host(seq.ctypes.data, len(cs), ln.ctypes.data, freq.ctypes.data, len(req), req.ctypes.data,
@@ -99,3 +99,21 @@ def test_an_entry_names_a_pebble_from_after_its_line(lanes, seed):
     assert out.joined > 0 and out.open == 0
     assert out.misplaced == 0
     check(out, scalar([a, b], req))
+
+
+@pytest.mark.parametrize("seed", [1, 2, 5, 8])
+def test_a_failing_walk_closes_its_record(lanes, seed):
+    """A call that owns entries joins another and then cannot walk its path
+    back: it reports the error, and no record stays open for others to wait
+    on."""
+    from distributedpanga_b200 import synth
+    rng = np.random.default_rng(seed)
+    a = rng.integers(0, 4, 40_000).astype(np.uint8)
+    b = synth.indels(rng, synth.substitute(rng, a, 0.1), 0.05, lambda k: rng.integers(1, 4, size=k), 0.5)
+    req = []
+    for x in (12_500, 200, 2800, 1500):
+        y = x * len(b) // len(a)
+        req.append([0, 1, 0, x - y - 25, x - y + 25, x + y, -1, -1])
+    out = on_lanes(lanes, [a, b], req, turns=300, seed=seed, cut=2, cells=400_000)
+    assert out.err.tolist() == [0, 0, 0x102, 0]
+    assert out.open == 0 and out.failed > 0
