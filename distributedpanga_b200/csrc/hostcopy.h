@@ -13,7 +13,7 @@
 #include <atomic>
 #include <cstdint>
 #include <cstring>
-#include <system_error>
+#include <exception>
 #include <thread>
 #include <cuda_runtime.h>
 
@@ -73,8 +73,8 @@ class HostCopier {
     for (int w = 1; w < n; w++) {
       try {
         t[w] = std::thread(work, w);
-      } catch (const std::system_error &) {
-        break;  // fewer threads, then
+      } catch (const std::exception &) {
+        break;  // no thread or no memory for one: fewer threads, then
       }
     }
     work(0);
