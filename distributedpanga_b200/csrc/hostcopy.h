@@ -7,8 +7,10 @@
 // copies and the faults of the chunks overlap: 50 MB of packed bases to fresh
 // memory 11.3 -> 2.5 ms, 17 MB of records in and 148 MB of entries and prefix
 // table out (pga_build_kmer_adapter) 37-43 -> 8-10.  Below STAGE_MIN starting
-// the threads (0.2 ms) costs what they save; those copies, and memory that is
-// pinned or managed, go to the driver.
+// the threads costs what they save; those copies, and memory that is pinned or
+// managed, go to the driver.  pga_gdb_load of warm memory, driver and staged: 4 MB
+// 0.28 and 0.32 ms, 5 MB 0.33 and 0.36, 6 MB 0.39 and 0.38, 8 MB 0.49 and 0.46,
+// 16 MB 0.92 and 0.73; pga_gdb_copy, 5 MB 0.34 and 0.37, 12 MB 0.78 and 0.57.
 #pragma once
 #include <atomic>
 #include <cstdint>
@@ -23,7 +25,7 @@ class HostCopier {
  public:
   static constexpr int WORKERS = 8;
   static constexpr size_t CHUNK = 1 << 20;
-  static constexpr size_t STAGE_MIN = 4 << 20;
+  static constexpr size_t STAGE_MIN = 6 << 20;
 
   // Copies `bytes` between `host` and `dev` in `st`'s order; a staged copy has
   // ended on return, any other is as cudaMemcpyAsync leaves it.
