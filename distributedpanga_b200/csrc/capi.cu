@@ -1172,10 +1172,14 @@ int prepare_workspace(pga_ctx *ctx, AlignLaunch &L, int ave_path) {
 }
 
 // Device-planned pairs that can make a call beyond which the alignment launch
-// is bounded by throughput and takes the five-CTA build: 2 x 20 Mbp
-// repeat-rich (0.19 M tasks in all) takes 54 ms of pair phase with two CTAs
-// and 60 with five, 2 x 200 Mbp (1.4 M) 321 and 179.
-constexpr int64_t ALIGN_MANY_PAIRS = 1 << 19;
+// is bounded by throughput and takes the five-CTA build.  Pair phase with two
+// and with five CTAs, repeat-rich genomes of short contigs: 115 K such pairs
+// (2 x 25 Mbp) 37 and 41 ms, 143 K 40 and 39, 164 K 46 and 43, 238 K (2 x 50 Mbp)
+// 67 and 57, 390 K 132 and 79, more than 524 K (2 x 120 Mbp) 211 and 123.  With
+// contigs that could share extensions, which the five-CTA build does not do, the
+// line lies higher (2 x 100 Mbp in chromosomes, 315 such pairs, 68 and 100 ms;
+// 60 + 4 Mbp, 15 K, 26 and 34; 2 x 200 Mbp repeat-rich 321 and 179).
+constexpr int64_t ALIGN_MANY_PAIRS = 1 << 17, ALIGN_MANY_PAIRS_LONG = 1 << 19;
 
 // Frees what the alignment no longer reads once both diagonal sorts are done
 // -- the index (records, LCPs, entries, scratch) and the unsorted seeds -- so
@@ -1472,9 +1476,10 @@ int run_align(pga_ctx *ctx) {
     L.nseeds[u] = ctx->nseed[u];
   }
   L.fo_pos = fo_pos;
-  // the launch is bounded by its longest tasks up to about half a million
-  // pairs, by throughput beyond: then the build with more resident warps
-  L.min_blocks = ctx->align_build ? ctx->align_build : nsmall > ALIGN_MANY_PAIRS ? 5 : 2;
+  // bounded by its longest tasks or, with many pairs, by throughput: then the
+  // build with more resident warps
+  const int64_t many = maxctg < SHARE_CONTIG ? ALIGN_MANY_PAIRS : ALIGN_MANY_PAIRS_LONG;
+  L.min_blocks = ctx->align_build ? ctx->align_build : nsmall > many ? 5 : 2;
   L.sred = sred;
   L.fo_last = sred + 8;
   L.fo_earlier = sred + 8 + nc;

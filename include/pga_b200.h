@@ -263,8 +263,9 @@ int pga_align_profile(const pga_ctx *ctx, int64_t *prof2);
  * kernel runs -- 2 (255 registers, two CTAs per SM: best when the launch is
  * bounded by its longest alignments), 3 (168 registers, three CTAs per SM),
  * 4 (128 registers, four) or 5 (96 registers, five CTAs per SM: best for
- * launches of many pairs); 0 (the default) picks 5 above 2^20 pairs, else 2.
- * The alignments are the same either way. */
+ * launches of many pairs); 0 (the default) picks 5 above 2^17 pairs that can
+ * make a call and are not cut into ranges (2^19 where a contig has 65,536 bases
+ * or more), else 2.  The alignments are the same either way. */
 int pga_align_set_build(pga_ctx *ctx, int ctas_per_sm);
 
 /* Tuning, no counterpart in the reference: when one Local_Alignment call of
@@ -273,9 +274,8 @@ int pga_align_set_build(pga_ctx *ctx, int ctas_per_sm);
  * which bounds the launch -- soon has the SM to itself; the remaining tasks
  * go to the other SMs.  0 turns this off;
  * -1 (the default) is 20000 for launches of the two-CTA build and off for
- * the builds of three to five CTAs per SM (launches of more than 2^20
- * pairs, bounded by throughput).  The alignments are the same for every
- * value. */
+ * the builds of three to five CTAs per SM (launches of many pairs, bounded by
+ * throughput).  The alignments are the same for every value. */
 int pga_align_set_long_waves(pga_ctx *ctx, int waves);
 
 /* Tuning, no counterpart in the reference: the width in bits (18..22) of the
