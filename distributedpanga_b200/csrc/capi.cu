@@ -844,12 +844,27 @@ void prepare_share(pga_ctx *ctx, AlignLaunch &L, int64_t nt) {
   L.share = (const aln::ShareTable *)base;
 }
 
+// Frees the shared extensions' pools.  Returns whether any were held.
+bool release_share(pga_ctx *ctx) {
+  bool any = false;
+  for (DBuf *b : {&ctx->share_tab, &ctx->share_ent, &ctx->share_list})
+    if (b->p) {
+      ctx->arena.release(b->p);
+      b->p = nullptr;
+      b->cap = 0;
+      any = true;
+    }
+  return any;
+}
+
 // Runs a plan: the warps take the tasks in plan order.  tout: one PairOut per
 // whole pair (at its place in the plan), fout: one per finish task; *cycles
 // grows by the launch's task cycles.  Pebbles live for one launch; candidate
 // traces, range candidates and survivors accumulate over the launches of one
 // pga_align.  A pool that overflows is grown (keeping what earlier launches
-// left in it) and the launch runs again from the same counters.
+// left in it) and the launch runs again from the same counters; without sharing
+// where the shared extensions' memory, or their scouts' pebbles, are what a launch
+// lacks.
 int align_launch(pga_ctx *ctx, AlignLaunch &L, const LaunchPlan &plan, std::vector<PairOut> &tout,
                  std::vector<PairOut> &fout, long long *cycles, long long *max_cycles, int64_t *max_task_calls) {
   const size_t ni = plan.tasks.size(), nf = plan.fins.size();
@@ -976,29 +991,38 @@ int align_launch(pga_ctx *ctx, AlignLaunch &L, const LaunchPlan &plan, std::vect
     bool grown = false;
     if (attempt < 6) {
       int r = PGA_OK;
+      auto grow = [&](auto take) {
+        if (r) return;
+        r = take();
+        if (r == PGA_ERR_NOMEM && release_share(ctx)) {
+          L.share = nullptr;
+          r = take();
+        }
+      };
       // pebble numbers are int: at most 2^31 - 1 pebbles
       const size_t max_cells = sizeof(aln::Pebble) * (size_t)0x7fffffff;
       if ((errs & aln::ALN_ERR_CELLS) && ctx->cells.cap < max_cells) {
-        r = r ? r : ensure(ctx, ctx->cells, std::min(2 * ctx->cells.cap, max_cells));
+        const size_t want = std::min(2 * ctx->cells.cap, max_cells);
+        grow([&] { return ensure(ctx, ctx->cells, want); });
         L.cell_cap = (int64_t)(ctx->cells.cap / sizeof(aln::Pebble));
         L.cells = P<aln::Pebble>(ctx->cells);
         grown = true;
       }
       if (errs & aln::ALN_ERR_TRACE) {
-        r = r ? r : grow_keep(ctx, ctx->cand, 2 * ctx->cand.cap, base[0]);
+        grow([&] { return grow_keep(ctx, ctx->cand, 2 * ctx->cand.cap, base[0]); });
         L.cand_cap = (int64_t)ctx->cand.cap;
         L.cand_bytes = P<uint8_t>(ctx->cand);
         grown = true;
       }
       if (errs & 0x800) {
-        r = r ? r : grow_keep(ctx, ctx->rng_ovl, 2 * ctx->rng_ovl.cap, sizeof(aln::Ovl) * base[1]);
+        grow([&] { return grow_keep(ctx, ctx->rng_ovl, 2 * ctx->rng_ovl.cap, sizeof(aln::Ovl) * base[1]); });
         L.rng_cap = (int64_t)(ctx->rng_ovl.cap / sizeof(aln::Ovl));
         L.rng_ovl = P<aln::Ovl>(ctx->rng_ovl);
         grown = true;
       }
       if (errs & 0x400) {
-        r = r ? r : grow_keep(ctx, ctx->recs, 2 * ctx->recs.cap, sizeof(AlnRec) * base[2]);
-        r = r ? r : grow_keep(ctx, ctx->outb, 2 * ctx->outb.cap, base[3]);
+        grow([&] { return grow_keep(ctx, ctx->recs, 2 * ctx->recs.cap, sizeof(AlnRec) * base[2]); });
+        grow([&] { return grow_keep(ctx, ctx->outb, 2 * ctx->outb.cap, base[3]); });
         L.rec_cap = (int64_t)(ctx->recs.cap / sizeof(AlnRec));
         L.out_cap = (int64_t)ctx->outb.cap;
         L.recs = P<AlnRec>(ctx->recs);
@@ -1007,14 +1031,19 @@ int align_launch(pga_ctx *ctx, AlignLaunch &L, const LaunchPlan &plan, std::vect
       }
       if ((errs & 0x1000) || ((errs & aln::ALN_ERR_OVLS) && !(errs & (0x400 | 0x800)))) {
         int64_t oc = 2 * L.ovl_cap;
-        r = r ? r : ensure(ctx, ctx->ovl, sizeof(aln::Ovl) * (size_t)L.nwarps * oc);
-        r = r ? r : ensure(ctx, ctx->perm, sizeof(int) * 2 * (size_t)L.nwarps * oc);
+        grow([&] { return ensure(ctx, ctx->ovl, sizeof(aln::Ovl) * (size_t)L.nwarps * oc); });
+        grow([&] { return ensure(ctx, ctx->perm, sizeof(int) * 2 * (size_t)L.nwarps * oc); });
         L.ovl_cap = oc;
         L.ovl = P<aln::Ovl>(ctx->ovl);
         L.perm = P<int>(ctx->perm);
         grown = true;
       }
       if (r) return r;
+    }
+    if (!grown && L.share && (errs & aln::ALN_ERR_CELLS)) {
+      L.share = nullptr;
+      attempt = -1;
+      continue;
     }
     if (!grown) {
       if (sred[3] && sred[6] < (unsigned long long)nt) {
@@ -3060,7 +3089,7 @@ int pga_align(pga_ctx *ctx, int64_t *nalign) {
   AlignScope scope(ctx);
   stage_begin(ctx, ST_ALIGN);
   int r = run_align(ctx);
-  if (r == PGA_ERR_NOMEM && release_for_align(ctx)) {
+  if (r == PGA_ERR_NOMEM && (release_share(ctx) | release_for_align(ctx))) {
     cudaGetLastError();
     r = run_align(ctx);
   }
