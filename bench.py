@@ -33,7 +33,8 @@ cpu_baseline = the reference pipeline compiled from source (oracle/_ref), or
 --impl reference = the reference pipeline (oracle/_ref) on every host core:
          one concurrent world-1 run per core on a sample, the aggregate rate
          (its driver has one alignment thread and gets its parallelism from
-         MPI ranks, which this host does not have)
+         MPI ranks, which this host does not have); unavailable where the
+         reference is not built
 served_form = a resident 1 Gbp target (with the record of its own
          Local_Alignment calls) against a Poisson stream of 12 query
          assemblies, beside the plain form on the same requests; every served
@@ -480,40 +481,34 @@ def run_reference(args, rank: int) -> None:
     """The reference arm: the reference's own pipeline on all the host's
     cores, each step one concurrent world-1 run per core (reference_runs) on a
     sample of the workload's generator (REF_SCALE, or --ref-scale), the
-    aggregate rate over the slowest run; rank 0 alone."""
+    aggregate rate over the slowest run; rank 0 alone.  Unavailable where the
+    reference is not built."""
     if rank != 0:
         return
     from oracle import binding as orc
+    if not orc.ref_available():
+        emit(rank, {"impl": "reference", "unavailable": "the reference pipeline (oracle/_ref) is not built: "
+                                                        "its sources are not on this machine"})
+        return
     vals = []
-    detail = None
-    ref = ReferenceSample(args.ref_scale) if orc.ref_available() else None
+    ref = ReferenceSample(args.ref_scale)
     nrun = reference_runs()
+    mbp = ref.mbp * nrun
     for it in range(args.warmup + args.steps):
-        if ref is not None:
-            mbp, sec = ref.mbp * nrun, ref.run_many(nrun)
-            kind, cores = "reference", nrun
-        else:
-            orc.build()
-            mbp, sec = port_sample(args.ref_scale)
-            kind, cores = "port", 1
+        sec = ref.run_many(nrun)
         if it >= args.warmup:
             vals.append(mbp / sec)
-        detail = (mbp, kind, cores)
     v = statistics.median(vals)
-    mbp, kind, cores = detail
-    if kind == "reference":
-        sample = (WL["name"] + " generator at scale %g (%.1f Mbp) per run, %d concurrent world-1 runs of the "
-                  "reference pipeline per step (one per host core; its driver has one alignment thread and no MPI "
-                  "is here), aggregate Mbp / the slowest run's TOTAL stage time"
-                  % (args.ref_scale, mbp / cores, cores))
-    else:
-        sample = WL["name"] + " generator at scale %g (%.1f Mbp) per step" % (args.ref_scale, mbp)
+    sample = (WL["name"] + " generator at scale %g (%.1f Mbp) per run, %d concurrent world-1 runs of the "
+              "reference pipeline per step (one per host core; its driver has one alignment thread and no MPI "
+              "is here), aggregate Mbp / the slowest run's TOTAL stage time"
+              % (args.ref_scale, ref.mbp, nrun))
     line = {"impl": "reference", "metric": METRIC, "value": v, "unit": UNIT, "n_gpus": args.gpus,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": mbp / v * 1000.0,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "u8",
             "data": "synthetic (seeded generator)",
             "config": {"workload": WORKLOADS[WL["name"]], "sample_scale": args.ref_scale, "sample": sample},
-            "cpu_baseline": {"value": v, "unit": UNIT, "cores": cores, "kind": kind, "sample": sample},
+            "cpu_baseline": {"value": v, "unit": UNIT, "cores": nrun, "kind": "reference", "sample": sample},
             "e2e": {"value": v, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
     emit(rank, line)
 
