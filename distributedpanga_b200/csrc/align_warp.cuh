@@ -59,6 +59,7 @@ struct __align__(16) RingCell {
   int HA, HM;
 };
 
+// MurmurHash3's 32-bit finaliser (A. Appleby, public domain).
 __device__ __forceinline__ uint32_t mix32(uint32_t h) {
   h ^= h >> 16;
   h *= 0x85ebca6bu;
@@ -353,7 +354,7 @@ __device__ __noinline__ bool cross_line(const WarpWork &W, const Wave &wave, uns
   }
   // which diagonals have the same head pebble: the first lane with this one's
   const int pat = __ffs(__match_any_sync(FULL, live ? HA : -2 - lane)) - 1;
-  // the state's key
+  // the state's key (the multipliers are the golden ratio's and a prime of xxHash)
   const uint32_t tl = (uint32_t)T, th = (uint32_t)(T >> 32) & HIST_HI;
   const uint32_t a = mix32(V + 0x9e3779b9u * (lane + 1)) + mix32(tl ^ 0x7f4a7c15u), b = mix32(th + HM) + mix32(NA ^ tl ^ pat << 16);
   const uint32_t h1 = __reduce_xor_sync(FULL, live ? mix32(a + 31 * b) : 0);
@@ -548,7 +549,7 @@ __device__ __noinline__ int narrow_waves(WarpWork &W, Wave &io, int stop) {
     T = __shfl_sync(FULL, T, sl);
     NA = k < low ? nlo : (k > hgh ? nhi : NA);
 
-    // snakes, 64 bases per round
+    // snakes: 16 * R bases, then 32 per round
     int run = 0;
     if (go) {
       run = match_loaded<R>(a, (ia & 15) << 1, b, (ib & 15) << 1);

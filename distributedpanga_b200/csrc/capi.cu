@@ -115,7 +115,7 @@ struct pga_ctx {
   bool capture = false;
   DBuf mlog_key, mlog_val, mlog_toff, mlog_trace, mlog_ctr;
   int64_t cap_calls = 0, cap_bytes = 0;
-  // the scoring tables of the last alignment
+  // the path average and mismatch penalty of the last alignment
   int ave_path_host = 0, dscore_host = 0;
   HostCopier copier;
   bool trace_valid = false;        // h_trace holds the last alignment's traces
@@ -178,8 +178,8 @@ struct pga_target {
   int64_t base_count[4] = {0, 0, 0, 0};
   DBuf bps, rec, start;  // sequence image, sorted records, prefix table (NPREFIX + 1)
   // The target's own run's Local_Alignment calls (pga_target_create_reuse):
-  // a table of their inputs and results (CallMemo), and the scoring tables
-  // they were made with.
+  // a table of their inputs and results (CallMemo), and the path average and
+  // mismatch penalty they were made with.
   struct Memo {
     bool valid = false;
     int ave_path = 0, dscore = 0;
@@ -1062,7 +1062,8 @@ int align_launch(pga_ctx *ctx, AlignLaunch &L, const LaunchPlan &plan, std::vect
 }
 
 // NUMERIC (with sentinels) and 2-bit packed copies of every contig, the base
-// frequencies if not given, and the scoring tables (New_Align_Spec).
+// frequencies if not given, and the path average and mismatch penalty
+// (New_Align_Spec).
 int prepare_sequences(pga_ctx *ctx, int *ave_path) {
   const int nc = ctx->ncontig;
   if (!ctx->have_numeric) {
@@ -1146,7 +1147,7 @@ int prepare_workspace(pga_ctx *ctx, AlignLaunch &L, int ave_path) {
   L.nwarps = 148 * 20;  // work spaces for the five-CTA build's resident warps
   L.vcap = 8192;
   L.point_cap = 4 * (ctx->maxctg / 100 + 4) + 64;
-  // Pools sized from the sequence total; align_run_tasks grows one that
+  // Pools sized from the sequence total; align_launch grows one that
   // overflows and reruns the launch.  Buffers keep their size across calls.
   int64_t seqtot = 0;
   for (int c = 0; c < ctx->ncontig; c++) seqtot += ctx->clen[c];
