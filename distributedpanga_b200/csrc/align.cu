@@ -508,6 +508,7 @@ struct WarpAligner {
     P.diffs = __ldcg(&c.diffs);
     P.tlen = tlen;
     P.trace_off = 0;
+    if (lane == 0) atomicAdd(X.joins + 3, 1u);
     return true;
   }
 

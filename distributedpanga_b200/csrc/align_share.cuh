@@ -105,6 +105,9 @@ struct ShareTable {
   int64_t list_cap;
   unsigned *nentry, *nrec;        // counters, zero at launch
   unsigned long long *nlist;
+  // joins whose path goes on past the next trace mark [0], ends before it [1]
+  // or at the line [2]; calls taken from a scout [3]
+  unsigned *joins;
   // the scouts' queue: queued [0, min(qtail, qcap)), taken below qhead; tasks
   // that have ended
   Scout *scouts;

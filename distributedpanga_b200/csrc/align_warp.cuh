@@ -1461,7 +1461,9 @@ grow:
     }
     const int dif = S.dif - __ldcg(&E.dif), kc = S.low + ((__ldcg(&E.lane) - S.low) & 31);
     const int head = W.C[S.cur][kc & vmask].HA;
-    if (status == SHARE_DONE && __ldcg(&R.tipd) <= __ldcg(&E.dif)) {
+    const bool own = status == SHARE_DONE && __ldcg(&R.tipd) <= __ldcg(&E.dif);
+    if (lane == 0) atomicAdd(X.joins + (own ? 2 : kind == SHARE_HEAD ? 1 : 0), 1u);
+    if (own) {
       // the owner found nothing past this wave: the tip is this extension's own
     } else if (kind == SHARE_HEAD) {
       // the owner's tip is before the next mark

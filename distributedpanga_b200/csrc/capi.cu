@@ -144,6 +144,7 @@ struct pga_ctx {
   int64_t align_stats[8] = {0};    // pga_align_stats
   float align_ms[4] = {0};         // pga_align_times
   int64_t align_work[4] = {0};     // pga_align_work
+  int64_t align_shared[8] = {0};   // pga_align_share_stats
   int64_t align_prof[2] = {0};     // pga_align_profile: SM cycles in Local_Alignment, in finishing steps
   // pga_local_alignment: requests, paths, trace pool
   DBuf lreq, lpath, ltoff, ltrace, lnext;
@@ -781,6 +782,7 @@ struct LaunchPlan {
 // 12.4 (250 kbp, 684 and 58,910), 2 x 20 Mbp repeat-rich 60 and 57 (10 kbp,
 // 98,578 and 90,791): the larger loop costs, and whole pairs repeat no path.
 constexpr int64_t SHARE_CONTIG = 4 * aln::SHARE_LINE;
+constexpr int SHARE_COUNTERS = 16;  // words
 
 void prepare_share(pga_ctx *ctx, AlignLaunch &L, int64_t nt) {
   L.share = nullptr;
@@ -827,6 +829,7 @@ void prepare_share(pga_ctx *ctx, AlignLaunch &L, int64_t nt) {
   X.qhead = counters + 4;
   X.qtail = counters + 5;
   X.ended = counters + 6;
+  X.joins = counters + 8;
   X.next_task = P<unsigned>(ctx->task_next);
   X.keys = (unsigned long long *)(base + keys);
   X.vals = (int *)(base + vals);
@@ -922,7 +925,7 @@ int align_launch(pga_ctx *ctx, AlignLaunch &L, const LaunchPlan &plan, std::vect
       CK(cudaMemcpyAsync(ctx->share_tab.p, &X, sizeof(X), cudaMemcpyHostToDevice, ctx->st));
       CK(cudaMemsetAsync(X.keys, 0, sizeof(unsigned long long) * ((size_t)X.mask + 1), ctx->st));
       CK(cudaMemsetAsync(X.vals, 0xff, sizeof(int) * ((size_t)X.mask + 1), ctx->st));
-      CK(cudaMemsetAsync(X.nentry, 0, 64, ctx->st));
+      CK(cudaMemsetAsync(X.nentry, 0, sizeof(unsigned) * SHARE_COUNTERS, ctx->st));
       CK(cudaMemsetAsync(X.scouts, 0, sizeof(aln::Scout) * (size_t)X.qcap, ctx->st));
       CK(cudaMemsetAsync(X.ckeys, 0, sizeof(unsigned long long) * ((size_t)X.cmask + 1), ctx->st));
       CK(cudaMemsetAsync(X.cvals, 0xff, sizeof(int) * ((size_t)X.cmask + 1), ctx->st));
@@ -957,6 +960,9 @@ int align_launch(pga_ctx *ctx, AlignLaunch &L, const LaunchPlan &plan, std::vect
       CK(cudaGetLastError());
       CK(cudaMemcpyAsync(fout.data(), ctx->fout.p, sizeof(PairOut) * nf, cudaMemcpyDeviceToHost, ctx->st));
     }
+    unsigned shared[SHARE_COUNTERS] = {0};
+    if (L.share && (nt || L.nsmall > 0))
+      CK(cudaMemcpyAsync(shared, ctx->share_host.nentry, sizeof(shared), cudaMemcpyDeviceToHost, ctx->st));
     unsigned long long used[4] = {0, 0, 0, 0}, prof[2] = {0, 0};
     CK(cudaMemcpyAsync(prof, L.prof, 16, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(&used[0], ctx->cand_next.p, 8, cudaMemcpyDeviceToHost, ctx->st));
@@ -980,6 +986,13 @@ int align_launch(pga_ctx *ctx, AlignLaunch &L, const LaunchPlan &plan, std::vect
       ctx->align_work[0] += (int64_t)sred[4];
       ctx->align_work[1] += (int64_t)sred[5];
       ctx->align_work[3] += nt + L.nsmall;
+      if (L.share) {
+        ctx->align_shared[0] += 1;
+        ctx->align_shared[1] += std::min(shared[0], (unsigned)ctx->share_host.entry_cap);
+        ctx->align_shared[2] += std::min(shared[1], (unsigned)ctx->share_host.rec_cap);
+        ctx->align_shared[3] += std::min(shared[5], (unsigned)ctx->share_host.qcap);
+        for (int i = 0; i < 4; i++) ctx->align_shared[4 + i] += shared[8 + i];
+      }
       *cycles += (long long)sred[1];
       if ((long long)(sred[2] >> 16) > *max_cycles) {
         *max_cycles = (long long)(sred[2] >> 16);
@@ -1339,6 +1352,7 @@ int run_align(pga_ctx *ctx) {
   if (r0) return r0;
   ctx->cand_used = ctx->rng_used = ctx->rec_used = ctx->out_used = 0;
   for (int i = 0; i < 4; i++) ctx->align_work[i] = 0;
+  for (int64_t &v : ctx->align_shared) v = 0;
   ctx->align_prof[0] = ctx->align_prof[1] = 0;
 
   // 4. Pair lists of both units.  They stay on the device; only the pairs
@@ -3228,6 +3242,12 @@ int pga_local_alignment_copy(pga_ctx *ctx, int32_t *path7, int64_t *trace_off, u
 int pga_align_work(const pga_ctx *ctx, int64_t *work4) {
   if (!ctx || !work4) return PGA_ERR_ARG;
   for (int i = 0; i < 4; i++) work4[i] = ctx->align_work[i];
+  return PGA_OK;
+}
+
+int pga_align_share_stats(const pga_ctx *ctx, int64_t *stats8) {
+  if (!ctx || !stats8) return PGA_ERR_ARG;
+  for (int i = 0; i < 8; i++) stats8[i] = ctx->align_shared[i];
   return PGA_OK;
 }
 

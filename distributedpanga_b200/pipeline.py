@@ -77,6 +77,7 @@ _SIGS = {
     "pga_align_times": (C.c_int, [vp, C.POINTER(C.c_float)]),
     "pga_align_work": (C.c_int, [vp, vp]),
     "pga_align_profile": (C.c_int, [vp, vp]),
+    "pga_align_share_stats": (C.c_int, [vp, vp]),
     "pga_local_alignment": (C.c_int, [vp, C.c_int64, vp, C.POINTER(C.c_int64)]),
     "pga_local_alignment_copy": (C.c_int, [vp, vp, vp, vp]),
     "pga_write_1aln": (C.c_int, [C.c_char_p, C.c_char_p, C.c_char_p, C.c_char_p, C.c_char_p, C.c_char_p, C.c_int,
@@ -468,6 +469,14 @@ class Device:
         a = np.zeros(2, dtype=np.int64)
         self._ck(self.L.pga_align_profile(self.h, a.ctypes.data_as(vp)), "align_profile")
         return {"local_alignment_cycles": int(a[0]), "finish_cycles": int(a[1])}
+
+    def share_stats(self) -> dict:
+        """What the calls of the last align() took from one another (pga_align_share_stats)."""
+        a = np.zeros(8, dtype=np.int64)
+        self._ck(self.L.pga_align_share_stats(self.h, a.ctypes.data_as(vp)), "align_share_stats")
+        keys = ("launches", "entries", "records", "scouts", "joins_past_mark", "joins_before_mark", "joins_own_tip",
+                "scouted_calls")
+        return {k: int(v) for k, v in zip(keys, a)}
 
     def set_build(self, ctas_per_sm: int):
         """Which build of the alignment kernel runs (0 automatic, or 2 to 5 CTAs per SM)."""

@@ -259,6 +259,16 @@ int pga_align_set_ranges(pga_ctx *ctx, int64_t range_seeds);
  * steps, each summed over warps (the rest of a task's cycles is the chain
  * scan and its bookkeeping). */
 int pga_align_profile(const pga_ctx *ctx, int64_t *prof2);
+
+/* What the calls of the last pga_align took from one another: stats8 = launches
+ * that shared extensions, states entered, extensions with an entry, scouts
+ * queued, joins whose path went on past the next trace mark, joins whose path
+ * ended before it, joins that found nothing past the line, calls whose result a
+ * scout had.  All zero where no launch shared (builds of three CTAs per SM and
+ * up, short contigs, mostly whole pairs).  Which calls meet depends on timing;
+ * the alignments do not. */
+int pga_align_share_stats(const pga_ctx *ctx, int64_t *stats8);
+
 /* Tuning, no counterpart in the reference: which build of the alignment
  * kernel runs -- 2 (255 registers, two CTAs per SM: best when the launch is
  * bounded by its longest alignments), 3 (168 registers, three CTAs per SM),

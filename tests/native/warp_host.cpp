@@ -54,6 +54,7 @@ struct Table {
     X.nentry = counters;
     X.nrec = counters + 1;
     X.nlist = &nlist;
+    X.joins = counters + 8;
     X.next_task = &next_task;
     X.ntasks = 1;
   }
