@@ -6,11 +6,14 @@
 // with two pinned chunks and a stream of its own, so that the transfers, the
 // copies and the faults of the chunks overlap: 50 MB of packed bases to fresh
 // memory 11.3 -> 2.5 ms, 17 MB of records in and 148 MB of entries and prefix
-// table out (pga_build_kmer_adapter) 37-43 -> 8-10.  Below STAGE_MIN starting
-// the threads costs what they save; those copies, and memory that is pinned or
-// managed, go to the driver.  pga_gdb_load of warm memory, driver and staged: 4 MB
-// 0.28 and 0.32 ms, 5 MB 0.33 and 0.36, 6 MB 0.39 and 0.38, 8 MB 0.49 and 0.46,
-// 16 MB 0.92 and 0.73; pga_gdb_copy, 5 MB 0.34 and 0.37, 12 MB 0.78 and 0.57.
+// table out (pga_build_kmer_adapter) 37-43 -> 8-10.  Below a size starting the
+// threads costs what they save; those copies, and memory that is pinned or
+// managed, go to the driver.  Where the line lies depends on the direction, and
+// going out on whether the destination's pages are there.  Driver, and 8 and 4
+// threads, us, each after 2 ms in which the threads' cores were idle:
+//   in                6 MB 304, 358, 298    8 MB 391, 410, 340   16 MB 750, 604, 525   48 MB 2640, 1370, 1300
+//   out, pages there  8 MB 512, 865, 864   16 MB 995, 1075, 970  20 MB 1230, 1073, 1050  48 MB 2890, 1875, 1800
+//   out, fresh pages  4 MB 1840, 1110, 1060  8 MB 3660, 1260, 1250  16 MB 7310, 1510, 2200  48 MB 21800, 3620, 5710
 #pragma once
 #include <atomic>
 #include <cstdint>
@@ -18,6 +21,8 @@
 #include <exception>
 #include <thread>
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 namespace pga {
 
@@ -25,7 +30,7 @@ class HostCopier {
  public:
   static constexpr int WORKERS = 8;
   static constexpr size_t CHUNK = 1 << 20;
-  static constexpr size_t STAGE_MIN = 6 << 20;
+  static constexpr size_t IN_MIN = 8 << 20, OUT_MIN = 20 << 20, FRESH_MIN = 4 << 20;  // least bytes staged
 
   // Copies `bytes` between `host` and `dev` in `st`'s order; a staged copy has
   // ended on return, any other is as cudaMemcpyAsync leaves it.
@@ -33,7 +38,9 @@ class HostCopier {
     const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
     void *dst = to_host ? host : dev;
     const void *src = to_host ? dev : host;
-    if (bytes < STAGE_MIN || !pageable(host) || !ready()) return cudaMemcpyAsync(dst, src, bytes, kind, st);
+    const bool faults = to_host && bytes >= FRESH_MIN && fresh(host, bytes);
+    if (bytes < (faults ? FRESH_MIN : to_host ? OUT_MIN : IN_MIN) || !pageable(host) || !ready())
+      return cudaMemcpyAsync(dst, src, bytes, kind, st);
     cudaError_t e = cudaEventRecord(before_, st);
     if (e != cudaSuccess) return e;
     const size_t chunks = (bytes + CHUNK - 1) / CHUNK;
@@ -71,7 +78,8 @@ class HostCopier {
     };
     std::thread t[WORKERS];
     int n = (int)std::thread::hardware_concurrency();
-    n = n < 1 ? 1 : n > WORKERS ? WORKERS : n;
+    const int most = faults ? WORKERS : WORKERS / 2;
+    n = n < 1 ? 1 : n > most ? most : n;
     for (int w = 1; w < n; w++) {
       try {
         t[w] = std::thread(work, w);
@@ -99,6 +107,17 @@ class HostCopier {
 
  private:
   static size_t length(size_t bytes, size_t c) { return bytes - c * CHUNK < CHUNK ? bytes - c * CHUNK : CHUNK; }
+  // Whether of 16 pages across the destination half or more are not there yet.
+  static bool fresh(const void *p, size_t bytes) {
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    int absent = 0;
+    for (int i = 0; i < 16; i++) {
+      unsigned char there = 1;
+      const uintptr_t at = ((uintptr_t)p + bytes / 16 * i) & ~(page - 1);
+      if (mincore((void *)at, 1, &there) == 0) absent += !(there & 1);
+    }
+    return absent >= 8;
+  }
   static bool pageable(const void *p) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
